@@ -62,6 +62,9 @@ __host__ __device__ __forceinline__ uint32_t morton3(uint32_t x, uint32_t y, uin
 struct Phys {
     float h, hh;
     float hh_le;      // the largest float r2 with sqrtf(r2) <= h: r2 <= hh_le is exactly sqrtf(r2) <= h
+    float eps_r2;     // the smallest float r2 with sqrtf(r2) >= 1e-8: r >= the kernels' epsilon
+    float minus_zero; // -0.f (pbf_sums.cuh: times)
+    int fast_root;    // the pair sums may take root and quotient by root_and_spiky's fast form
     float poly6f;     // 315 / (64 pi h^9)
     float spikyf;     // -45 / (pi h^6)
     float rho0, inv_rho0;
@@ -80,6 +83,7 @@ struct Phys {
 struct SceneDev {
     float min_ext[3];     // grid origin, solver units
     uint32_t ext[3];      // cells are clamped to [0, ext]
+    uint32_t ext_code[3]; // ext as the axis's bits of a Morton code
     uint32_t table_base;  // first entry of this scene's cell table
     uint32_t first, count;
     float dt, inv_dt, scale;

@@ -36,6 +36,14 @@ cudaError_t scan_u32(const uint32_t *in, uint32_t *out, uint32_t *total, uint64_
 // PBF stages (pbf.cu).  Arrays are indexed by particle over the whole batch.
 struct HostParticlesOut;
 
+// Whether the hit rows of rows.cu carry a skin, per scene and step.
+struct RowPolicy {
+    uint32_t keep;      // this step's do
+    uint32_t asked;     // particles of the second search
+    uint32_t used;      // those of them whose rows lasted
+    uint32_t without;   // steps since they last did
+};
+
 struct StepView {
     const SceneDev *scenes;
     const WellDev *wells;
@@ -105,6 +113,13 @@ struct StepView {
     const HostParticlesOut *hout;
     // the build pass counts the Verlet rows [0] and hit rows [1] that overflowed
     uint32_t *over;
+    // the gathers run on the hit rows of rows.cu, else (null) on the list kernels of
+    // pbf.cu: the first particle of every group -- a cell's particles up to where the
+    // index under group_mask wraps -- and the groups' number (zeroed every step)
+    uint32_t *groups, *group_count, group_mask;
+    uint32_t *moved;       // per particle: at a cell's first, the largest movement in the cell
+    uint8_t *lasting;      // per group
+    RowPolicy *row_policy, *row_policy_next;  // per scene: of the step before, and of this one
     // null, or [0] warps of the checked passes that ran on their near rows and [1]
     // warps that filtered their candidates instead (accumulated until read)
     uint32_t *near_stats;
@@ -130,6 +145,12 @@ void launch_list_policy(const StepView &s, cudaStream_t st);
 uint32_t slots_of_step(uint32_t iterations);
 void launch_delta(const StepView &s, const float4 *ps_in, float4 *ps_out, int iteration, bool last,
                   cudaStream_t st);
+// the gather passes over hit rows (rows.cu)
+cudaError_t launch_row_lambda(const StepView &s, const float4 *ps, int iteration, cudaStream_t st);
+cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_out, bool last, cudaStream_t st);
+cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaStream_t st,
+                                      const std::function<void()> &between);
+uint32_t row_group_mask(int profile, uint64_t n);  // StepView::group_mask for n particles
 // ref-profile colour diffusion of the sorted colours (col1, in place); agg and count
 // are n-entry scratch arrays
 void launch_diffuse(const StepView &s, uint4 *agg, uint32_t *count, cudaStream_t st);

@@ -18,18 +18,10 @@
 #include <cuda_runtime.h>
 
 #include "fgb_internal.h"
+#include "pbf_sums.cuh"
 
 namespace fgb {
 namespace {
-
-constexpr int kRef = FGB_PROFILE_REF;
-
-// Squared distance of a pair in the baseline profile's gathers: two fused
-// multiply-adds, as the oracle's baseline restatement computes it (the ref profile
-// keeps the reference's sum of three products).
-__device__ __forceinline__ float dist2(float dx, float dy, float dz) {
-    return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-}
 
 // Predicted position of one particle in solver units (oclsph.hpp:297-323).
 __device__ __forceinline__ float3 predict(const Phys &ph, const SceneDev &S, const WellDev *wells, int32_t type,
@@ -104,7 +96,8 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
                                 float4 *__restrict__ x1, float4 *__restrict__ v1, int32_t *__restrict__ type1,
                                 uint32_t *__restrict__ col1, uint32_t *__restrict__ slot1,
                                 float4 *__restrict__ ps, uint2 *__restrict__ cells, uint64_t cells_n,
-                                uint32_t *err, uint32_t *mass_range) {
+                                uint32_t *err, uint32_t *mass_range, uint32_t *__restrict__ groups,
+                                uint32_t *group_count, uint32_t group_mask) {
     // the smallest mass's bits and the complement of the largest's, both by atomicMin
     // (one pair per CTA); the masses are all equal when range[0] == ~range[1]
     __shared__ uint32_t s_lo, s_hi;
@@ -127,6 +120,17 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
         ps[i] = make_float4(p.x, p.y, p.z, xj.w);
         lo = min(lo, __float_as_uint(xj.w));
         hi = min(hi, ~__float_as_uint(xj.w));
+        if (groups) {  // list the groups of each cell's particles, one atomic a warp
+            const bool start = (i & group_mask) == 0 || keys[i - 1] != key;
+            const unsigned m = __activemask(), b = __ballot_sync(m, start);
+            if (b) {
+                const int leader = __ffs(m) - 1;
+                uint32_t at = 0;
+                if ((int)(threadIdx.x & 31u) == leader) at = atomicAdd(group_count, (uint32_t)__popc(b));
+                at = __shfl_sync(m, at, leader);
+                if (start) groups[at + __popc(b & lanemask_lt())] = i;
+            }
+        }
         const uint64_t c = (uint64_t)S.table_base + morton_of(key, mbits);
         if (c >= cells_n) {
             raise_error(err, ERR_CELL_RANGE);
@@ -574,41 +578,8 @@ __device__ __forceinline__ void lambda_body(const GatherArgs &A, uint32_t a, con
     const uint32_t key = A.keys[a];
     const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
     const float4 pa = ps[a];
-    float rho = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, g2 = 0.f;
-    auto body = [&](uint32_t b, const float4 &pb) {
-        const float dx = pa.x - pb.x, dy = pa.y - pb.y, dz = pa.z - pb.z;
-        if (PROFILE == kRef) {
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 <= ph.hh_le)) return;  // sqrtf(r2) > h: no contribution
-            const float r = sqrtf(r2);
-            if (r <= ph.h) {
-                const float t = ph.hh - r * r;
-                rho = __fmaf_rn(pa.w, ph.poly6f * (t * t * t), rho);
-                if (r >= kKernelEpsilon) {
-                    const float hr = ph.h - r;
-                    const float sc = ph.spikyf * ((hr * hr) / r);
-                    gx = __fmaf_rn(dx * sc, ph.inv_rho0, gx);
-                    gy = __fmaf_rn(dy * sc, ph.inv_rho0, gy);
-                    gz = __fmaf_rn(dz * sc, ph.inv_rho0, gz);
-                }
-            }
-        } else {
-            const float q2 = dist2(dx, dy, dz);
-            if (q2 <= ph.hh) {
-                const float t = ph.hh - q2;
-                rho = __fmaf_rn(pb.w, t * t * t, rho);
-                const float r = sqrtf(q2);
-                if (r >= kKernelEpsilon) {
-                    const float hr = ph.h - r;
-                    const float sc = pb.w * ((hr * hr) / r);
-                    gx = __fmaf_rn(sc, dx, gx);
-                    gy = __fmaf_rn(sc, dy, gy);
-                    gz = __fmaf_rn(sc, dz, gz);
-                    g2 = __fmaf_rn(sc * sc, q2, g2);
-                }
-            }
-        }
-    };
+    LambdaSum<PROFILE> sum;
+    auto body = [&](uint32_t, const float4 &pb) { sum.add(ph, pa, pb.x, pb.y, pb.z, pb.w); };
     // a later pass whose near row still holds every neighbour iterates it directly;
     // the choice is made per warp (all lanes or none), as a warp that mixed the two
     // paths would run both one after the other
@@ -678,20 +649,8 @@ __device__ __forceinline__ void lambda_body(const GatherArgs &A, uint32_t a, con
             else for_candidates(A, S, a, key, list, sp, body);
         }
     }
-    float dens, lam;
-    if (PROFILE == kRef) {
-        dens = rho;
-        const float norm2 = gx * gx + gy * gy + gz * gz;
-        const float C = dens / ph.rho0 - 1.f;
-        lam = -C / (norm2 + ph.cfm);
-    } else {
-        dens = rho * ph.poly6f;
-        const float gs = ph.spikyf * ph.inv_rho0;
-        const float sx = gx * gs, sy = gy * gs, sz = gz * gs;
-        const float denom = (sx * sx + sy * sy + sz * sz) + g2 * (gs * gs);
-        const float C = dens * ph.inv_rho0 - 1.f;
-        lam = -C / (denom + ph.cfm);
-    }
+    float dens;
+    const float lam = sum.finish(ph, &dens);
     lambda[a] = lam;
     density[a] = dens;
     if (A.plam) A.plam[a] = make_float4(pa.x, pa.y, pa.z, lam);
@@ -703,96 +662,6 @@ __global__ void __launch_bounds__(256) k_lambda(GatherArgs A, const float4 *__re
     for_tiles<kTiles>(A, [&](uint32_t a) {
         lambda_body<PROFILE, MODE>(A, a, GlobalSpace<char>{ps, nullptr, A.type}, ps, lambda, density);
     });
-}
-
-__device__ __forceinline__ float corr_pow(float ratio, float n) {
-    if (n == 4.f) {
-        const float r2 = ratio * ratio;
-        return r2 * r2;
-    }
-    return powf(ratio, n);
-}
-
-__device__ __forceinline__ float dot3(const float *a, const float *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
-
-// oclsph_collision.h:7-58 (first containing triangle within 40 world units wins).
-__device__ void collide_triangles(const TriDev *__restrict__ tris, uint32_t first, uint32_t count, float *pos,
-                                  float *vel) {
-    for (uint32_t i = 0; i < count; ++i) {
-        const TriDev t = tris[first + i];
-        float e1[3], e2[3], nrm[3];
-        for (int a = 0; a < 3; ++a) {
-            e1[a] = t.b[a] - t.a[a];
-            e2[a] = t.c[a] - t.a[a];
-        }
-        nrm[0] = e1[1] * e2[2] - e1[2] * e2[1];
-        nrm[1] = e1[2] * e2[0] - e1[0] * e2[2];
-        nrm[2] = e1[0] * e2[1] - e1[1] * e2[0];
-        const float len = sqrtf(dot3(nrm, nrm));
-        const float nn[3] = {nrm[0] / len, nrm[1] / len, nrm[2] / len};
-        const float dist = dot3(nn, t.a) - dot3(nn, pos);
-        if (-40.f <= dist && dist <= 40.f) {
-            const float p0[3] = {pos[0] + nn[0] * dist, pos[1] + nn[1] * dist, pos[2] + nn[2] * dist};
-            float v0[3], v1[3], v2[3];
-            for (int a = 0; a < 3; ++a) {
-                v0[a] = t.c[a] - t.a[a];
-                v1[a] = t.b[a] - t.a[a];
-                v2[a] = p0[a] - t.a[a];
-            }
-            const float d00 = dot3(v0, v0), d01 = dot3(v0, v1), d02 = dot3(v0, v2);
-            const float d11 = dot3(v1, v1), d12 = dot3(v1, v2);
-            const float inv = 1.f / (d00 * d11 - d01 * d01);
-            const float u = (d11 * d02 - d01 * d12) * inv;
-            const float w = (d00 * d12 - d01 * d02) * inv;
-            if ((u >= 0.f) && (w >= 0.f) && (u + w < 1.f)) {
-                const float vn = dot3(vel, nn);
-                for (int a = 0; a < 3; ++a) {
-                    vel[a] = vel[a] - (nn[a] * 2.f) * vn;
-                    pos[a] = p0[a];
-                }
-                return;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void collide_sphere(const SceneDev &S, float *pos) {
-    if (!S.sphere_enabled) return;
-    const float d[3] = {pos[0] - S.sphere[0], pos[1] - S.sphere[1], pos[2] - S.sphere[2]};
-    const float r = S.sphere[3];
-    const float d2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    if (!(d2 < r * r)) return;
-    const float dist = sqrtf(d2);
-    if (dist > 0.f) {
-        const float s = r / dist;
-        for (int a = 0; a < 3; ++a) pos[a] = S.sphere[a] + d[a] * s;
-    } else {
-        pos[0] = S.sphere[0];
-        pos[1] = S.sphere[1] + r;
-        pos[2] = S.sphere[2];
-    }
-}
-
-
-// Final position and velocity of particle a into the caller's arrays (fgb_advance
-// with direct host I/O): the step's last kernel stores them beside its own writes.
-__device__ __forceinline__ void store_host_motion(const HostParticlesOut *__restrict__ hout, uint32_t a,
-                                                  const float4 &xa, const float4 &va) {
-    if (!hout) return;
-    const uint32_t stride = hout->stride;  // 0: packed arrays, else the caller's records
-    float *pp = hout->position, *pv = hout->velocity;
-    if (pp) {
-        float *q = stride ? (float *)((char *)pp + (size_t)a * stride) : pp + 3 * (size_t)a;
-        q[0] = xa.x;
-        q[1] = xa.y;
-        q[2] = xa.z;
-    }
-    if (pv) {
-        float *q = stride ? (float *)((char *)pv + (size_t)a * stride) : pv + 3 * (size_t)a;
-        q[0] = va.x;
-        q[1] = va.y;
-        q[2] = va.z;
-    }
 }
 
 template <int PROFILE, int MODE, class Sp>
@@ -812,43 +681,10 @@ __device__ __forceinline__ void delta_body(const GatherArgs &A, uint32_t a, cons
     const uint32_t key = A.keys[a];
     const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
     const float la = lambda[a];
-    float px = 0.f, py = 0.f, pz = 0.f;
+    DeltaSum<PROFILE> sum;
     // lam_b() is lambda of b (gathered beside p_b on rows, loaded on demand on walks)
-    auto body = [&](uint32_t b, const float4 &pb, auto lam_b) {
-        const float dx = pa.x - pb.x, dy = pa.y - pb.y, dz = pa.z - pb.z;
-        if (PROFILE == kRef) {
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            if (!(r2 <= ph.hh_le)) return;  // sqrtf(r2) > h: no contribution
-            const float r = sqrtf(r2);
-            float w = 0.f;
-            if (r <= ph.h) {
-                const float t = ph.hh - r * r;
-                w = ph.poly6f * (t * t * t);
-            }
-            const float corr = -ph.corr_k * corr_pow(w / ph.corr_ref, ph.corr_n);
-            const float factor = (la + lam_b() + corr) / ph.rho0;
-            if (r >= kKernelEpsilon && r <= ph.h) {
-                const float hr = ph.h - r;
-                const float sc = ph.spikyf * ((hr * hr) / r);
-                px = __fmaf_rn(dx * sc, factor, px);
-                py = __fmaf_rn(dy * sc, factor, py);
-                pz = __fmaf_rn(dz * sc, factor, pz);
-            }
-        } else {
-            const float q2 = dist2(dx, dy, dz);
-            if (q2 <= ph.hh) {
-                const float r = sqrtf(q2);
-                if (r >= kKernelEpsilon) {
-                    const float t = ph.hh - q2;
-                    const float corr = -ph.corr_k * corr_pow((t * t * t) * ph.inv_corr_wdq, ph.corr_n);
-                    const float hr = ph.h - r;
-                    const float sc = sp.mass(pb) * ((hr * hr) / r) * (la + lam_b() + corr);
-                    px = __fmaf_rn(sc, dx, px);
-                    py = __fmaf_rn(sc, dy, py);
-                    pz = __fmaf_rn(sc, dz, pz);
-                }
-            }
-        }
+    auto body = [&](uint32_t, const float4 &pb, auto lam_b) {
+        sum.add(ph, pa, la, pb.x, pb.y, pb.z, lam_b, sp.mass(pb));
     };
     if (have_hits(A, a)) {
         if constexpr (Sp::kPacked) {
@@ -862,31 +698,9 @@ __device__ __forceinline__ void delta_body(const GatherArgs &A, uint32_t a, cons
             body(b, pb, [&] { return sp.lam(b, pb); });
         });
     }
-    float world[3];
-    if (PROFILE == kRef) {
-        world[0] = (pa.x + px) * S.scale;
-        world[1] = (pa.y + py) * S.scale;
-        world[2] = (pa.z + pz) * S.scale;
-    } else {
-        const float gs = ph.spikyf * ph.inv_rho0;
-        world[0] = (pa.x + px * gs) * S.scale;
-        world[1] = (pa.y + py * gs) * S.scale;
-        world[2] = (pa.z + pz * gs) * S.scale;
-        collide_sphere(S, world);
-    }
-    float4 va = v[a];
-    float vel[3] = {va.x, va.y, va.z};
-    if (S.tri_count) {
-        collide_triangles(A.tris, S.tri_first, S.tri_count, world, vel);
-        v[a] = make_float4(vel[0], vel[1], vel[2], va.w);
-    }
-    float q[3];
-    for (int d = 0; d < 3; ++d) {
-        float w = world[d];
-        w = fmaxf(S.min_b[d], w);
-        w = fminf(S.max_b[d], w);
-        q[d] = w / S.scale;
-    }
+    float4 va;
+    float q[3], vel[3];
+    sum.move(ph, S, A.tris, pa, a, v, q, va, vel);
     ps_out[a] = make_float4(q[0], q[1], q[2], pa.w);
     if (A.cap) {
         // distance moved since the grid was built, for the list bound of the next pass
@@ -910,25 +724,7 @@ __device__ __forceinline__ void delta_body(const GatherArgs &A, uint32_t a, cons
             }
         }
     }
-    if (last) {
-        const float4 xa = x[a];
-        const float xo[3] = {xa.x, xa.y, xa.z};
-        float nv[3], nx[3];
-        for (int d = 0; d < 3; ++d) {
-            const float dd = q[d] - xo[d] / S.scale;
-            if (PROFILE == kRef) {
-                nx[d] = q[d] * S.scale;
-                nv[d] = __fmaf_rn(dd, S.inv_dt, vel[d]) * ph.damping;
-            } else {
-                nv[d] = dd * S.inv_dt;
-            }
-        }
-        v[a] = make_float4(nv[0], nv[1], nv[2], va.w);
-        if (PROFILE == kRef) {
-            x[a] = make_float4(nx[0], nx[1], nx[2], xa.w);
-            store_host_motion(hout, a, x[a], v[a]);
-        }
-    }
+    if (last) finalise<PROFILE>(ph, S, a, q, va, vel, x, v, hout);
 }
 
 template <int PROFILE, int MODE, bool kTiles>
@@ -947,12 +743,6 @@ __global__ void __launch_bounds__(256)
             delta_body<PROFILE, MODE>(A, a, GlobalSpace<float>{ps_in, lambda, A.type}, ps_in, lambda, ps_out, x, v,
                                       last, hout);
     });
-}
-
-__device__ __forceinline__ void cross3(const float *a, const float *b, float *o) {
-    o[0] = a[1] * b[2] - a[2] * b[1];
-    o[1] = a[2] * b[0] - a[0] * b[2];
-    o[2] = a[0] * b[1] - a[1] * b[0];
 }
 
 // Pass A: vorticity omega and the XSPH sum (fluid neighbours only).
@@ -992,32 +782,12 @@ __device__ __forceinline__ void vorticity_body(const GatherArgs &A, uint32_t a, 
         if (!near) A.near[a] = 0;
     }
     const bool list = near ? false : use_list<kCheck>(A, S, a, key, mcd);
-    const float va[3] = {va4.x, va4.y, va4.z};
-    float o[3] = {0.f, 0.f, 0.f}, xs[3] = {0.f, 0.f, 0.f};
+    VorticitySum sum;
     // fluid_known: b came from a filtered hit row, which holds fluid particles only;
     // vel_b() is v of b (gathered beside p_b on rows, loaded on demand on walks)
     auto body = [&](uint32_t b, const float4 &pb, auto vel_b, bool fluid_known) {
         if (!fluid_known && S.obstacles && !sp.fluid(b)) return;
-        const float d[3] = {pa.x - pb.x, pa.y - pb.y, pa.z - pb.z};
-        const float r2 = dist2(d[0], d[1], d[2]);
-        if (!(r2 <= ph.hh)) return;
-        const float4 vb = vel_b();
-        const float vab[3] = {vb.x - va[0], vb.y - va[1], vb.z - va[2]};
-        const float t = ph.hh - r2;
-        const float mw = pb.w * (t * t * t);
-        xs[0] = __fmaf_rn(mw, vab[0], xs[0]);
-        xs[1] = __fmaf_rn(mw, vab[1], xs[1]);
-        xs[2] = __fmaf_rn(mw, vab[2], xs[2]);
-        const float r = sqrtf(r2);
-        if (r >= kKernelEpsilon) {
-            const float hr = ph.h - r;
-            const float sc = pb.w * ((hr * hr) / r);
-            float cr[3];
-            cross3(vab, d, cr);
-            o[0] = __fmaf_rn(sc, cr[0], o[0]);
-            o[1] = __fmaf_rn(sc, cr[1], o[1]);
-            o[2] = __fmaf_rn(sc, cr[2], o[2]);
-        }
+        sum.add(ph, pa, va4, pb.x, pb.y, pb.z, pb.w, vel_b);
     };
     auto any = [&](uint32_t b, const float4 &pb) {
         body(b, pb, [&] { return sp.x(b); }, false);
@@ -1044,16 +814,7 @@ __device__ __forceinline__ void vorticity_body(const GatherArgs &A, uint32_t a, 
             for_candidates(A, S, a, key, list, sp, any);
         }
     }
-    const float gs = ph.spikyf * ph.inv_rho0;
-    const float ws = ph.poly6f * ph.inv_rho0;
-    // omega = sum_b m_b / rho0 (v_b - v_a) x grad_b W(x_a - x_b), and grad_b W = -grad_a W
-    // = -spikyf (h - r)^2 d / r: the sum o carries grad_a's factor, so its sign flips
-    const float ox = -(o[0] * gs), oy = -(o[1] * gs), oz = -(o[2] * gs);
-    const float om = sqrtf(ox * ox + oy * oy + oz * oz);
-    omega[a] = make_float4(ox, oy, oz, om);
-    if (A.pom) A.pom[a] = make_float4(pa.x, pa.y, pa.z, om);
-    vx[a] = make_float4(__fmaf_rn(ph.xsph_c, xs[0] * ws, va[0]), __fmaf_rn(ph.xsph_c, xs[1] * ws, va[1]),
-                        __fmaf_rn(ph.xsph_c, xs[2] * ws, va[2]), va4.w);
+    sum.finish(ph, a, pa, va4, omega, A.pom, vx);
 }
 
 template <bool kTiles>
@@ -1079,60 +840,31 @@ __device__ __forceinline__ void apply_body(const GatherArgs &A, uint32_t a, cons
     const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
     const float4 pa = ps[a];
     const float4 oa = omega[a];
-    float e[3] = {0.f, 0.f, 0.f};
+    ApplySum sum;
     // fluid_known: b came from a filtered hit row, which holds fluid particles only;
-    // om_b() is omega of b (gathered beside p_b on rows, loaded on demand on walks)
+    // om_b() is |omega| of b (gathered beside p_b on rows, loaded on demand on walks)
     auto body = [&](uint32_t b, const float4 &pb, auto om_b, bool fluid_known) {
         if (!fluid_known && S.obstacles && !sp.fluid(b)) return;
-        const float d[3] = {pa.x - pb.x, pa.y - pb.y, pa.z - pb.z};
-        const float r2 = dist2(d[0], d[1], d[2]);
-        if (!(r2 <= ph.hh)) return;
-        const float r = sqrtf(r2);
-        if (!(r >= kKernelEpsilon)) return;
-        const float hr = ph.h - r;
-        const float sc = sp.mass(pb) * ((hr * hr) / r) * (om_b().w - oa.w);
-        e[0] = __fmaf_rn(sc, d[0], e[0]);
-        e[1] = __fmaf_rn(sc, d[1], e[1]);
-        e[2] = __fmaf_rn(sc, d[2], e[2]);
+        sum.add(ph, pa, oa.w, pb.x, pb.y, pb.z, om_b, sp.mass(pb));
     };
     if (have_hits(A, a)) {
         // a near row (still marked) holds obstacles too; a filtered row fluid only
         const bool fluid_rows = !(A.near && A.near[a]);
         if constexpr (Sp::kPacked) {
             auto row = [&](uint32_t b, const float4 &pb) {
-                body(b, pb, [&] { return make_float4(0.f, 0.f, 0.f, pb.w); }, fluid_rows);
+                body(b, pb, [&] { return pb.w; }, fluid_rows);
             };
             for_row(A.hlist, A.hcap, a, A.hcount[a], sp, row);
         } else {
-            auto row = [&](uint32_t b, const float4 &pb, auto om_b) { body(b, pb, om_b, fluid_rows); };
+            auto row = [&](uint32_t b, const float4 &pb, auto om_b) { body(b, pb, [&] { return om_b().w; }, fluid_rows); };
             for_row_x(A.hlist, A.hcap, a, A.hcount[a], sp, row);
         }
     } else {
         for_candidates(A, S, a, key, use_list<kStored>(A, S, a, key), sp, [&](uint32_t b, const float4 &pb) {
-            body(b, pb, [&] { return Sp::kPacked ? make_float4(0.f, 0.f, 0.f, pb.w) : sp.omega_of(b); }, false);
+            body(b, pb, [&] { return Sp::kPacked ? pb.w : sp.omega_of(b).w; }, false);
         });
     }
-    const float gs = ph.spikyf * ph.inv_rho0;
-    const float ex = e[0] * gs, ey = e[1] * gs, ez = e[2] * gs;
-    const float el = sqrtf(ex * ex + ey * ey + ez * ez);
-    float N[3] = {0.f, 0.f, 0.f};
-    if (el > 0.f) {
-        N[0] = ex / el;
-        N[1] = ey / el;
-        N[2] = ez / el;
-    }
-    const float om[3] = {oa.x, oa.y, oa.z};
-    float f[3];
-    cross3(N, om, f);
-    const float4 vxa = vx[a];
-    const float ve = ph.vort_eps, dt = S.dt;
-    const float4 vn = make_float4(__fmaf_rn(dt, f[0] * ve, vxa.x), __fmaf_rn(dt, f[1] * ve, vxa.y),
-                                  __fmaf_rn(dt, f[2] * ve, vxa.z), vxa.w);
-    v[a] = vn;
-    const float4 xa = x[a];
-    const float4 xn = make_float4(pa.x * S.scale, pa.y * S.scale, pa.z * S.scale, xa.w);
-    x[a] = xn;
-    store_host_motion(hout, a, xn, vn);
+    sum.finish(ph, S, a, pa, oa, vx, v, x, hout);
 }
 
 template <bool kTiles>
@@ -1371,7 +1103,7 @@ void launch_reorder_cells(const StepView &s, cudaStream_t st) {
     k_reorder_cells<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.wells, s.ph, s.n, s.mbits, s.keys_sorted,
                                                       s.vals_sorted, s.x0, s.v0, s.type0, s.col0, s.slot0, s.x1,
                                                       s.v1, s.type1, s.col1, s.slot1, s.ps_grid, s.cells, s.cells_n,
-                                                      s.err, s.mass_range);
+                                                      s.err, s.mass_range, s.groups, s.group_count, s.group_mask);
 }
 
 // Grid and tile counter of one gather launch (slot: its place among the step's

@@ -1,0 +1,609 @@
+// pbf_sums.cuh -- the pair sums of the gather passes and what each particle does with
+// them, shared by the row kernels (pbf.cu) and the tile kernels (tiles.cu).
+//
+// Every sum adds its neighbours in the order it is given them, with the reference's
+// formulas; both kernel families visit the same neighbours in the same order, so they
+// compute the same bits.
+#pragma once
+
+#include "fgb_internal.h"
+
+namespace fgb {
+
+constexpr int kRef = FGB_PROFILE_REF;
+
+// Squared distance of a pair in the baseline profile's gathers: two fused
+// multiply-adds, as the oracle's baseline restatement computes it (the ref profile
+// keeps the reference's sum of three products).
+__device__ __forceinline__ float dist2(float dx, float dy, float dz) {
+    return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+}
+
+__device__ __forceinline__ float corr_pow(float ratio, float n) {
+    if (n == 4.f) {
+        const float r2 = ratio * ratio;
+        return r2 * r2;
+    }
+    return powf(ratio, n);
+}
+
+__device__ __forceinline__ float dot3(const float *a, const float *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+
+// oclsph_collision.h:7-58 (first containing triangle within 40 world units wins).
+__device__ inline void collide_triangles(const TriDev *__restrict__ tris, uint32_t first, uint32_t count, float *pos,
+                                  float *vel) {
+    for (uint32_t i = 0; i < count; ++i) {
+        const TriDev t = tris[first + i];
+        float e1[3], e2[3], nrm[3];
+        for (int a = 0; a < 3; ++a) {
+            e1[a] = t.b[a] - t.a[a];
+            e2[a] = t.c[a] - t.a[a];
+        }
+        nrm[0] = e1[1] * e2[2] - e1[2] * e2[1];
+        nrm[1] = e1[2] * e2[0] - e1[0] * e2[2];
+        nrm[2] = e1[0] * e2[1] - e1[1] * e2[0];
+        const float len = sqrtf(dot3(nrm, nrm));
+        const float nn[3] = {nrm[0] / len, nrm[1] / len, nrm[2] / len};
+        const float dist = dot3(nn, t.a) - dot3(nn, pos);
+        if (-40.f <= dist && dist <= 40.f) {
+            const float p0[3] = {pos[0] + nn[0] * dist, pos[1] + nn[1] * dist, pos[2] + nn[2] * dist};
+            float v0[3], v1[3], v2[3];
+            for (int a = 0; a < 3; ++a) {
+                v0[a] = t.c[a] - t.a[a];
+                v1[a] = t.b[a] - t.a[a];
+                v2[a] = p0[a] - t.a[a];
+            }
+            const float d00 = dot3(v0, v0), d01 = dot3(v0, v1), d02 = dot3(v0, v2);
+            const float d11 = dot3(v1, v1), d12 = dot3(v1, v2);
+            const float inv = 1.f / (d00 * d11 - d01 * d01);
+            const float u = (d11 * d02 - d01 * d12) * inv;
+            const float w = (d00 * d12 - d01 * d02) * inv;
+            if ((u >= 0.f) && (w >= 0.f) && (u + w < 1.f)) {
+                const float vn = dot3(vel, nn);
+                for (int a = 0; a < 3; ++a) {
+                    vel[a] = vel[a] - (nn[a] * 2.f) * vn;
+                    pos[a] = p0[a];
+                }
+                return;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void collide_sphere(const SceneDev &S, float *pos) {
+    if (!S.sphere_enabled) return;
+    const float d[3] = {pos[0] - S.sphere[0], pos[1] - S.sphere[1], pos[2] - S.sphere[2]};
+    const float r = S.sphere[3];
+    const float d2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    if (!(d2 < r * r)) return;
+    const float dist = sqrtf(d2);
+    if (dist > 0.f) {
+        const float s = r / dist;
+        for (int a = 0; a < 3; ++a) pos[a] = S.sphere[a] + d[a] * s;
+    } else {
+        pos[0] = S.sphere[0];
+        pos[1] = S.sphere[1] + r;
+        pos[2] = S.sphere[2];
+    }
+}
+
+
+// Final position and velocity of particle a into the caller's arrays (fgb_advance
+// with direct host I/O): the step's last kernel stores them beside its own writes.
+__device__ __forceinline__ void store_host_motion(const HostParticlesOut *__restrict__ hout, uint32_t a,
+                                                  const float4 &xa, const float4 &va) {
+    if (!hout) return;
+    const uint32_t stride = hout->stride;  // 0: packed arrays, else the caller's records
+    float *pp = hout->position, *pv = hout->velocity;
+    if (pp) {
+        float *q = stride ? (float *)((char *)pp + (size_t)a * stride) : pp + 3 * (size_t)a;
+        q[0] = xa.x;
+        q[1] = xa.y;
+        q[2] = xa.z;
+    }
+    if (pv) {
+        float *q = stride ? (float *)((char *)pv + (size_t)a * stride) : pv + 3 * (size_t)a;
+        q[0] = va.x;
+        q[1] = va.y;
+        q[2] = va.z;
+    }
+}
+
+__device__ __forceinline__ void cross3(const float *a, const float *b, float *o) {
+    o[0] = a[1] * b[2] - a[2] * b[1];
+    o[1] = a[2] * b[0] - a[0] * b[2];
+    o[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+
+// Two floats in one 64-bit register pair, for the packed add, mul and fma (each half
+// rounds as the scalar operation does).
+struct Two {
+    uint64_t v;
+    __device__ __forceinline__ Two() {}
+    __device__ __forceinline__ explicit Two(uint64_t v_) : v(v_) {}
+    __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
+    __device__ __forceinline__ float lo() const { return __uint_as_float((uint32_t)v); }
+    __device__ __forceinline__ float hi() const { return __uint_as_float((uint32_t)(v >> 32)); }
+};
+__device__ __forceinline__ Two operator-(const Two &a, const Two &b) {
+    Two r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Two operator+(const Two &a, const Two &b) {
+    Two r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Two operator*(const Two &a, const Two &b) {
+    Two r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Two fma(const Two &a, const Two &b, const Two &c) {
+    Two r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Two operator-(const Two &a) { return Two(-a.lo(), -a.hi()); }
+// A product that a sum or a difference takes up: ptxas fuses mul.rn.f32x2 with the add
+// that follows (it leaves the scalar form alone), so the product is a multiply-add of
+// minus zero, which rounds as the product does; the zero comes from the kernel's
+// arguments, where the compiler does not know it.
+__device__ __forceinline__ Two times(const Phys &ph, const Two &a, const Two &b) { return fma(a, b, Two(ph.minus_zero)); }
+// r^2 of a pair of neighbours, as dist2
+__device__ __forceinline__ Two dist2(const Two &dx, const Two &dy, const Two &dz) {
+    return fma(dx, dx, fma(dy, dy, dz * dz));
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Of a pair of neighbours at squared distances q2 <= h^2: r = sqrt(q2) and
+// s = (h - r)^2 / r, both correctly rounded -- the bits of sqrtf and of the division.
+//
+// kFast (Phys::fast_root): one approximate reciprocal square root y serves both.  A
+// Newton step on q2 y gives the root, a Newton step on y the reciprocal of r, and the
+// quotient is corrected by its exact remainder (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990: with the correctly rounded
+// reciprocal and a faithful quotient the corrected quotient is correctly rounded).  The
+// reciprocal's error is below 2^-43 before its rounding, so it can be misrounded only for
+// the few mantissas whose reciprocals lie that near the midpoint of two floats; the host
+// checks the quotients of those for the solver's h (fast_root.h) and
+// clears fast_root if one fails.  17 packed operations for two neighbours, where the
+// compiler's root and quotient take about 60 instructions with their range checks.
+// Below q2 = 1e-30 (only there does the approximation leave the normal range) r is
+// meaningless; its users drop s below eps_r2.
+template <bool kFast>
+__device__ __forceinline__ void root_and_spiky(const Phys &ph, const Two &q2, Two &r, Two &s) {
+    if constexpr (kFast) {
+        const Two y(rsqrt_approx(q2.lo()), rsqrt_approx(q2.hi()));
+        const Two g = q2 * y;
+        r = fma(fma(-g, g, q2), y * Two(0.5f), g);
+        const Two hr = Two(ph.h) - r, a = hr * hr, nr = -r;
+        const Two inv = fma(fma(nr, y, Two(1.f)), y, y);
+        const Two w = a * inv;
+        s = fma(fma(nr, w, a), inv, w);
+    } else {
+        const float r0 = sqrtf(q2.lo()), r1 = sqrtf(q2.hi());
+        const float h0 = ph.h - r0, h1 = ph.h - r1;
+        r = Two(r0, r1);
+        s = Two((h0 * h0) / r0, (h1 * h1) / r1);
+    }
+}
+
+// a / c of a pair, correctly rounded, for a constant c with inv_c = 1 / c correctly rounded.
+// kFast: Markstein's correction again; a is zero or within 2^+-90 (else the division).
+template <bool kFast>
+__device__ __forceinline__ Two over_const(const Two &a, float c, float inv_c) {
+    if constexpr (kFast) {
+        const Two w = a * Two(inv_c);
+        return fma(fma(Two(-c), w, a), Two(inv_c), w);
+    }
+    return Two(a.lo() / c, a.hi() / c);
+}
+
+// Density and constraint gradients of one particle (oclsph_kernel.h:305-346).
+template <int PROFILE>
+struct LambdaSum {
+    float rho = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, g2 = 0.f;
+
+    __device__ __forceinline__ void add(const Phys &ph, const float4 &pa, float bx, float by, float bz, float mb) {
+        const float dx = pa.x - bx, dy = pa.y - by, dz = pa.z - bz;
+        if (PROFILE == kRef) {
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            if (!(r2 <= ph.hh_le)) return;  // sqrtf(r2) > h: no contribution
+            const float r = sqrtf(r2);
+            if (r <= ph.h) {
+                const float t = ph.hh - r * r;
+                rho = __fmaf_rn(pa.w, ph.poly6f * (t * t * t), rho);
+                if (r >= kKernelEpsilon) {
+                    const float hr = ph.h - r;
+                    const float sc = ph.spikyf * ((hr * hr) / r);
+                    gx = __fmaf_rn(dx * sc, ph.inv_rho0, gx);
+                    gy = __fmaf_rn(dy * sc, ph.inv_rho0, gy);
+                    gz = __fmaf_rn(dz * sc, ph.inv_rho0, gz);
+                }
+            }
+        } else {
+            const float q2 = dist2(dx, dy, dz);
+            if (q2 <= ph.hh) {
+                const float t = ph.hh - q2;
+                rho = __fmaf_rn(mb, t * t * t, rho);
+                const float r = sqrtf(q2);
+                if (r >= kKernelEpsilon) {
+                    const float hr = ph.h - r;
+                    const float sc = mb * ((hr * hr) / r);
+                    gx = __fmaf_rn(sc, dx, gx);
+                    gy = __fmaf_rn(sc, dy, gy);
+                    gz = __fmaf_rn(sc, dz, gz);
+                    g2 = __fmaf_rn(sc * sc, q2, g2);
+                }
+            }
+        }
+    }
+
+    // two neighbours in order; r^2 above h^2 (a staged point at infinity) adds nothing
+    template <bool kFast>
+    __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, const Two &bx, const Two &by, const Two &bz,
+                                         const Two &mb) {
+        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
+        Two r, s;
+        if (PROFILE == kRef) {
+            const Two q2 = (times(ph, dx, dx) + times(ph, dy, dy)) + times(ph, dz, dz);
+            root_and_spiky<kFast>(ph, q2, r, s);
+            const Two t = Two(ph.hh) - times(ph, r, r), w = Two(ph.poly6f) * (t * t * t);
+            const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;
+            one<kFast>(ph, pa, q2.lo(), w.lo(), kx.lo(), ky.lo(), kz.lo());
+            one<kFast>(ph, pa, q2.hi(), w.hi(), kx.hi(), ky.hi(), kz.hi());
+        } else {
+            const Two q2 = dist2(dx, dy, dz);
+            root_and_spiky<kFast>(ph, q2, r, s);
+            const Two t = Two(ph.hh) - q2, w = t * t * t, sc = mb * s, ss = sc * sc;
+            one(ph, q2.lo(), mb.lo(), w.lo(), sc.lo(), ss.lo(), dx.lo(), dy.lo(), dz.lo());
+            one(ph, q2.hi(), mb.hi(), w.hi(), sc.hi(), ss.hi(), dx.hi(), dy.hi(), dz.hi());
+        }
+    }
+    __device__ __forceinline__ void one(const Phys &ph, float q2, float m, float w, float sc, float ss, float dx,
+                                        float dy, float dz) {
+        if (q2 <= ph.hh) {
+            rho = __fmaf_rn(m, w, rho);
+            if (q2 >= ph.eps_r2) {
+                gx = __fmaf_rn(sc, dx, gx);
+                gy = __fmaf_rn(sc, dy, gy);
+                gz = __fmaf_rn(sc, dz, gz);
+                g2 = __fmaf_rn(ss, q2, g2);
+            }
+        }
+    }
+    template <bool kFast>
+    __device__ __forceinline__ void one(const Phys &ph, const float4 &pa, float q2, float w, float kx, float ky,
+                                        float kz) {
+        if (!(q2 <= ph.hh_le)) return;
+        // on top of each other, at fast_root's h: r^2 vanishes beside h^2 (and the fast root
+        // of r^2 below 1e-30 is meaningless)
+        if (kFast && q2 < ph.eps_r2) w = ph.poly6f * (ph.hh * ph.hh * ph.hh);
+        rho = __fmaf_rn(pa.w, w, rho);
+        if (q2 >= ph.eps_r2) {
+            gx = __fmaf_rn(kx, ph.inv_rho0, gx);
+            gy = __fmaf_rn(ky, ph.inv_rho0, gy);
+            gz = __fmaf_rn(kz, ph.inv_rho0, gz);
+        }
+    }
+
+    // lambda, and the density in *dens
+    __device__ __forceinline__ float finish(const Phys &ph, float *dens) const {
+        if (PROFILE == kRef) {
+            *dens = rho;
+            const float norm2 = gx * gx + gy * gy + gz * gz;
+            const float C = rho / ph.rho0 - 1.f;
+            return -C / (norm2 + ph.cfm);
+        }
+        *dens = rho * ph.poly6f;
+        const float gs = ph.spikyf * ph.inv_rho0;
+        const float sx = gx * gs, sy = gy * gs, sz = gz * gs;
+        const float denom = (sx * sx + sy * sy + sz * sz) + g2 * (gs * gs);
+        const float C = *dens * ph.inv_rho0 - 1.f;
+        return -C / (denom + ph.cfm);
+    }
+};
+
+// Position correction of one particle (oclsph_kernel.h:348-384).
+template <int PROFILE>
+struct DeltaSum {
+    float px = 0.f, py = 0.f, pz = 0.f;
+
+    // la: the particle's lambda; lam_b(): the neighbour's
+    template <class L>
+    __device__ __forceinline__ void add(const Phys &ph, const float4 &pa, float la, float bx, float by, float bz,
+                                        L &&lam_b, float mb) {
+        const float dx = pa.x - bx, dy = pa.y - by, dz = pa.z - bz;
+        if (PROFILE == kRef) {
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            if (!(r2 <= ph.hh_le)) return;  // sqrtf(r2) > h: no contribution
+            const float r = sqrtf(r2);
+            float w = 0.f;
+            if (r <= ph.h) {
+                const float t = ph.hh - r * r;
+                w = ph.poly6f * (t * t * t);
+            }
+            const float corr = -ph.corr_k * corr_pow(w / ph.corr_ref, ph.corr_n);
+            const float factor = (la + lam_b() + corr) / ph.rho0;
+            if (r >= kKernelEpsilon && r <= ph.h) {
+                const float hr = ph.h - r;
+                const float sc = ph.spikyf * ((hr * hr) / r);
+                px = __fmaf_rn(dx * sc, factor, px);
+                py = __fmaf_rn(dy * sc, factor, py);
+                pz = __fmaf_rn(dz * sc, factor, pz);
+            }
+        } else {
+            const float q2 = dist2(dx, dy, dz);
+            if (q2 <= ph.hh) {
+                const float r = sqrtf(q2);
+                if (r >= kKernelEpsilon) {
+                    const float t = ph.hh - q2;
+                    const float corr = -ph.corr_k * corr_pow((t * t * t) * ph.inv_corr_wdq, ph.corr_n);
+                    const float hr = ph.h - r;
+                    const float sc = mb * ((hr * hr) / r) * (la + lam_b() + corr);
+                    px = __fmaf_rn(sc, dx, px);
+                    py = __fmaf_rn(sc, dy, py);
+                    pz = __fmaf_rn(sc, dz, pz);
+                }
+            }
+        }
+    }
+
+    // two neighbours in order, their lambdas in lb
+    template <bool kFast>
+    __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, float la, const Two &bx, const Two &by,
+                                         const Two &bz, const Two &lb, const Two &mb) {
+        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
+        Two r, s, k;
+        if (PROFILE == kRef) {
+            const Two q2 = (times(ph, dx, dx) + times(ph, dy, dy)) + times(ph, dz, dz);
+            root_and_spiky<kFast>(ph, q2, r, s);
+            const Two t = Two(ph.hh) - times(ph, r, r), w = Two(ph.poly6f) * (t * t * t);
+            const Two c =
+                times(ph, Two(-ph.corr_k), corr<kFast>(ph, over_const<kFast>(w, ph.corr_ref, ph.inv_corr_ref)));
+            const Two sum = (Two(la) + lb) + c;
+            Two f = over_const<kFast>(sum, ph.rho0, ph.inv_rho0);
+            if (kFast) {
+                // outside over_const's range (a sum that cancelled, or one that ran away)
+                const float s0 = fabsf(sum.lo()), s1 = fabsf(sum.hi());
+                if (!(fminf(s0, s1) > 1e-27f && fmaxf(s0, s1) < 1e27f))
+                    f = Two(sum.lo() / ph.rho0, sum.hi() / ph.rho0);
+            }
+            const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;
+            if (q2.lo() <= ph.hh_le && q2.lo() >= ph.eps_r2) move_by(f.lo(), kx.lo(), ky.lo(), kz.lo());
+            if (q2.hi() <= ph.hh_le && q2.hi() >= ph.eps_r2) move_by(f.hi(), kx.hi(), ky.hi(), kz.hi());
+        } else {
+            const Two q2 = dist2(dx, dy, dz);
+            root_and_spiky<kFast>(ph, q2, r, s);
+            const Two t = Two(ph.hh) - q2;
+            const Two c = times(ph, Two(-ph.corr_k), corr<kFast>(ph, (t * t * t) * Two(ph.inv_corr_wdq)));
+            const Two sc = mb * s * ((Two(la) + lb) + c);
+            if (q2.lo() <= ph.hh && q2.lo() >= ph.eps_r2) move_by(sc.lo(), dx.lo(), dy.lo(), dz.lo());
+            if (q2.hi() <= ph.hh && q2.hi() >= ph.eps_r2) move_by(sc.hi(), dx.hi(), dy.hi(), dz.hi());
+        }
+    }
+    __device__ __forceinline__ void move_by(float f, float kx, float ky, float kz) {
+        px = __fmaf_rn(kx, f, px);
+        py = __fmaf_rn(ky, f, py);
+        pz = __fmaf_rn(kz, f, pz);
+    }
+    // corr_pow of a pair (fast_root asks for the fourth power)
+    template <bool kFast>
+    static __device__ __forceinline__ Two corr(const Phys &ph, const Two &ratio) {
+        if constexpr (kFast) {
+            const Two r2 = ratio * ratio;
+            return r2 * r2;
+        }
+        return Two(corr_pow(ratio.lo(), ph.corr_n), corr_pow(ratio.hi(), ph.corr_n));
+    }
+
+    // The corrected p* after the colliders and the bounds (solver units) in q[3], and
+    // the particle's velocity as they leave it (va: as stored, vel: after a triangle).
+    __device__ __forceinline__ void move(const Phys &ph, const SceneDev &S, const TriDev *tris, const float4 &pa,
+                                         uint32_t a, float4 *__restrict__ v, float *q, float4 &va, float *vel) const {
+        float world[3];
+        if (PROFILE == kRef) {
+            world[0] = (pa.x + px) * S.scale;
+            world[1] = (pa.y + py) * S.scale;
+            world[2] = (pa.z + pz) * S.scale;
+        } else {
+            const float gs = ph.spikyf * ph.inv_rho0;
+            world[0] = (pa.x + px * gs) * S.scale;
+            world[1] = (pa.y + py * gs) * S.scale;
+            world[2] = (pa.z + pz * gs) * S.scale;
+            collide_sphere(S, world);
+        }
+        va = v[a];
+        vel[0] = va.x;
+        vel[1] = va.y;
+        vel[2] = va.z;
+        if (S.tri_count) {
+            collide_triangles(tris, S.tri_first, S.tri_count, world, vel);
+            v[a] = make_float4(vel[0], vel[1], vel[2], va.w);
+        }
+        for (int d = 0; d < 3; ++d) {
+            float w = world[d];
+            w = fmaxf(S.min_b[d], w);
+            w = fminf(S.max_b[d], w);
+            q[d] = w / S.scale;
+        }
+    }
+};
+
+// Final velocity (and, in the ref profile, position) after the step's last correction
+// (oclsph_kernel.h:404-416).
+template <int PROFILE>
+__device__ __forceinline__ void finalise(const Phys &ph, const SceneDev &S, uint32_t a, const float *q,
+                                         const float4 &va, const float *vel, float4 *__restrict__ x,
+                                         float4 *__restrict__ v, const HostParticlesOut *__restrict__ hout) {
+    const float4 xa = x[a];
+    const float xo[3] = {xa.x, xa.y, xa.z};
+    float nv[3], nx[3];
+    for (int d = 0; d < 3; ++d) {
+        const float dd = q[d] - xo[d] / S.scale;
+        if (PROFILE == kRef) {
+            nx[d] = q[d] * S.scale;
+            nv[d] = __fmaf_rn(dd, S.inv_dt, vel[d]) * ph.damping;
+        } else {
+            nv[d] = dd * S.inv_dt;
+        }
+    }
+    v[a] = make_float4(nv[0], nv[1], nv[2], va.w);
+    if (PROFILE == kRef) {
+        x[a] = make_float4(nx[0], nx[1], nx[2], xa.w);
+        store_host_motion(hout, a, x[a], v[a]);
+    }
+}
+
+// Vorticity and the XSPH sum of one particle over its fluid neighbours.
+struct VorticitySum {
+    float o[3] = {0.f, 0.f, 0.f}, xs[3] = {0.f, 0.f, 0.f};
+
+    // vel_b(): the neighbour's velocity
+    template <class V>
+    __device__ __forceinline__ void add(const Phys &ph, const float4 &pa, const float4 &va, float bx, float by,
+                                        float bz, float mb, V &&vel_b) {
+        const float d[3] = {pa.x - bx, pa.y - by, pa.z - bz};
+        const float r2 = dist2(d[0], d[1], d[2]);
+        if (!(r2 <= ph.hh)) return;
+        const float4 vb = vel_b();
+        const float vab[3] = {vb.x - va.x, vb.y - va.y, vb.z - va.z};
+        const float t = ph.hh - r2;
+        const float mw = mb * (t * t * t);
+        xs[0] = __fmaf_rn(mw, vab[0], xs[0]);
+        xs[1] = __fmaf_rn(mw, vab[1], xs[1]);
+        xs[2] = __fmaf_rn(mw, vab[2], xs[2]);
+        const float r = sqrtf(r2);
+        if (r >= kKernelEpsilon) {
+            const float hr = ph.h - r;
+            const float sc = mb * ((hr * hr) / r);
+            float cr[3];
+            cross3(vab, d, cr);
+            o[0] = __fmaf_rn(sc, cr[0], o[0]);
+            o[1] = __fmaf_rn(sc, cr[1], o[1]);
+            o[2] = __fmaf_rn(sc, cr[2], o[2]);
+        }
+    }
+
+    // two neighbours in order, at velocities (ux, uy, uz)
+    template <bool kFast>
+    __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, const float4 &va, const Two &bx,
+                                         const Two &by, const Two &bz, const Two &mb, const Two &ux, const Two &uy,
+                                         const Two &uz) {
+        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
+        const Two q2 = dist2(dx, dy, dz);
+        Two r, s;
+        root_and_spiky<kFast>(ph, q2, r, s);
+        const Two vx = ux - Two(va.x), vy = uy - Two(va.y), vz = uz - Two(va.z);
+        const Two t = Two(ph.hh) - q2, mw = mb * (t * t * t), sc = mb * s;
+        const Two cx = times(ph, vy, dz) - times(ph, vz, dy), cy = times(ph, vz, dx) - times(ph, vx, dz),
+                  cz = times(ph, vx, dy) - times(ph, vy, dx);
+        one(ph, q2.lo(), mw.lo(), vx.lo(), vy.lo(), vz.lo(), sc.lo(), cx.lo(), cy.lo(), cz.lo());
+        one(ph, q2.hi(), mw.hi(), vx.hi(), vy.hi(), vz.hi(), sc.hi(), cx.hi(), cy.hi(), cz.hi());
+    }
+    __device__ __forceinline__ void one(const Phys &ph, float q2, float mw, float vx, float vy, float vz, float sc,
+                                        float cx, float cy, float cz) {
+        if (!(q2 <= ph.hh)) return;
+        xs[0] = __fmaf_rn(mw, vx, xs[0]);
+        xs[1] = __fmaf_rn(mw, vy, xs[1]);
+        xs[2] = __fmaf_rn(mw, vz, xs[2]);
+        if (q2 >= ph.eps_r2) {
+            o[0] = __fmaf_rn(sc, cx, o[0]);
+            o[1] = __fmaf_rn(sc, cy, o[1]);
+            o[2] = __fmaf_rn(sc, cz, o[2]);
+        }
+    }
+
+    // omega with |omega| in w, pom (p* with |omega| in w; null: not kept) and vx
+    __device__ __forceinline__ void finish(const Phys &ph, uint32_t a, const float4 &pa, const float4 &va,
+                                           float4 *__restrict__ omega, float4 *__restrict__ pom,
+                                           float4 *__restrict__ vx) const {
+        const float gs = ph.spikyf * ph.inv_rho0;
+        const float ws = ph.poly6f * ph.inv_rho0;
+        // omega = sum_b m_b / rho0 (v_b - v_a) x grad_b W(x_a - x_b), and grad_b W = -grad_a W
+        // = -spikyf (h - r)^2 d / r: the sum o carries grad_a's factor, so its sign flips
+        const float ox = -(o[0] * gs), oy = -(o[1] * gs), oz = -(o[2] * gs);
+        const float om = sqrtf(ox * ox + oy * oy + oz * oz);
+        omega[a] = make_float4(ox, oy, oz, om);
+        if (pom) pom[a] = make_float4(pa.x, pa.y, pa.z, om);
+        vx[a] = make_float4(__fmaf_rn(ph.xsph_c, xs[0] * ws, va.x), __fmaf_rn(ph.xsph_c, xs[1] * ws, va.y),
+                            __fmaf_rn(ph.xsph_c, xs[2] * ws, va.z), va.w);
+    }
+};
+
+// eta = grad |omega| of one particle over its fluid neighbours, and the step's end:
+// N = eta / |eta|, f = eps (N x omega), v = vx + dt f, x = p*.
+struct ApplySum {
+    float e[3] = {0.f, 0.f, 0.f};
+
+    // oa: the particle's |omega|; om_b(): the neighbour's
+    template <class O>
+    __device__ __forceinline__ void add(const Phys &ph, const float4 &pa, float oa, float bx, float by, float bz,
+                                        O &&om_b, float mb) {
+        const float d[3] = {pa.x - bx, pa.y - by, pa.z - bz};
+        const float r2 = dist2(d[0], d[1], d[2]);
+        if (!(r2 <= ph.hh)) return;
+        const float r = sqrtf(r2);
+        if (!(r >= kKernelEpsilon)) return;
+        const float hr = ph.h - r;
+        const float sc = mb * ((hr * hr) / r) * (om_b() - oa);
+        e[0] = __fmaf_rn(sc, d[0], e[0]);
+        e[1] = __fmaf_rn(sc, d[1], e[1]);
+        e[2] = __fmaf_rn(sc, d[2], e[2]);
+    }
+
+    // two neighbours in order, their |omega| in ob
+    template <bool kFast>
+    __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, float oa, const Two &bx, const Two &by,
+                                         const Two &bz, const Two &ob, const Two &mb) {
+        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
+        const Two q2 = dist2(dx, dy, dz);
+        Two r, s;
+        root_and_spiky<kFast>(ph, q2, r, s);
+        const Two sc = mb * s * (ob - Two(oa));
+        if (q2.lo() <= ph.hh && q2.lo() >= ph.eps_r2) one(sc.lo(), dx.lo(), dy.lo(), dz.lo());
+        if (q2.hi() <= ph.hh && q2.hi() >= ph.eps_r2) one(sc.hi(), dx.hi(), dy.hi(), dz.hi());
+    }
+    __device__ __forceinline__ void one(float sc, float dx, float dy, float dz) {
+        e[0] = __fmaf_rn(sc, dx, e[0]);
+        e[1] = __fmaf_rn(sc, dy, e[1]);
+        e[2] = __fmaf_rn(sc, dz, e[2]);
+    }
+
+    __device__ __forceinline__ void finish(const Phys &ph, const SceneDev &S, uint32_t a, const float4 &pa,
+                                           const float4 &oa, const float4 *__restrict__ vx, float4 *__restrict__ v,
+                                           float4 *__restrict__ x, const HostParticlesOut *__restrict__ hout) const {
+        const float gs = ph.spikyf * ph.inv_rho0;
+        const float ex = e[0] * gs, ey = e[1] * gs, ez = e[2] * gs;
+        const float el = sqrtf(ex * ex + ey * ey + ez * ez);
+        float N[3] = {0.f, 0.f, 0.f};
+        if (el > 0.f) {
+            N[0] = ex / el;
+            N[1] = ey / el;
+            N[2] = ez / el;
+        }
+        const float om[3] = {oa.x, oa.y, oa.z};
+        float f[3];
+        cross3(N, om, f);
+        const float4 vxa = vx[a];
+        const float ve = ph.vort_eps, dt = S.dt;
+        const float4 vn = make_float4(__fmaf_rn(dt, f[0] * ve, vxa.x), __fmaf_rn(dt, f[1] * ve, vxa.y),
+                                      __fmaf_rn(dt, f[2] * ve, vxa.z), vxa.w);
+        v[a] = vn;
+        const float4 xa = x[a];
+        const float4 xn = make_float4(pa.x * S.scale, pa.y * S.scale, pa.z * S.scale, xa.w);
+        x[a] = xn;
+        store_host_motion(hout, a, xn, vn);
+    }
+};
+
+}  // namespace fgb

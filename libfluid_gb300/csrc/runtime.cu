@@ -35,6 +35,7 @@
 #include <sys/mman.h>
 #include <unistd.h>
 
+#include "fast_root.h"
 #include "fgb_internal.h"
 
 namespace fgb {
@@ -202,6 +203,9 @@ uint32_t bits_for(uint32_t v) {
     return b;
 }
 
+// The smallest float T with sqrtf(T) >= thr (below).
+float sqrt_lt_bound(float thr);
+
 Phys make_phys(const fgb_params &p) {
     Phys ph{};
     const float h = p.h, hh = h * h, hhh = h * h * h;
@@ -240,6 +244,9 @@ Phys make_phys(const fgb_params &p) {
     ph.mc_size = p.mc_particle_size;
     ph.mc_infl = p.mc_particle_influence;
     ph.profile = p.profile;
+    ph.eps_r2 = sqrt_lt_bound(kKernelEpsilon);
+    ph.minus_zero = -0.f;
+    ph.fast_root = fast_root_exact(ph);
     return ph;
 }
 
@@ -267,6 +274,7 @@ void scene_geometry(const fgb_params &p, const fgb_config &c, SceneDev &S) {
         uint32_t ei = e > 0.f ? (uint32_t)e : 0u;
         if (ei > 1023u) ei = 1023u;
         S.ext[a] = ei;
+        S.ext_code[a] = spread10(ei) << a;
     }
     S.dt = c.dt;
     S.inv_dt = 1.f / c.dt;
@@ -455,6 +463,8 @@ static constexpr uint64_t kPieceMin = 1u << 18;
 static constexpr uint32_t kMaxRowCap = 1024;  // Verlet and hit rows, entries per particle
 static constexpr uint32_t kPieces = 4;
 
+static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu
+
 // Autotuner cache key: physics profile and floor(log2(particles)).
 static uint32_t tune_bucket(int32_t profile, uint64_t n) {
     uint32_t b = 0;
@@ -481,7 +491,11 @@ struct fgb_solver {
     std::map<uint32_t, Tuned> tuned;
     // row capacities (Verlet, hit) that batches grew to, per (profile, log2 n) bucket:
     // later batches of the bucket start there
-    std::map<uint32_t, std::pair<uint32_t, uint32_t>> caps;
+    struct Caps {
+        uint32_t list, hit;
+    };
+    std::map<uint32_t, Caps> caps;
+    std::map<uint32_t, uint32_t> cell_caps;  // the same for the hit rows of rows.cu
     fgb_batch *cached = nullptr;  // single-scene batch behind fgb_advance
     uint64_t cached_n = 0;
     fgb_config cached_cfg{};
@@ -573,6 +587,14 @@ struct fgb_batch {
     float near_frac = 0.05f;  // near-row skin, fraction of h (0: near rows off)
     Dev<uint8_t> near;
     int block = 128;  // threads per CTA of the gather kernels
+    // the gathers run on hit rows from one warp per cell (rows.cu), else on the list
+    // kernels (pbf.cu)
+    bool cell_rows = false;
+    uint32_t cell_hits = 96;  // entries of a hit row of rows.cu
+    uint32_t group_mask = 31;
+    Dev<uint32_t> groups, group_count, moved;
+    Dev<uint8_t> lasting;
+    Dev<RowPolicy> row_policy[2];  // by the state set a step reads
     Dev<float> lambda, density;
     Dev<float4> plam;             // the lambda pass's p* with lambda in w (delta reads)
     Dev<float4> pom;              // the vorticity pass's p* with |omega| in w (apply reads)
@@ -698,6 +720,14 @@ struct fgb_batch {
         s.near_skin = near_skin;
         s.hout = advance_io ? hout_dev.p : nullptr;
         s.over = over.p;
+        s.groups = cell_rows ? groups.p : nullptr;
+        s.group_count = group_count.p;
+        s.group_mask = group_mask;
+        s.moved = moved.p;
+        s.lasting = lasting.p;
+        s.row_policy = row_policy[c].p;
+        s.row_policy_next = row_policy[c ^ 1].p;
+        if (cell_rows) s.hcap = cell_hits;
         s.near_stats = row_stats && over.p ? over.p + 2 : nullptr;
         return s;
     }
@@ -732,11 +762,14 @@ struct fgb_batch {
         mark(k, st);
         if (io_up) FGB_CUDA(cudaStreamWaitEvent(st, io_up, cudaEventWaitExternal), "step: upload event");
         FGB_CUDA(cudaMemsetAsync(cells.p, 0, cells_n * sizeof(uint2), st), "step: clear cells");
-        if (persistent)
+        if (persistent && !cell_rows)
             FGB_CUDA(cudaMemsetAsync(queue.p, 0, slots_of_step(iterations) * sizeof(uint32_t), st),
                      "step: clear tile counters");
         FGB_CUDA(cudaMemsetAsync(mass_range.p, 0xff, 2 * sizeof(uint32_t), st), "step: clear mass range");
-        if (cellmax.p) FGB_CUDA(cudaMemsetAsync(cellmax.p, 0, cells_n * sizeof(uint32_t), st), "step: clear cellmax");
+        if (cell_rows)
+            FGB_CUDA(cudaMemsetAsync(group_count.p, 0, sizeof(uint32_t), st), "step: clear group count");
+        if (s.cap && cellmax.p)
+            FGB_CUDA(cudaMemsetAsync(cellmax.p, 0, cells_n * sizeof(uint32_t), st), "step: clear cellmax");
         launch_reorder_cells(s, st);
         l += 1;
         if (ph.profile == FGB_PROFILE_REF) {
@@ -749,13 +782,22 @@ struct fgb_batch {
         const float4 *pin = ps_grid.p;
         for (uint32_t it = 0; it < iterations; ++it) {
             float4 *pout = ps[it & 1].p;
+            if (cell_rows) {
+                FGB_CUDA(launch_row_lambda(s, pin, (int)it, st), "step: lambda rows");
+                mark(k, st);
+                FGB_CUDA(launch_row_delta(s, pin, pout, it + 1 == iterations, st), "step: delta rows");
+                mark(k, st);
+                l += 3;
+                pin = pout;
+                continue;
+            }
             launch_lambda(s, pin, (int)it, st);  // the first also builds the Verlet lists (two kernels)
             mark(k, st);
             // the list bound at the next pass needs the neighbours' displacement at that
             // pass only: the cell maxima restart at every delta pass (the step's first
             // starts from the clear above), so an iteration that overshoots does not keep
             // lists invalid after the next one has moved the particles back
-            if (it > 0 && cellmax.p)
+            if (it > 0 && s.cap && cellmax.p)
                 FGB_CUDA(cudaMemsetAsync(cellmax.p, 0, cells_n * sizeof(uint32_t), st), "step: clear cellmax");
             launch_delta(s, pin, pout, (int)it, it + 1 == iterations, st);
             mark(k, st);
@@ -763,9 +805,12 @@ struct fgb_batch {
             pin = pout;
         }
         if (ph.profile != FGB_PROFILE_REF) {
-            launch_velocity_terms(s, pin, st, [&] { mark(k, st); });
+            if (cell_rows)
+                FGB_CUDA(launch_row_velocity_terms(s, pin, st, [&] { mark(k, st); }), "step: velocity rows");
+            else
+                launch_velocity_terms(s, pin, st, [&] { mark(k, st); });
             mark(k, st);
-            l += 2;
+            l += cell_rows ? 3 : 2;
         }
         if (s.list_policy && s.cap) {
             launch_list_policy(s, st);
@@ -969,6 +1014,16 @@ struct fgb_batch {
     int grow_rows() {
         if (!st_over.p) return FGB_OK;
         const uint64_t lim = std::max<uint64_t>(n / 100, 1);
+        if (cell_rows) {
+            // a row that overflowed holds up its warp's other rows: hardly any may
+            if (st_over.p[1] <= n / 5000 || cell_hits >= kMaxCellHits) return FGB_OK;
+            FGB_CUDA(cudaStreamSynchronize(stream()), "grow hit rows sync");
+            cell_hits = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 1) & ~1u);
+            st_over.p[0] = st_over.p[1] = 0;
+            drop_graphs();
+            solver->cell_caps[tune_bucket(solver->params.profile, n)] = cell_hits;
+            return alloc_cell_rows(capacity ? capacity : n);
+        }
         const bool gl = list_cap && st_over.p[0] > lim && list_cap < kMaxRowCap;
         const bool gh = hit_cap && st_over.p[1] > lim && hit_cap < kMaxRowCap;
         if (!gl && !gh) return FGB_OK;
@@ -988,7 +1043,23 @@ struct fgb_batch {
         for (auto &g : graph)
             if (g) cudaGraphExecDestroy(g), g = nullptr;
         graphs_ok = false;
-        solver->caps[tune_bucket(solver->params.profile, n)] = {list_cap, hit_cap};
+        solver->caps[tune_bucket(solver->params.profile, n)] = fgb_solver::Caps{list_cap, hit_cap};
+        return FGB_OK;
+    }
+
+    void drop_graphs() {
+        for (auto &g : graph)
+            if (g) cudaGraphExecDestroy(g), g = nullptr;
+        graphs_ok = false;
+    }
+
+    // The hit rows of rows.cu for cap particles, interleaved by 32 of them.  Every row
+    // starts as overflowed: one that a step did not write is never read.
+    int alloc_cell_rows(uint64_t cap) {
+        PoolScope scope(&solver->pool);
+        FGB_CUDA(hlist.alloc((cap + 31) / 32 * 32 * cell_hits), "hit rows");
+        FGB_CUDA(hcount.alloc(cap), "hit rows");
+        FGB_CUDA(cudaMemsetAsync(hcount.p, 0xff, cap * sizeof(uint16_t), stream()), "hit rows");
         return FGB_OK;
     }
 
@@ -1158,6 +1229,16 @@ static bool packed_off() {
     return e && strcmp(e, "0") == 0;
 }
 
+// Settings of the list kernels (pbf.cu) that ask for them: a caller that sets one gets the kernels
+// it is about.
+static bool list_kernels_asked() {
+    for (const char *name : {"FGB_VERLET", "FGB_NEAR_SKIN", "FGB_LIST_CAP", "FGB_HIT_CAP", "FGB_LIST_SKIN",
+                             "FGB_LIST_POLICY", "FGB_LIST_MIN_USE", "FGB_PERSISTENT", "FGB_PPT", "FGB_PACKED",
+                             "FGB_ROW_STATS"})
+        if (getenv(name)) return true;
+    return false;
+}
+
 static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     PoolScope scope(&b->solver->pool);
     const fgb_params &p = b->solver->params;
@@ -1169,23 +1250,32 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     b->sort_scratch_bytes = radix_scratch_bytes(cap);
     FGB_CUDA(b->sort_scratch.alloc(b->sort_scratch_bytes), "batch alloc");
     FGB_CUDA(b->ps_grid.alloc(cap), "batch alloc");
-    if (b->list_cap) {
+    if (b->cell_rows) {
+        FGB_CUDA(b->groups.alloc(cap), "batch alloc groups");
+        FGB_CUDA(b->lasting.alloc(cap), "batch alloc groups");
+        FGB_CUDA(b->moved.alloc(cap), "batch alloc groups");
+        FGB_CUDA(b->group_count.alloc(1), "batch alloc groups");
+        int rc = b->alloc_cell_rows(cap);
+        if (rc) return rc;
+    }
+    if (!b->cell_rows && b->list_cap) {
+        FGB_CUDA(b->cellmax.alloc(std::max<uint64_t>(b->cells_n, 1)), "batch alloc");
         FGB_CUDA(b->nlist.alloc(cap * b->list_cap), "batch alloc neighbour lists");
         FGB_CUDA(b->ncount.alloc(cap), "batch alloc");
         FGB_CUDA(b->disp.alloc(cap), "batch alloc");
         FGB_CUDA(b->valid.alloc(cap), "batch alloc");
     }
-    if (b->hit_cap) {
+    if (!b->cell_rows && b->hit_cap) {
         FGB_CUDA(b->hlist.alloc(cap * b->hit_cap), "batch alloc hit lists");
         FGB_CUDA(b->hcount.alloc(cap), "batch alloc");
     }
-    if (b->list_cap && b->hit_cap) FGB_CUDA(b->near.alloc(cap), "batch alloc");
+    if (!b->cell_rows && b->list_cap && b->hit_cap) FGB_CUDA(b->near.alloc(cap), "batch alloc");
     FGB_CUDA(b->lambda.alloc(cap), "batch alloc");
-    if (!packed_off()) FGB_CUDA(b->plam.alloc(cap), "batch alloc");
+    if (b->cell_rows || !packed_off()) FGB_CUDA(b->plam.alloc(cap), "batch alloc");
     FGB_CUDA(b->mass_range.alloc(2), "batch alloc");
     FGB_CUDA(b->density.alloc(cap), "batch alloc");
     if (p.profile != FGB_PROFILE_REF) {
-        if (!packed_off()) FGB_CUDA(b->pom.alloc(cap), "batch alloc");
+        if (b->cell_rows || !packed_off()) FGB_CUDA(b->pom.alloc(cap), "batch alloc");
         FGB_CUDA(b->omega.alloc(cap), "batch alloc");
         FGB_CUDA(b->vx.alloc(cap), "batch alloc");
     } else {
@@ -1288,8 +1378,8 @@ static int batch_init(fgb_batch *b) {
     {
         auto it = s->caps.find(tune_bucket(p.profile, n));
         if (it != s->caps.end()) {
-            b->list_cap = it->second.first;
-            b->hit_cap = it->second.second;
+            b->list_cap = it->second.list;
+            b->hit_cap = it->second.hit;
         }
     }
     if (const char *e = getenv("FGB_LIST_CAP")) b->list_cap = (uint32_t)atoi(e);
@@ -1323,17 +1413,29 @@ static int batch_init(fgb_batch *b) {
     }
     if (b->list_cap > 4096) b->list_cap = 4096;
     b->list_cap = (b->list_cap + 3u) & ~3u;  // rows move as 16-byte vectors
-    if (b->list_cap) FGB_CUDA(b->cellmax.alloc(std::max<uint64_t>(table, 1)), "batch alloc");
     if (const char *e = getenv("FGB_HIT_CAP")) b->hit_cap = (uint32_t)atoi(e);
     if (const char *e = getenv("FGB_NEAR_SKIN")) b->near_frac = (float)atof(e);
     if (b->hit_cap > 4096) b->hit_cap = 4096;
     b->hit_cap = (b->hit_cap + 3u) & ~3u;  // rows move as 16-byte vectors
+    if (!list_kernels_asked()) {
+        b->cell_rows = true;
+        b->group_mask = row_group_mask(p.profile, n);
+        const std::vector<RowPolicy> init(b->n_scenes, RowPolicy{1, 0, 0, 0});  // the first step keeps the skin
+        for (auto &pol : b->row_policy) {
+            FGB_CUDA(pol.alloc(b->n_scenes), "batch alloc");
+            FGB_CUDA(cudaMemcpy(pol.p, init.data(), init.size() * sizeof(RowPolicy), cudaMemcpyHostToDevice),
+                     "batch alloc");
+        }
+        if (p.profile == FGB_PROFILE_REF) b->cell_hits = 256;  // its constants clump the fluid
+        auto it = s->cell_caps.find(tune_bucket(p.profile, n));
+        if (it != s->cell_caps.end()) b->cell_hits = it->second;
+    }
     int rc = alloc_step_arrays(b, n);
     if (rc) return rc;
     FGB_CUDA(b->err.alloc(1), "batch alloc");
     FGB_CUDA(b->st_flags.ensure(1), "batch alloc");
     b->st_flags.p[0] = 0;
-    if (b->list_cap || b->hit_cap) {
+    if (b->cell_rows || b->list_cap || b->hit_cap) {
         FGB_CUDA(b->over.alloc(6), "batch alloc");
         FGB_CUDA(cudaMemset(b->over.p, 0, 6 * sizeof(uint32_t)), "batch alloc");
         const char *e = getenv("FGB_ROW_STATS");
@@ -2050,6 +2152,11 @@ int fgb_batch_probe(fgb_batch *b, uint32_t what, void *host_out, uint64_t bytes)
     case FGB_PROBE_LIST_VALID: src = b->valid.p; break;
     case FGB_PROBE_DISPLACEMENT: src = b->disp.p; break;
     case FGB_PROBE_NEAR_ROW: src = b->near.p; break;
+    }
+    if (b->cell_rows && what >= FGB_PROBE_LIST_COUNT && what <= FGB_PROBE_NEAR_ROW) {
+        // the kernels of rows.cu keep no lists or near rows: every list is overflowed, none valid
+        memset(host_out, what == FGB_PROBE_LIST_COUNT ? 0xff : 0, bytes);
+        return FGB_OK;
     }
     if (!src) return fail(FGB_ERR_INVALID, "probe: array not allocated yet");
     cudaStream_t st = b->stream();
