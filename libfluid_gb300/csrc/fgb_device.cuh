@@ -63,7 +63,6 @@ struct Phys {
     float h, hh;
     float hh_le;      // the largest float r2 with sqrtf(r2) <= h: r2 <= hh_le is exactly sqrtf(r2) <= h
     float eps_r2;     // the smallest float r2 with sqrtf(r2) >= 1e-8: r >= the kernels' epsilon
-    float minus_zero; // -0.f (pbf_sums.cuh: times)
     int fast_root;    // the pair sums may take root and quotient by root_and_spiky's fast form
     float poly6f;     // 315 / (64 pi h^9)
     float spikyf;     // -45 / (pi h^6)

@@ -116,43 +116,26 @@ __device__ __forceinline__ void cross3(const float *a, const float *b, float *o)
 }
 
 
-// Two floats in one 64-bit register pair, for the packed add, mul and fma (each half
-// rounds as the scalar operation does).
+// A value for each of two neighbours.  The pair form lets their roots and quotients run
+// beside each other.  (The packed add, mul and fma of two floats issue at half the rate of
+// the scalar ones here, 1.65 against 3.73 a clock and SM, and their register pairs cost
+// moves: the delta pass takes 112 us with scalar operations and 117 with packed ones, and
+// ptxas fuses a packed product with the sum that follows, which changes its bits.)
 struct Two {
-    uint64_t v;
+    float a, b;
     __device__ __forceinline__ Two() {}
-    __device__ __forceinline__ explicit Two(uint64_t v_) : v(v_) {}
-    __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-    __device__ __forceinline__ explicit Two(float a) : Two(a, a) {}
-    __device__ __forceinline__ float lo() const { return __uint_as_float((uint32_t)v); }
-    __device__ __forceinline__ float hi() const { return __uint_as_float((uint32_t)(v >> 32)); }
+    __device__ __forceinline__ Two(float a_, float b_) : a(a_), b(b_) {}
+    __device__ __forceinline__ explicit Two(float v) : a(v), b(v) {}
+    __device__ __forceinline__ float lo() const { return a; }
+    __device__ __forceinline__ float hi() const { return b; }
 };
-__device__ __forceinline__ Two operator-(const Two &a, const Two &b) {
-    Two r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
+__device__ __forceinline__ Two operator-(const Two &x, const Two &y) { return Two(x.a - y.a, x.b - y.b); }
+__device__ __forceinline__ Two operator+(const Two &x, const Two &y) { return Two(x.a + y.a, x.b + y.b); }
+__device__ __forceinline__ Two operator*(const Two &x, const Two &y) { return Two(x.a * y.a, x.b * y.b); }
+__device__ __forceinline__ Two operator-(const Two &x) { return Two(-x.a, -x.b); }
+__device__ __forceinline__ Two fma(const Two &x, const Two &y, const Two &z) {
+    return Two(__fmaf_rn(x.a, y.a, z.a), __fmaf_rn(x.b, y.b, z.b));
 }
-__device__ __forceinline__ Two operator+(const Two &a, const Two &b) {
-    Two r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ Two operator*(const Two &a, const Two &b) {
-    Two r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ Two fma(const Two &a, const Two &b, const Two &c) {
-    Two r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ Two operator-(const Two &a) { return Two(-a.lo(), -a.hi()); }
-// A product that a sum or a difference takes up: ptxas fuses mul.rn.f32x2 with the add
-// that follows (it leaves the scalar form alone), so the product is a multiply-add of
-// minus zero, which rounds as the product does; the zero comes from the kernel's
-// arguments, where the compiler does not know it.
-__device__ __forceinline__ Two times(const Phys &ph, const Two &a, const Two &b) { return fma(a, b, Two(ph.minus_zero)); }
 // r^2 of a pair of neighbours, as dist2
 __device__ __forceinline__ Two dist2(const Two &dx, const Two &dy, const Two &dz) {
     return fma(dx, dx, fma(dy, dy, dz * dz));
@@ -175,8 +158,8 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // reciprocal's error is below 2^-43 before its rounding, so it can be misrounded only for
 // the few mantissas whose reciprocals lie that near the midpoint of two floats; the host
 // checks the quotients of those for the solver's h (fast_root.h) and
-// clears fast_root if one fails.  17 packed operations for two neighbours, where the
-// compiler's root and quotient take about 60 instructions with their range checks.
+// clears fast_root if one fails.  17 operations a neighbour, where the compiler's
+// root and quotient take about 30 with their range checks.
 // Below q2 = 1e-30 (only there does the approximation leave the normal range) r is
 // meaningless; its users drop s below eps_r2.
 template <bool kFast>
@@ -255,9 +238,9 @@ struct LambdaSum {
         const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
         Two r, s;
         if (PROFILE == kRef) {
-            const Two q2 = (times(ph, dx, dx) + times(ph, dy, dy)) + times(ph, dz, dz);
+            const Two q2 = (dx * dx + dy * dy) + dz * dz;
             root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - times(ph, r, r), w = Two(ph.poly6f) * (t * t * t);
+            const Two t = Two(ph.hh) - r * r, w = Two(ph.poly6f) * (t * t * t);
             const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;
             one<kFast>(ph, pa, q2.lo(), w.lo(), kx.lo(), ky.lo(), kz.lo());
             one<kFast>(ph, pa, q2.hi(), w.hi(), kx.hi(), ky.hi(), kz.hi());
@@ -365,11 +348,11 @@ struct DeltaSum {
         const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
         Two r, s, k;
         if (PROFILE == kRef) {
-            const Two q2 = (times(ph, dx, dx) + times(ph, dy, dy)) + times(ph, dz, dz);
+            const Two q2 = (dx * dx + dy * dy) + dz * dz;
             root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - times(ph, r, r), w = Two(ph.poly6f) * (t * t * t);
+            const Two t = Two(ph.hh) - r * r, w = Two(ph.poly6f) * (t * t * t);
             const Two c =
-                times(ph, Two(-ph.corr_k), corr<kFast>(ph, over_const<kFast>(w, ph.corr_ref, ph.inv_corr_ref)));
+                Two(-ph.corr_k) * corr<kFast>(ph, over_const<kFast>(w, ph.corr_ref, ph.inv_corr_ref));
             const Two sum = (Two(la) + lb) + c;
             Two f = over_const<kFast>(sum, ph.rho0, ph.inv_rho0);
             if (kFast) {
@@ -385,7 +368,7 @@ struct DeltaSum {
             const Two q2 = dist2(dx, dy, dz);
             root_and_spiky<kFast>(ph, q2, r, s);
             const Two t = Two(ph.hh) - q2;
-            const Two c = times(ph, Two(-ph.corr_k), corr<kFast>(ph, (t * t * t) * Two(ph.inv_corr_wdq)));
+            const Two c = Two(-ph.corr_k) * corr<kFast>(ph, (t * t * t) * Two(ph.inv_corr_wdq));
             const Two sc = mb * s * ((Two(la) + lb) + c);
             if (q2.lo() <= ph.hh && q2.lo() >= ph.eps_r2) move_by(sc.lo(), dx.lo(), dy.lo(), dz.lo());
             if (q2.hi() <= ph.hh && q2.hi() >= ph.eps_r2) move_by(sc.hi(), dx.hi(), dy.hi(), dz.hi());
@@ -505,8 +488,8 @@ struct VorticitySum {
         root_and_spiky<kFast>(ph, q2, r, s);
         const Two vx = ux - Two(va.x), vy = uy - Two(va.y), vz = uz - Two(va.z);
         const Two t = Two(ph.hh) - q2, mw = mb * (t * t * t), sc = mb * s;
-        const Two cx = times(ph, vy, dz) - times(ph, vz, dy), cy = times(ph, vz, dx) - times(ph, vx, dz),
-                  cz = times(ph, vx, dy) - times(ph, vy, dx);
+        const Two cx = vy * dz - vz * dy, cy = vz * dx - vx * dz,
+                  cz = vx * dy - vy * dx;
         one(ph, q2.lo(), mw.lo(), vx.lo(), vy.lo(), vz.lo(), sc.lo(), cx.lo(), cy.lo(), cz.lo());
         one(ph, q2.hi(), mw.hi(), vx.hi(), vy.hi(), vz.hi(), sc.hi(), cx.hi(), cy.hi(), cz.hi());
     }

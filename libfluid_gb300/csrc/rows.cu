@@ -16,8 +16,8 @@
 // a violent flow it fails nearly everywhere and the longer rows are wasted: the step before
 // tells, per scene, whether they are worth keeping (RowPolicy).
 //
-// The passes (k_row_*) run one thread per particle over its row, two neighbours at a time
-// in packed float pairs, the neighbours' data through L1.  Every pass tests its range
+// The passes (k_row_*) run one thread per particle over its row, two neighbours at a time,
+// the neighbours' data through L1.  Every pass tests its range
 // again, so the sums are those of the 27-cell walk of pbf.cu, bit for bit.
 #include <algorithm>
 #include <cstdint>

@@ -245,7 +245,6 @@ Phys make_phys(const fgb_params &p) {
     ph.mc_infl = p.mc_particle_influence;
     ph.profile = p.profile;
     ph.eps_r2 = sqrt_lt_bound(kKernelEpsilon);
-    ph.minus_zero = -0.f;
     ph.fast_root = fast_root_exact(ph);
     return ph;
 }
