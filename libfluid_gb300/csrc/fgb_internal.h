@@ -116,6 +116,7 @@ struct StepView {
     // the gathers run on the hit rows of rows.cu, else (null) on the list kernels of
     // pbf.cu: the first particle of every group -- a cell's particles up to where the
     // index under group_mask wraps -- and the groups' number (zeroed every step)
+    uint32_t none;  // the entry past the particles that lies at infinity: what fills a hit row's last quad
     uint32_t *groups, *group_count, group_mask;
     uint32_t *moved;       // per particle: at a cell's first, the largest movement in the cell
     uint8_t *lasting;      // per group

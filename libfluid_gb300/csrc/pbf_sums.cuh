@@ -358,7 +358,8 @@ struct DeltaSum {
             if (kFast) {
                 // outside over_const's range (a sum that cancelled, or one that ran away)
                 const float s0 = fabsf(sum.lo()), s1 = fabsf(sum.hi());
-                if (!(fminf(s0, s1) > 1e-27f && fmaxf(s0, s1) < 1e27f))
+                if ((q2.lo() <= ph.hh_le && !(s0 > 1e-27f && s0 < 1e27f)) ||
+                    (q2.hi() <= ph.hh_le && !(s1 > 1e-27f && s1 < 1e27f)))
                     f = Two(sum.lo() / ph.rho0, sum.hi() / ph.rho0);
             }
             const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;

@@ -40,9 +40,11 @@ struct RowArgs {
     const uint32_t *groups;      // first particle of every group, in no particular order
     const uint32_t *group_count;
     uint32_t group_mask;         // a group ends with its cell or where index & mask wraps
-    uint2 *hrows;                // hit rows, see row_of
+    uint4 *hrows;                // hit rows, see row_of
     uint16_t *hcount;
-    uint32_t hcap;               // entries a hit row has room for (even)
+    uint32_t hcap;               // entries a hit row has room for (a multiple of four)
+    uint32_t none;               // the index that fills a row's last quad: the far entry past the particles
+    int fetch;                   // the passes ask for their rows ahead (fetch_rows)
     const uint32_t *mass_range;
     uint32_t *over;              // hit rows that overflowed (null: not counted)
     const float4 *ps_grid;       // the grid positions
@@ -53,21 +55,23 @@ struct RowArgs {
     RowPolicy *policy_next;
 };
 
-// A particle's hit row: its i-th pair at [32 i].  Rows of 32 consecutive particles interleave.
-__device__ __forceinline__ uint2 *row_of(const RowArgs &A, uint32_t a) {
-    return A.hrows + (size_t)(a >> 5) * (A.hcap >> 1) * 32 + (a & 31u);
+// A particle's hit row: its i-th four entries at [32 i].  Rows of 32 consecutive particles
+// interleave.
+__device__ __forceinline__ uint4 *row_of(const RowArgs &A, uint32_t a) {
+    return A.hrows + (size_t)(a >> 5) * (A.hcap >> 2) * 32 + (a & 31u);
 }
 
 constexpr uint32_t kCellBlock = 128, kCellWarps = kCellBlock / 32;
+constexpr uint32_t kFetchFrom = 400000;   // particles from which the passes ask for their rows ahead
 constexpr float kRowSkin = 0.1f;          // the skin of rows that last, in h
 constexpr uint32_t kHeld = 8;             // candidates a lane holds at a time
 constexpr uint32_t kHeldAll = 32 * kHeld;  // candidates a warp holds
 constexpr uint32_t kGroup = 4;            // particles whose hits are collected before they are written
-constexpr uint32_t kPitch = kHeldAll + 2;
+constexpr uint32_t kPitch = kHeldAll + 8;  // room to fill the last quad; the four lists in different banks
 
 struct CellShared {
-    uint32_t map[kHeldAll];               // sorted indices of the candidates held
-    uint32_t hits[kGroup * kPitch];  // hits of a group's particles among them, in order
+    uint32_t map[kHeldAll];                         // sorted indices of the candidates held
+    alignas(16) uint32_t hits[kGroup * kPitch];  // hits of a group's particles among them, in order
 };
 
 // The lane's neighbour cell of the cell with Morton code m: its table index, or false
@@ -108,6 +112,10 @@ __device__ __forceinline__ void append_hits(float r2, uint32_t b, uint32_t befor
         : "+r"(to)
         : "f"(r2), "r"(b), "r"(before)
         : "memory");
+}
+
+__device__ __forceinline__ void fill(uint32_t at, uint32_t b) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(b) : "memory");
 }
 
 // Whether this step's first search keeps the skin for a scene: it did in the step before
@@ -236,6 +244,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
                     for (uint32_t j = four; j < last; ++j) {
                         if (obstacles && A.type[first + j] == FGB_TYPE_OBSTACLE) continue;  // no sums: an empty row
                         const uint32_t list = lists + 4 * (j - four) * kPitch, to = test(rounds, first + j, list);
+                        if (lane < 3) fill(to + 4 * lane, A.none);
                         if (lane == j) found += (to - list) >> 2;
                     }
                 };
@@ -247,20 +256,19 @@ __global__ void __launch_bounds__(kCellBlock, 7)
                 default: each(Rounds<4>{}); break;
                 }
                 __syncwarp();
-                // the four's hits to their rows: lane 4 p + j takes pair p of the j-th
-                const uint32_t j = four + (lane & 3u), a = first + j;
+                // the four's hits to their rows: lane 4 p + j takes quad p of the j-th
+                const uint32_t j = four + (lane & 3u);
                 const uint32_t lo = __shfl_sync(0xffffffffu, earlier, j),
                                hi = min(__shfl_sync(0xffffffffu, found, j), A.hcap);
                 if (j >= own) continue;
                 const uint32_t *have = sh.hits + (lane & 3u) * kPitch;
-                if ((lo & 1u) == 0) {
-                    uint32_t e = lo + 2 * (lane >> 2);
-                    const uint2 *p = reinterpret_cast<const uint2 *>(have + (e - lo));
-                    uint2 *row = row_of(A, a) + (e >> 1) * 32;
-                    for (; e < hi; e += 16, p += 8, row += 8 * 32) *row = *p;
-                } else {  // a later segment that starts within a pair
-                    uint32_t *row = reinterpret_cast<uint32_t *>(row_of(A, a));
-                    for (uint32_t e = lo + (lane >> 2); e < hi; e += 8) row[(e >> 1) * 64 + (e & 1u)] = have[e - lo];
+                uint4 *row = row_of(A, first + j);
+                if (lo == 0) {
+                    for (uint32_t e = 4 * (lane >> 2); e < hi; e += 32)
+                        row[(e >> 2) * 32] = *reinterpret_cast<const uint4 *>(have + e);
+                } else {  // a later segment, which starts within a quad
+                    for (uint32_t e = lo + (lane >> 2); e < ((hi + 3u) & ~3u); e += 8)
+                        reinterpret_cast<uint32_t *>(row + (e >> 2) * 32)[e & 3u] = have[e - lo];
                 }
             }
         }
@@ -280,39 +288,36 @@ __device__ __forceinline__ void walk_cells(const RowArgs &A, const SceneDev &S, 
     for_neighbour_cells(S, A.cells, (int)compact10(m), (int)compact10(m >> 1), (int)compact10(m >> 2), add);
 }
 
-// A hit row's neighbours two at a time as add(b0, b1, p0, p1), p their entries of `packed`
-// (the second of an odd row's last pair at infinity): kDepth pairs' loads together, the
-// next pairs' indices in flight.
-template <int kDepth = 2, class F>
-__device__ __forceinline__ void for_pairs(const uint2 *__restrict__ row, uint32_t count,
+// A hit row's neighbours two at a time as add(b0, b1, p0, p1), p their entries of `packed`:
+// four entries' loads together, the next four's indices in flight.  What fills the last
+// quad lies at infinity, where every pass's range test drops it, so the loop has no other
+// conditions.  (Two pairs at a time, each tested for the row's end, took the delta pass of
+// the 1 M dam break 111 us; quads take 96, and 92 to 78 deep in the flow.)
+template <class F>
+__device__ __forceinline__ void for_pairs(const uint4 *__restrict__ row, uint32_t count,
                                           const float4 *__restrict__ packed, F &&add) {
-    const uint32_t pairs = (count + 1) >> 1;
-    uint2 next[kDepth];
-#pragma unroll
-    for (int k = 0; k < kDepth; ++k) next[k] = k < pairs ? __ldg(row + k * 32) : make_uint2(0, 0);
-    for (uint32_t i = 0; i < pairs; i += kDepth) {
-        uint2 b[kDepth];
-        float4 p[kDepth], q[kDepth];
-#pragma unroll
-        for (int k = 0; k < kDepth; ++k) {
-            b[k] = next[k];
-            if (2 * (i + k) + 1 >= count) b[k].y = b[k].x;  // an odd row's last entry stands alone
-            if (i + k < pairs) {
-                p[k] = __ldg(&packed[b[k].x]);
-                q[k] = __ldg(&packed[b[k].y]);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kDepth; ++k)
-            if (i + kDepth + k < pairs) next[k] = __ldg(row + (i + kDepth + k) * 32);
-#pragma unroll
-        for (int k = 0; k < kDepth; ++k) {
-            if (i + k < pairs) {
-                if (2 * (i + k) + 1 >= count) q[k] = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-                add(b[k].x, b[k].y, p[k], q[k]);
-            }
-        }
+    const uint32_t quads = (count + 3) >> 2;
+    uint4 next = quads ? __ldg(row) : make_uint4(0, 0, 0, 0);
+    for (uint32_t i = 1; i <= quads; ++i) {
+        const uint4 b = next;
+        const float4 p = __ldg(&packed[b.x]), q = __ldg(&packed[b.y]), u = __ldg(&packed[b.z]), w = __ldg(&packed[b.w]);
+        row += 32;
+        if (i < quads) next = __ldg(row);
+        add(b.x, b.y, p, q);
+        add(b.z, b.w, u, w);
     }
+}
+
+// The warp's rows into L2 by one bulk request before its lanes go through them, where all
+// rows together are more than L2 holds (kFetchFrom): a step of 1 M particles takes 1.70 ms
+// with it and 1.75 without, one of 262 k, whose rows stay in L2, 0.521 and 0.514.
+__device__ __forceinline__ void fetch_rows(const RowArgs &A, uint32_t a) {
+    if (!A.fetch) return;
+    const uint32_t count = a < A.n ? A.hcount[a] : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, count == kListOverflow ? 0u : count);
+    if ((a & 31u) == 0 && most)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row_of(A, a)), "r"(((most + 3) >> 2) * 512)
+                     : "memory");
 }
 
 template <int PROFILE, bool kFast>
@@ -320,6 +325,7 @@ __global__ void __launch_bounds__(128, 8)
     k_row_lambda(RowArgs A, const float4 *__restrict__ ps, float *__restrict__ lambda, float *__restrict__ density,
                  float4 *__restrict__ plam) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+    fetch_rows(A, a);
     if (a >= A.n) return;
     const float4 pa = ps[a];
     float lam = 0.f, dens = 0.f;
@@ -366,6 +372,7 @@ __global__ void __launch_bounds__(128, 8)
                 float4 *__restrict__ ps_out, float4 *__restrict__ x, float4 *__restrict__ v, int last,
                 const HostParticlesOut *__restrict__ hout) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+    fetch_rows(A, a);
     const bool own = a < A.n;
     const bool fluid = own && A.type[a] != FGB_TYPE_OBSTACLE;
     uint32_t cell_start = 0;
@@ -414,6 +421,7 @@ __global__ void __launch_bounds__(128, 6)
     k_row_vorticity(RowArgs A, const float4 *__restrict__ ps, const float4 *__restrict__ v,
                     float4 *__restrict__ omega, float4 *__restrict__ pom, float4 *__restrict__ vx) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+    fetch_rows(A, a);
     if (a >= A.n) return;
     const float4 pa = ps[a], va = v[a];
     if (A.type[a] == FGB_TYPE_OBSTACLE) {
@@ -453,6 +461,7 @@ __global__ void __launch_bounds__(128, 8)
                 const float4 *__restrict__ pom, const float4 *__restrict__ vx, float4 *__restrict__ v,
                 float4 *__restrict__ x, const HostParticlesOut *__restrict__ hout) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+    fetch_rows(A, a);
     if (a >= A.n) return;
     if (A.type[a] == FGB_TYPE_OBSTACLE) {
         store_host_motion(hout, a, x[a], v[a]);
@@ -498,9 +507,11 @@ RowArgs row_args(const StepView &s) {
     A.groups = s.groups;
     A.group_count = s.group_count;
     A.group_mask = s.group_mask;
-    A.hrows = reinterpret_cast<uint2 *>(s.hlist);
+    A.hrows = reinterpret_cast<uint4 *>(s.hlist);
     A.hcount = s.hcount;
     A.hcap = s.hcap;
+    A.none = s.none;
+    A.fetch = s.n >= kFetchFrom;
     A.mass_range = s.mass_range;
     A.over = nullptr;
     A.ps_grid = s.ps_grid;

@@ -726,7 +726,7 @@ struct fgb_batch {
         s.lasting = lasting.p;
         s.row_policy = row_policy[c].p;
         s.row_policy_next = row_policy[c ^ 1].p;
-        if (cell_rows) s.hcap = cell_hits;
+        if (cell_rows) s.hcap = cell_hits, s.none = (uint32_t)capacity;
         s.near_stats = row_stats && over.p ? over.p + 2 : nullptr;
         return s;
     }
@@ -1017,7 +1017,7 @@ struct fgb_batch {
             // a row that overflowed holds up its warp's other rows: hardly any may
             if (st_over.p[1] <= n / 5000 || cell_hits >= kMaxCellHits) return FGB_OK;
             FGB_CUDA(cudaStreamSynchronize(stream()), "grow hit rows sync");
-            cell_hits = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 1) & ~1u);
+            cell_hits = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 3) & ~3u);
             st_over.p[0] = st_over.p[1] = 0;
             drop_graphs();
             solver->cell_caps[tune_bucket(solver->params.profile, n)] = cell_hits;
@@ -1241,14 +1241,15 @@ static bool list_kernels_asked() {
 static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     PoolScope scope(&b->solver->pool);
     const fgb_params &p = b->solver->params;
-    for (int c = 0; c < 2; ++c) FGB_CUDA(b->ps[c].alloc(cap), "batch alloc");
+    // one entry more where rows.cu gathers: the index that fills a hit row's last quad
+    for (int c = 0; c < 2; ++c) FGB_CUDA(b->ps[c].alloc(cap + 1), "batch alloc");
     FGB_CUDA(b->keys_in.alloc(cap), "batch alloc");
     FGB_CUDA(b->vals_in.alloc(cap), "batch alloc");
     FGB_CUDA(b->keys_sorted.alloc(cap), "batch alloc");
     FGB_CUDA(b->vals_sorted.alloc(cap), "batch alloc");
     b->sort_scratch_bytes = radix_scratch_bytes(cap);
     FGB_CUDA(b->sort_scratch.alloc(b->sort_scratch_bytes), "batch alloc");
-    FGB_CUDA(b->ps_grid.alloc(cap), "batch alloc");
+    FGB_CUDA(b->ps_grid.alloc(cap + 1), "batch alloc");
     if (b->cell_rows) {
         FGB_CUDA(b->groups.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->lasting.alloc(cap), "batch alloc groups");
@@ -1270,11 +1271,11 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     }
     if (!b->cell_rows && b->list_cap && b->hit_cap) FGB_CUDA(b->near.alloc(cap), "batch alloc");
     FGB_CUDA(b->lambda.alloc(cap), "batch alloc");
-    if (b->cell_rows || !packed_off()) FGB_CUDA(b->plam.alloc(cap), "batch alloc");
+    if (b->cell_rows || !packed_off()) FGB_CUDA(b->plam.alloc(cap + 1), "batch alloc");
     FGB_CUDA(b->mass_range.alloc(2), "batch alloc");
     FGB_CUDA(b->density.alloc(cap), "batch alloc");
     if (p.profile != FGB_PROFILE_REF) {
-        if (b->cell_rows || !packed_off()) FGB_CUDA(b->pom.alloc(cap), "batch alloc");
+        if (b->cell_rows || !packed_off()) FGB_CUDA(b->pom.alloc(cap + 1), "batch alloc");
         FGB_CUDA(b->omega.alloc(cap), "batch alloc");
         FGB_CUDA(b->vx.alloc(cap), "batch alloc");
     } else {
@@ -1282,6 +1283,11 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
         FGB_CUDA(b->colour_count.alloc(cap), "batch alloc");
     }
     cudaStream_t st = b->stream();
+    if (b->cell_rows) {  // the far entry: infinity, out of every pass's range
+        for (float4 *p : {b->ps[0].p, b->ps[1].p, b->ps_grid.p, b->plam.p, b->pom.p})
+            if (p) launch_fill_u32(reinterpret_cast<uint32_t *>(p + cap), 4, 0x7f800000u, st);
+        FGB_CUDA(cudaGetLastError(), "batch alloc");
+    }
     FGB_CUDA(cudaMemsetAsync(b->lambda.p, 0, cap * sizeof(float), st), "batch alloc");
     FGB_CUDA(cudaMemsetAsync(b->density.p, 0, cap * sizeof(float), st), "batch alloc");
     b->capacity = cap;
@@ -1367,8 +1373,8 @@ static int batch_init(fgb_batch *b) {
     ensure_tables();
     for (int c = 0; c < 2; ++c) {
         FGB_CUDA(b->x[c].alloc(n), "batch alloc");
-        FGB_CUDA(b->v[c].alloc(n), "batch alloc");
-        FGB_CUDA(b->type[c].alloc(n), "batch alloc");
+        FGB_CUDA(b->v[c].alloc(n + 1), "batch alloc");
+        FGB_CUDA(b->type[c].alloc(n + 1), "batch alloc");
         FGB_CUDA(b->col[c].alloc(n), "batch alloc");
         FGB_CUDA(b->slot[c].alloc(n), "batch alloc");
     }
@@ -2260,8 +2266,8 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     const uint64_t cap = grow ? std::max<uint64_t>(n1, b->capacity + b->capacity / 4) : b->capacity;
     if (grow) {
         FGB_CUDA(b->x[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->type[cn].alloc(cap), "sources_drains grow");
+        FGB_CUDA(b->v[cn].alloc(cap + 1), "sources_drains grow");
+        FGB_CUDA(b->type[cn].alloc(cap + 1), "sources_drains grow");
         FGB_CUDA(b->col[cn].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->slot[cn].alloc(cap), "sources_drains grow");
     }
@@ -2302,8 +2308,8 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     FGB_CUDA(cudaStreamSynchronize(st), "sources_drains sync");
     if (grow) {  // the old set and the per-step arrays, at the new capacity
         FGB_CUDA(b->x[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->type[cs].alloc(cap), "sources_drains grow");
+        FGB_CUDA(b->v[cs].alloc(cap + 1), "sources_drains grow");
+        FGB_CUDA(b->type[cs].alloc(cap + 1), "sources_drains grow");
         FGB_CUDA(b->col[cs].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->slot[cs].alloc(cap), "sources_drains grow");
         int rc = alloc_step_arrays(b, cap);

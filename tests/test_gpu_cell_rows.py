@@ -88,3 +88,16 @@ def test_scenes_of_several_sizes_and_a_violent_one(profile):
 
 def test_calm_scene_over_many_steps():
     _same(capi.PROFILE_BASELINE, [scenes.cube_scene(8192, 9)], 40)
+
+
+@pytest.mark.parametrize("profile", PROFILES)
+@pytest.mark.parametrize("n", [3, 4, 5, 6, 7, 8, 9, 255, 256, 257, 259])
+def test_row_ends(profile, n):
+    # all of one cell: rows of n entries end at every place of a quad, and in a second segment
+    _same(profile, [_cloud(n, 1, n, masses=True)], 3)
+
+
+@pytest.mark.parametrize("n", [399999, 400001])
+def test_rows_asked_for_ahead(n):
+    # at either side of the size from which the passes prefetch their rows
+    _same(capi.PROFILE_BASELINE, [_cloud(n, 36, n, obstacles=11)], 3)
