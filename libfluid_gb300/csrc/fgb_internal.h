@@ -118,6 +118,7 @@ struct StepView {
     // index under group_mask wraps -- and the groups' number (zeroed every step)
     uint32_t none;  // the entry past the particles that lies at infinity: what fills a hit row's last quad
     uint32_t *groups, *group_count, group_mask;
+    float4 *pv;            // per particle: p* and mass, velocity after the last delta pass
     uint32_t *moved;       // per particle: at a cell's first, the largest movement in the cell
     uint8_t *lasting;      // per group
     RowPolicy *row_policy, *row_policy_next;  // per scene: of the step before, and of this one

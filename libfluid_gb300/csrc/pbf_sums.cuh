@@ -423,10 +423,10 @@ struct DeltaSum {
     }
 };
 
-// Final velocity (and, in the ref profile, position) after the step's last correction
+// Final velocity (returned, too; in the ref profile also position) after the step's last correction
 // (oclsph_kernel.h:404-416).
 template <int PROFILE>
-__device__ __forceinline__ void finalise(const Phys &ph, const SceneDev &S, uint32_t a, const float *q,
+__device__ __forceinline__ float4 finalise(const Phys &ph, const SceneDev &S, uint32_t a, const float *q,
                                          const float4 &va, const float *vel, float4 *__restrict__ x,
                                          float4 *__restrict__ v, const HostParticlesOut *__restrict__ hout) {
     const float4 xa = x[a];
@@ -441,11 +441,13 @@ __device__ __forceinline__ void finalise(const Phys &ph, const SceneDev &S, uint
             nv[d] = dd * S.inv_dt;
         }
     }
-    v[a] = make_float4(nv[0], nv[1], nv[2], va.w);
+    const float4 now = make_float4(nv[0], nv[1], nv[2], va.w);
+    v[a] = now;
     if (PROFILE == kRef) {
         x[a] = make_float4(nx[0], nx[1], nx[2], xa.w);
-        store_host_motion(hout, a, x[a], v[a]);
+        store_host_motion(hout, a, x[a], now);
     }
+    return now;
 }
 
 // Vorticity and the XSPH sum of one particle over its fluid neighbours.

@@ -308,6 +308,13 @@ __device__ __forceinline__ void for_pairs(const uint4 *__restrict__ row, uint32_
     }
 }
 
+// 32 aligned bytes by one load
+__device__ __forceinline__ void load_two(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
 // The warp's rows into L2 by one bulk request before its lanes go through them, where all
 // rows together are more than L2 holds (kFetchFrom): a step of 1 M particles takes 1.70 ms
 // with it and 1.75 without, one of 262 k, whose rows stay in L2, 0.521 and 0.514.
@@ -370,7 +377,7 @@ template <int PROFILE, bool kFast>
 __global__ void __launch_bounds__(128, 8)
     k_row_delta(RowArgs A, const float4 *__restrict__ ps_in, const float4 *__restrict__ plam,
                 float4 *__restrict__ ps_out, float4 *__restrict__ x, float4 *__restrict__ v, int last,
-                const HostParticlesOut *__restrict__ hout) {
+                float4 *__restrict__ pv, const HostParticlesOut *__restrict__ hout) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
     fetch_rows(A, a);
     const bool own = a < A.n;
@@ -379,6 +386,7 @@ __global__ void __launch_bounds__(128, 8)
     float moved = 0.f;
     if (own && !fluid) {
         ps_out[a] = ps_in[a];
+        if (PROFILE != kRef && last) pv[2 * (size_t)a] = ps_in[a], pv[2 * (size_t)a + 1] = v[a];
         if (PROFILE == kRef && last) store_host_motion(hout, a, x[a], v[a]);
     }
     if (fluid) {
@@ -406,7 +414,13 @@ __global__ void __launch_bounds__(128, 8)
         float q[3], vel[3];
         sum.move(ph, S, A.tris, pa, a, v, q, va, vel);
         ps_out[a] = make_float4(q[0], q[1], q[2], pa.w);
-        if (last) finalise<PROFILE>(ph, S, a, q, va, vel, x, v, hout);
+        if (last) {
+            const float4 now = finalise<PROFILE>(ph, S, a, q, va, vel, x, v, hout);
+            if (PROFILE != kRef) {
+                pv[2 * (size_t)a] = make_float4(q[0], q[1], q[2], pa.w);
+                pv[2 * (size_t)a + 1] = now;
+            }
+        }
         const float4 g = __ldg(&A.ps_grid[a]);
         const float ex = q[0] - g.x, ey = q[1] - g.y, ez = q[2] - g.z;
         moved = sqrtf(ex * ex + ey * ey + ez * ez);
@@ -415,15 +429,19 @@ __global__ void __launch_bounds__(128, 8)
     if (PROFILE != kRef || !last) keep_moved(A, fluid, cell_start, moved);  // a search follows
 }
 
-// Pass A of the velocity terms: fluid neighbours only, which rows do not tell apart.
+// Pass A of the velocity terms: fluid neighbours only, which rows do not tell apart.  The
+// neighbours' positions and velocities come from one record of 32 bytes each (pv, by the
+// last delta pass) by one load: 32 lanes' records cost the L1 a third less than a position
+// and a velocity apart.  158 to 146 us at 1 M, 2 of it given back by the delta pass.
 template <bool kFast>
 __global__ void __launch_bounds__(128, 6)
-    k_row_vorticity(RowArgs A, const float4 *__restrict__ ps, const float4 *__restrict__ v,
-                    float4 *__restrict__ omega, float4 *__restrict__ pom, float4 *__restrict__ vx) {
+    k_row_vorticity(RowArgs A, const float4 *__restrict__ pv, float4 *__restrict__ omega, float4 *__restrict__ pom,
+                    float4 *__restrict__ vx) {
     const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
     fetch_rows(A, a);
     if (a >= A.n) return;
-    const float4 pa = ps[a], va = v[a];
+    float4 pa, va;
+    load_two(pv + 2 * (size_t)a, pa, va);
     if (A.type[a] == FGB_TYPE_OBSTACLE) {
         omega[a] = make_float4(0.f, 0.f, 0.f, 0.f);
         vx[a] = va;
@@ -436,21 +454,35 @@ __global__ void __launch_bounds__(128, 6)
     const bool obstacles = S.obstacles != 0;
     const uint32_t count = A.hcount[a];
     VorticitySum sum;
-    if (count != kListOverflow)
-        for_pairs(row_of(A, a), count, ps, [&](uint32_t b0, uint32_t b1, float4 p, float4 q) {
-            const float4 u = __ldg(&v[b0]), w = __ldg(&v[b1]);
-            if (obstacles) {
-                if (__ldg(&A.type[b0]) == FGB_TYPE_OBSTACLE) p.x = INFINITY;
-                if (__ldg(&A.type[b1]) == FGB_TYPE_OBSTACLE) q.x = INFINITY;
-            }
-            sum.template add2<kFast>(ph, pa, va, Two(p.x, q.x), Two(p.y, q.y), Two(p.z, q.z), Two(p.w, q.w),
-                                     Two(u.x, w.x), Two(u.y, w.y), Two(u.z, w.z));
-        });
-    else
+    auto two = [&](uint32_t b0, uint32_t b1, float4 p, const float4 &u, float4 q, const float4 &w) {
+        if (obstacles) {
+            if (__ldg(&A.type[b0]) == FGB_TYPE_OBSTACLE) p.x = INFINITY;
+            if (__ldg(&A.type[b1]) == FGB_TYPE_OBSTACLE) q.x = INFINITY;
+        }
+        sum.template add2<kFast>(ph, pa, va, Two(p.x, q.x), Two(p.y, q.y), Two(p.z, q.z), Two(p.w, q.w),
+                                 Two(u.x, w.x), Two(u.y, w.y), Two(u.z, w.z));
+    };
+    if (count != kListOverflow) {
+        const uint4 *row = row_of(A, a);
+        const uint32_t quads = (count + 3) >> 2;
+        uint4 next = quads ? __ldg(row) : make_uint4(0, 0, 0, 0);
+        for (uint32_t i = 1; i <= quads; ++i) {
+            const uint4 b = next;
+            float4 p[4], u[4];
+            load_two(pv + 2 * (size_t)b.x, p[0], u[0]);
+            load_two(pv + 2 * (size_t)b.y, p[1], u[1]);
+            load_two(pv + 2 * (size_t)b.z, p[2], u[2]);
+            load_two(pv + 2 * (size_t)b.w, p[3], u[3]);
+            row += 32;
+            if (i < quads) next = __ldg(row);
+            two(b.x, b.y, p[0], u[0], p[1], u[1]);
+            two(b.z, b.w, p[2], u[2], p[3], u[3]);
+        }
+    } else
         walk_cells(A, S, key, [&](uint32_t b) {
             if (obstacles && __ldg(&A.type[b]) == FGB_TYPE_OBSTACLE) return;
-            const float4 p = __ldg(&ps[b]);
-            sum.add(ph, pa, va, p.x, p.y, p.z, p.w, [&] { return __ldg(&v[b]); });
+            const float4 p = __ldg(&pv[2 * (size_t)b]);
+            sum.add(ph, pa, va, p.x, p.y, p.z, p.w, [&] { return __ldg(&pv[2 * (size_t)b + 1]); });
         });
     sum.finish(ph, a, pa, va, omega, pom, vx);
 }
@@ -569,7 +601,7 @@ cudaError_t lambda_as(const StepView &s, const float4 *ps, int iteration, cudaSt
 template <int PROFILE, bool kFast>
 cudaError_t delta_as(const StepView &s, const float4 *ps_in, float4 *ps_out, bool last, cudaStream_t st) {
     k_row_delta<PROFILE, kFast><<<row_grid(s), 128, 0, st>>>(row_args(s), ps_in, s.plam, ps_out, s.x1, s.v1,
-                                                                  last ? 1 : 0, s.hout);
+                                                                  last ? 1 : 0, s.pv, s.hout);
     return cudaGetLastError();
 }
 
@@ -578,7 +610,7 @@ cudaError_t velocity_as(const StepView &s, const float4 *ps, cudaStream_t st, co
     cudaError_t e = rows_of(s, ps, s.iterations, st);
     if (e != cudaSuccess) return e;
     const RowArgs A = row_args(s);
-    k_row_vorticity<kFast><<<row_grid(s), 128, 0, st>>>(A, ps, s.v1, s.omega, s.pom, s.vx);
+    k_row_vorticity<kFast><<<row_grid(s), 128, 0, st>>>(A, s.pv, s.omega, s.pom, s.vx);
     if (between) between();
     k_row_apply<kFast><<<row_grid(s), 128, 0, st>>>(A, ps, s.omega, s.pom, s.vx, s.v1, s.x1, s.hout);
     return cudaGetLastError();

@@ -596,6 +596,7 @@ struct fgb_batch {
     Dev<RowPolicy> row_policy[2];  // by the state set a step reads
     Dev<float> lambda, density;
     Dev<float4> plam;             // the lambda pass's p* with lambda in w (delta reads)
+    Dev<float4> pv;  // rows.cu: p*, mass and velocity of a particle in one record of 32 bytes
     Dev<float4> pom;              // the vorticity pass's p* with |omega| in w (apply reads)
     Dev<uint32_t> mass_range;     // {min mass, ~max mass} bits of the step
     Dev<float4> omega, vx;
@@ -682,6 +683,7 @@ struct fgb_batch {
         s.ps_a = ps[0].p;
         s.ps_b = ps[1].p;
         s.lambda = lambda.p;
+        s.pv = pv.p;
         s.plam = plam.p;
         s.pom = pom.p;
         s.mass_range = mass_range.p;
@@ -1276,6 +1278,7 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     FGB_CUDA(b->density.alloc(cap), "batch alloc");
     if (p.profile != FGB_PROFILE_REF) {
         if (b->cell_rows || !packed_off()) FGB_CUDA(b->pom.alloc(cap + 1), "batch alloc");
+        if (b->cell_rows) FGB_CUDA(b->pv.alloc(2 * (cap + 1)), "batch alloc");
         FGB_CUDA(b->omega.alloc(cap), "batch alloc");
         FGB_CUDA(b->vx.alloc(cap), "batch alloc");
     } else {
@@ -1286,6 +1289,7 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     if (b->cell_rows) {  // the far entry: infinity, out of every pass's range
         for (float4 *p : {b->ps[0].p, b->ps[1].p, b->ps_grid.p, b->plam.p, b->pom.p})
             if (p) launch_fill_u32(reinterpret_cast<uint32_t *>(p + cap), 4, 0x7f800000u, st);
+        if (b->pv.p) launch_fill_u32(reinterpret_cast<uint32_t *>(b->pv.p + 2 * cap), 8, 0x7f800000u, st);
         FGB_CUDA(cudaGetLastError(), "batch alloc");
     }
     FGB_CUDA(cudaMemsetAsync(b->lambda.p, 0, cap * sizeof(float), st), "batch alloc");
@@ -1373,7 +1377,7 @@ static int batch_init(fgb_batch *b) {
     ensure_tables();
     for (int c = 0; c < 2; ++c) {
         FGB_CUDA(b->x[c].alloc(n), "batch alloc");
-        FGB_CUDA(b->v[c].alloc(n + 1), "batch alloc");
+        FGB_CUDA(b->v[c].alloc(n), "batch alloc");
         FGB_CUDA(b->type[c].alloc(n + 1), "batch alloc");
         FGB_CUDA(b->col[c].alloc(n), "batch alloc");
         FGB_CUDA(b->slot[c].alloc(n), "batch alloc");
@@ -2266,7 +2270,7 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     const uint64_t cap = grow ? std::max<uint64_t>(n1, b->capacity + b->capacity / 4) : b->capacity;
     if (grow) {
         FGB_CUDA(b->x[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cn].alloc(cap + 1), "sources_drains grow");
+        FGB_CUDA(b->v[cn].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->type[cn].alloc(cap + 1), "sources_drains grow");
         FGB_CUDA(b->col[cn].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->slot[cn].alloc(cap), "sources_drains grow");
@@ -2308,7 +2312,7 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     FGB_CUDA(cudaStreamSynchronize(st), "sources_drains sync");
     if (grow) {  // the old set and the per-step arrays, at the new capacity
         FGB_CUDA(b->x[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cs].alloc(cap + 1), "sources_drains grow");
+        FGB_CUDA(b->v[cs].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->type[cs].alloc(cap + 1), "sources_drains grow");
         FGB_CUDA(b->col[cs].alloc(cap), "sources_drains grow");
         FGB_CUDA(b->slot[cs].alloc(cap), "sources_drains grow");
