@@ -1,12 +1,22 @@
 // rows.cu -- hit rows from one warp per grid cell, and the gather passes over them.
 //
-// k_cell_rows gives a warp the particles of one cell (up to a group of them): its lanes
+// k_cell_rows gives a warp the particles of one cell (up to a group of them).  Its lanes
 // hold the candidates of the cell's 27 neighbour cells, in the reference's order (z, y, x
-// ascending, each cell in sorted order: oclsph_kernel.h:155-183), in registers, and test
-// them all at once against each of the particles; a ballot ranks those within range, and
-// they go to the particle's hit row as sorted indices, in order.  The candidates are loaded
-// once for all particles of the group, every lane tests 32 different ones, and no lane
-// waits for another's longer list.
+// ascending, each cell in sorted order: oclsph_kernel.h:155-183), a few in a row each, and
+// test them all at once against each of the particles; a running sum over the lanes places
+// those within range, and they go to the particle's hit row as sorted indices, in order.
+// The candidates are loaded once for all particles of the group and no lane waits for
+// another's longer list.
+//
+// The test runs on pairs of candidates in 16 bits, relative to the group's first particle,
+// with a margin that covers its rounding (kHalfMargin): rows hold all that 32 bits would
+// find and about 1 % more, which the passes drop.  Instruction issue bounds the search: of
+// 175 warp instructions a particle (1 M dam break, before the candidates were gathered
+// straight to their lanes), 21 went to a cell's setup, 34 to its candidates, 120 to the
+// particle: 36 tests, 27 appends, 10 the running sum, 12 the writing of its row.  In 32 bits
+// with a ballot for every 32 candidates it took 222.  The first lambda stage (search and
+// sums) of the 1 M dam break at steps 5, 30 and 100: 357, 387 and 357 us before, 319, 334
+// and 323 now.
 //
 // Rows that last.  The step's first search keeps every candidate within h plus a skin of
 // the grid positions.  Such a row holds every neighbour within h, in order, while no
@@ -21,6 +31,7 @@
 // again, so the sums are those of the 27-cell walk of pbf.cu, bit for bit.
 #include <algorithm>
 #include <cstdint>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "fgb_internal.h"
@@ -50,6 +61,7 @@ struct RowArgs {
     const float4 *ps_grid;       // the grid positions
     uint32_t *moved;             // largest movement in a cell since then (float bits), at its first particle
     uint8_t *lasting;            // per group: its rows are the first search's, with the skin
+    float inv_h;
     float skin, skin_r2;         // the skin, and (h + skin)^2
     const RowPolicy *policy;     // per scene, of the step before; policy_next of this one
     RowPolicy *policy_next;
@@ -64,14 +76,14 @@ __device__ __forceinline__ uint4 *row_of(const RowArgs &A, uint32_t a) {
 constexpr uint32_t kCellBlock = 128, kCellWarps = kCellBlock / 32;
 constexpr uint32_t kFetchFrom = 400000;   // particles from which the passes ask for their rows ahead
 constexpr float kRowSkin = 0.1f;          // the skin of rows that last, in h
-constexpr uint32_t kHeld = 8;             // candidates a lane holds at a time
-constexpr uint32_t kHeldAll = 32 * kHeld;  // candidates a warp holds
-constexpr uint32_t kGroup = 4;            // particles whose hits are collected before they are written
+constexpr uint32_t kHeldAll = 256;        // candidates a warp holds at a time
+constexpr uint32_t kList = 4;             // particles whose hits are collected before they are written
 constexpr uint32_t kPitch = kHeldAll + 8;  // room to fill the last quad; the four lists in different banks
 
 struct CellShared {
-    uint32_t map[kHeldAll];                         // sorted indices of the candidates held
-    alignas(16) uint32_t hits[kGroup * kPitch];  // hits of a group's particles among them, in order
+    alignas(16) uint32_t map[kHeldAll];         // sorted indices of the candidates held
+    alignas(16) uint32_t hits[kList * kPitch];  // hits of four of the group's particles among them, in order
+    uint4 own[32];                              // the group's particles: x, y and z twice in 16 bits, all bits if it has sums
 };
 
 // The lane's neighbour cell of the cell with Morton code m: its table index, or false
@@ -92,27 +104,41 @@ __device__ __forceinline__ bool neighbour_cell(const SceneDev &S, uint32_t m, in
     return ok;
 }
 
-// Where r2 is negative: store b to the warp's list at shared address `to`, in lane order;
-// `to` moves past the entries.  Written out so that the store is predicated: as a branch it
-// cost more instructions than the test.
-__device__ __forceinline__ void append_hits(float r2, uint32_t b, uint32_t before, uint32_t &to) {
+// If `hits` has the bit: store b at shared address `to`, which moves on.  Written out so that
+// both are predicated.
+__device__ __forceinline__ void append_if(uint32_t hits, uint32_t bit, uint32_t b, uint32_t &to) {
     asm volatile(
         "{\n\t"
         ".reg .pred hit;\n\t"
-        ".reg .b32 in, at;\n\t"
-        "setp.lt.f32 hit, %1, 0f00000000;\n\t"
-        "vote.sync.ballot.b32 in, hit, 0xffffffff;\n\t"
-        "and.b32 at, in, %3;\n\t"
-        "popc.b32 at, at;\n\t"
-        "mad.lo.u32 at, at, 4, %0;\n\t"
-        "@hit st.shared.u32 [at], %2;\n\t"
-        "popc.b32 in, in;\n\t"
-        "mad.lo.u32 %0, in, 4, %0;\n\t"
+        ".reg .b32 in;\n\t"
+        "and.b32 in, %1, %2;\n\t"
+        "setp.ne.u32 hit, in, 0;\n\t"
+        "@hit st.shared.u32 [%0], %3;\n\t"
+        "@hit add.u32 %0, %0, 4;\n\t"
         "}"
         : "+r"(to)
-        : "f"(r2), "r"(b), "r"(before)
+        : "r"(hits), "r"(bit), "r"(b)
         : "memory");
 }
+
+// Sums of the lanes up to and including this one.
+__device__ __forceinline__ uint32_t running_sum(uint32_t v) {
+#define FGB_ADD_FROM(d)                                            \
+    asm("{\n\t.reg .pred in;\n\t.reg .b32 t;\n\t"                  \
+        "shfl.sync.up.b32 t|in, %0, " #d ", 0, 0xffffffff;\n\t"    \
+        "@in add.u32 %0, %0, t;\n\t}"                              \
+        : "+r"(v))
+    FGB_ADD_FROM(1);
+    FGB_ADD_FROM(2);
+    FGB_ADD_FROM(4);
+    FGB_ADD_FROM(8);
+    FGB_ADD_FROM(16);
+#undef FGB_ADD_FROM
+    return v;
+}
+
+__device__ __forceinline__ uint32_t bits_of(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
+__device__ __forceinline__ __half2 half2_of(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 
 __device__ __forceinline__ void fill(uint32_t at, uint32_t b) {
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(b) : "memory");
@@ -133,10 +159,18 @@ __device__ __forceinline__ RowPolicy decide(const RowPolicy &p) {
     return n;
 }
 
-template <int R>
-struct Rounds {
-    static constexpr int value = R;
+template <uint32_t P>
+struct Pairs {
+    static constexpr uint32_t value = P;
 };
+
+// The largest distance, in h, of a particle from the group's origin along an axis at which
+// the 16-bit test holds, and the test's margin on (reach / h)^2.  Rounded to 16 bits, such a
+// particle is off by at most 2^-11, a candidate in reach of it (below 3.2) by 2^-10 and their
+// difference (below 2) by 2^-11: 2^-9 along an axis.  At a distance up to 1.11 the square is
+// over by 2 * 2^-9 * sqrt(3) * 1.11 + 3 * 2^-18 < 0.00753, and the two roundings of the sum
+// before its sign is settled add 2 * 2^-11 (it stays within 2): below 0.0086 in all.
+constexpr float kHalfReach = 2.f, kHalfMargin = 0.0087f;
 
 // kFirst: the step's first search (the grid positions); else a later one, which leaves the
 // groups whose rows still last.
@@ -144,7 +178,7 @@ template <bool kFirst>
 __global__ void __launch_bounds__(kCellBlock, 7)
     k_cell_rows(RowArgs A, const float4 *__restrict__ ps, float r2max, uint32_t n_scenes, int count_use) {
     __shared__ CellShared s_warp[kCellWarps];
-    const uint32_t lane = threadIdx.x & 31u, before = lanemask_lt();
+    const uint32_t lane = threadIdx.x & 31u;
     CellShared &sh = s_warp[threadIdx.x >> 5];
     const uint32_t lists = (uint32_t)__cvta_generic_to_shared(sh.hits);
     const uint32_t warps = gridDim.x * kCellWarps, groups = *A.group_count;
@@ -167,9 +201,8 @@ __global__ void __launch_bounds__(kCellBlock, 7)
         uint32_t cell;
         uint2 range = make_uint2(0, 0);
         if (neighbour_cell(S, morton_of(key, A.mbits), dx, dy, dz, cell) && lane < 27) range = __ldg(&A.cells[cell]);
-        const uint32_t count = range.y > range.x ? range.y - range.x : 0u;
+        const uint32_t count = range.y > range.x ? range.y - range.x : 0u, from = range.x;
         const uint32_t end = min(__shfl_sync(0xffffffffu, range.y, 13), (first | A.group_mask) + 1);
-        const uint32_t own = end > first ? end - first : 0u;  // at most 32
         float reach2 = r2max;
         if (kFirst) {
             const bool keep = decide(A.policy[scene]).keep != 0;
@@ -177,7 +210,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
             if (lane == 0) A.lasting[c] = keep ? 1 : 0;
         } else {
             const bool lasts = A.lasting[c] != 0;
-            const uint32_t m = count ? __ldg(&A.moved[range.x]) : 0u;
+            const uint32_t m = count ? __ldg(&A.moved[from]) : 0u;
             const float bound = __uint_as_float(__shfl_sync(0xffffffffu, m, 13)) +
                                 __uint_as_float(__reduce_max_sync(0xffffffffu, m));
             const bool skip = lasts && bound <= A.skin;
@@ -186,96 +219,166 @@ __global__ void __launch_bounds__(kCellBlock, 7)
                     report();
                     seen_scene = scene;
                 }
-                asked += own;
-                if (skip) used += own;
+                const uint32_t group = end > first ? end - first : 0u;
+                asked += group;
+                if (skip) used += group;
             }
             if (skip) continue;
             if (lasts && lane == 0) A.lasting[c] = 0;
         }
-        uint32_t upto = count;  // candidates up to and including the lane's cell
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, upto, d);
-            if ((int)lane >= d) upto += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, upto, 31), from = upto - count;
+        const uint32_t upto = running_sum(count);  // candidates up to and including the lane's cell
+        const uint32_t total = __shfl_sync(0xffffffffu, upto, 31), before = upto - count;
         const bool obstacles = S.obstacles != 0;
-        uint32_t found = 0;  // lane j: hits of the group's j-th particle
-        for (uint32_t seg = 0; seg < total; seg += kHeldAll) {
-            // candidates [seg, seg + 256): the lanes list their cells' indices, then each
-            // takes every 32nd candidate
+        // 16-bit positions are taken from the group's first particle, in units of h
+        const float inv_h = A.inv_h;
+        const float4 origin = __ldg(&ps[first]);
+        const float ox = -origin.x * inv_h, oy = -origin.y * inv_h, oz = -origin.z * inv_h;
+        const __half2 less = __half2half2(__hneg(__float2half_ru(reach2 * inv_h * inv_h + kHalfMargin)));
+        for (uint32_t base = first; base < end; base += 32) {
+            const uint32_t own = min(end - base, 32u);
+            uint32_t found = 0;  // lane j: the hits of the j-th particle
+            bool far = false;
             __syncwarp();
-            {
-                const uint32_t lo = max(from, seg), hi = min(upto, seg + kHeldAll);
-                uint32_t b = range.x + (lo - from);
-                for (uint32_t k = lo; k < hi; ++k) sh.map[k - seg] = b++;
+            if (lane < own) {
+                const float4 p = __ldg(&ps[base + lane]);
+                const float x = __fmaf_rn(p.x, inv_h, ox), y = __fmaf_rn(p.y, inv_h, oy), z = __fmaf_rn(p.z, inv_h, oz);
+                const bool none = obstacles && A.type[base + lane] == FGB_TYPE_OBSTACLE;  // no sums: an empty row
+                far = !none && !(fabsf(x) <= kHalfReach && fabsf(y) <= kHalfReach && fabsf(z) <= kHalfReach);
+                sh.own[lane] = make_uint4(bits_of(__floats2half2_rn(x, x)), bits_of(__floats2half2_rn(y, y)),
+                                          bits_of(__floats2half2_rn(z, z)), none || far ? 0u : 0xffffffffu);
             }
-            __syncwarp();
-            uint32_t idx[kHeld];
-            float X[kHeld], Y[kHeld], Z[kHeld];
-#pragma unroll
-            for (uint32_t q = 0; q < kHeld; ++q) {
-                const uint32_t at = 32 * q + lane;
-                X[q] = INFINITY, Y[q] = Z[q] = 0.f, idx[q] = 0;
-                if (seg + at < total) {
-                    idx[q] = sh.map[at];
-                    const float4 p = __ldg(&ps[idx[q]]);
-                    X[q] = p.x, Y[q] = p.y, Z[q] = p.z;
-                }
-            }
-            // particle a against the first R candidates of every lane; the shared address
-            // past its list
-            auto test = [&](auto rounds, uint32_t a, uint32_t to) {
-                const float4 pa = __ldg(&ps[a]);
-#pragma unroll
-                for (int q = 0; q < decltype(rounds)::value; ++q) {
-                    const float ex = X[q] - pa.x, ey = Y[q] - pa.y, ez = Z[q] - pa.z;
-                    append_hits(__fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmaf_rn(ez, ez, -reach2))), idx[q], before, to);
-                }
-                return to;
-            };
-            const uint32_t held = min((total - seg + 31) >> 5, kHeld);
-            for (uint32_t four = 0; four < own; four += kGroup) {
-                const uint32_t earlier = found;  // hits of earlier segments
-                const uint32_t last = min(four + kGroup, own);
+            const unsigned fars = __ballot_sync(0xffffffffu, far);
+            for (uint32_t seg = 0; seg < total; seg += kHeldAll) {
+                // candidates [seg, seg + 256): the lanes list their cells' indices
                 __syncwarp();
-                auto each = [&](auto rounds) {
+                {
+                    const uint32_t lo = max(before, seg), hi = min(upto, seg + kHeldAll);
+                    uint32_t b = from + (lo - before);
+                    uint32_t *to = sh.map + (lo - seg);
+                    for (uint32_t k = lo; k < hi; k += 4, to += 4, b += 4) {
+                        to[0] = b;
+                        if (k + 1 < hi) to[1] = b + 1;
+                        if (k + 2 < hi) to[2] = b + 2;
+                        if (k + 3 < hi) to[3] = b + 3;
+                    }
+                }
+                __syncwarp();
+                const uint32_t here = min(total - seg, kHeldAll);
+                auto segment = [&](auto pairs) {
+                    constexpr uint32_t P = decltype(pairs)::value;  // the lane's 2 P candidates in a row
+                    __half2 X[P], Y[P], Z[P];
+                    uint32_t idx[2 * P];
+#pragma unroll
+                    for (uint32_t k = 0; k < P; ++k) {
+                        const uint2 i = reinterpret_cast<const uint2 *>(sh.map)[lane * P + k];
+                        idx[2 * k] = i.x, idx[2 * k + 1] = i.y;
+                    }
+#pragma unroll
+                    for (uint32_t k = 0; k < P; ++k) {
+                        float4 p = make_float4(INFINITY, INFINITY, INFINITY, 0.f), q = p;
+                        if (2 * (lane * P + k) < here) p = __ldg(&ps[idx[2 * k]]);
+                        if (2 * (lane * P + k) + 1 < here) q = __ldg(&ps[idx[2 * k + 1]]);
+                        X[k] = __floats2half2_rn(__fmaf_rn(p.x, inv_h, ox), __fmaf_rn(q.x, inv_h, ox));
+                        Y[k] = __floats2half2_rn(__fmaf_rn(p.y, inv_h, oy), __fmaf_rn(q.y, inv_h, oy));
+                        Z[k] = __floats2half2_rn(__fmaf_rn(p.z, inv_h, oz), __fmaf_rn(q.z, inv_h, oz));
+                    }
+                    // the lane's candidates within reach of the j-th particle: 2 k and 2 k + 1 at
+                    // bits 16 - P + k and 32 - P + k
+                    auto hits_of = [&](uint32_t j) {
+                        const uint4 o = sh.own[j];
+                        const __half2 x = half2_of(o.x), y = half2_of(o.y), z = half2_of(o.z);
+                        uint32_t hits = 0;
+#pragma unroll
+                        for (uint32_t k = 0; k < P; ++k) {
+                            const __half2 ex = __hsub2(X[k], x), ey = __hsub2(Y[k], y), ez = __hsub2(Z[k], z);
+                            const __half2 r2 = __hfma2(ex, ex, __hfma2(ey, ey, __hfma2(ez, ez, less)));
+                            hits = hits >> 1 | (bits_of(r2) & 0x80008000u);
+                        }
+                        return hits & o.w;
+                    };
+                    auto append = [&](uint32_t hits, uint32_t to) {
+#pragma unroll
+                        for (uint32_t k = 0; k < P; ++k) {
+                            append_if(hits, 1u << (16 - P + k), idx[2 * k], to);
+                            append_if(hits, 1u << (32 - P + k), idx[2 * k + 1], to);
+                        }
+                    };
 #pragma unroll 1
-                    for (uint32_t j = four; j < last; ++j) {
-                        if (obstacles && A.type[first + j] == FGB_TYPE_OBSTACLE) continue;  // no sums: an empty row
-                        const uint32_t list = lists + 4 * (j - four) * kPitch, to = test(rounds, first + j, list);
-                        if (lane < 3) fill(to + 4 * lane, A.none);
-                        if (lane == j) found += (to - list) >> 2;
+                    for (uint32_t four = 0; four < own; four += kList) {
+                        const uint32_t earlier = found;  // hits of earlier segments
+                        const uint32_t last = min(four + kList, own);
+                        __syncwarp();
+#pragma unroll 1
+                        for (uint32_t j = four; j < last; j += 2) {
+                            const bool two = j + 1 < last;
+                            const uint32_t h0 = hits_of(j), h1 = two ? hits_of(j + 1) : 0u;
+                            const uint32_t n = __popc(h0) | __popc(h1) << 16;
+                            const uint32_t sum = running_sum(n), at = sum - n;
+                            const uint32_t all = __shfl_sync(0xffffffffu, sum, 31);
+                            const uint32_t list = lists + 4 * (j - four) * kPitch;
+                            append(h0, list + 4 * (at & 0xffffu));
+                            if (lane < 3) fill(list + 4 * ((all & 0xffffu) + lane), A.none);
+                            if (lane == j) found += all & 0xffffu;
+                            if (two) {
+                                append(h1, list + 4 * kPitch + 4 * (at >> 16));
+                                if (lane < 3) fill(list + 4 * kPitch + 4 * ((all >> 16) + lane), A.none);
+                                if (lane == j + 1) found += all >> 16;
+                            }
+                        }
+                        __syncwarp();
+                        // the four's hits to their rows: lane 4 p + j takes quad p of the j-th
+                        const uint32_t j = four + (lane & 3u);
+                        const uint32_t lo = __shfl_sync(0xffffffffu, earlier, j),
+                                       hi = min(__shfl_sync(0xffffffffu, found, j), A.hcap);
+                        if (j >= own) continue;
+                        const uint32_t *have = sh.hits + (lane & 3u) * kPitch;
+                        uint4 *row = row_of(A, base + j);
+                        if (lo == 0) {
+                            for (uint32_t e = 4 * (lane >> 2); e < hi; e += 32)
+                                row[(e >> 2) * 32] = *reinterpret_cast<const uint4 *>(have + e);
+                        } else {  // a later segment, which starts within a quad
+                            for (uint32_t e = lo + (lane >> 2); e < ((hi + 3u) & ~3u); e += 8)
+                                reinterpret_cast<uint32_t *>(row + (e >> 2) * 32)[e & 3u] = have[e - lo];
+                        }
                     }
                 };
-                switch (held) {
-                case 8: each(Rounds<8>{}); break;
-                case 7: each(Rounds<7>{}); break;
-                case 6: each(Rounds<6>{}); break;
-                case 5: each(Rounds<5>{}); break;
-                default: each(Rounds<4>{}); break;
-                }
-                __syncwarp();
-                // the four's hits to their rows: lane 4 p + j takes quad p of the j-th
-                const uint32_t j = four + (lane & 3u);
-                const uint32_t lo = __shfl_sync(0xffffffffu, earlier, j),
-                               hi = min(__shfl_sync(0xffffffffu, found, j), A.hcap);
-                if (j >= own) continue;
-                const uint32_t *have = sh.hits + (lane & 3u) * kPitch;
-                uint4 *row = row_of(A, first + j);
-                if (lo == 0) {
-                    for (uint32_t e = 4 * (lane >> 2); e < hi; e += 32)
-                        row[(e >> 2) * 32] = *reinterpret_cast<const uint4 *>(have + e);
-                } else {  // a later segment, which starts within a quad
-                    for (uint32_t e = lo + (lane >> 2); e < ((hi + 3u) & ~3u); e += 8)
-                        reinterpret_cast<uint32_t *>(row + (e >> 2) * 32)[e & 3u] = have[e - lo];
+                if (here <= 128)
+                    segment(Pairs<2>{});
+                else if (here <= 192)
+                    segment(Pairs<3>{});
+                else
+                    segment(Pairs<4>{});
+                // particles too far from the group's origin for 16 bits
+                if (fars) __syncwarp();
+                for (unsigned rest = fars; rest; rest &= rest - 1) {
+                    const uint32_t j = __ffs(rest) - 1;
+                    const float4 pa = __ldg(&ps[base + j]);
+                    uint32_t *row = reinterpret_cast<uint32_t *>(row_of(A, base + j));
+                    uint32_t at = __shfl_sync(0xffffffffu, found, j);
+                    for (uint32_t k = 0; k < here; k += 32) {
+                        bool hit = false;
+                        uint32_t b = 0;
+                        if (k + lane < here) {
+                            b = sh.map[k + lane];
+                            const float4 p = __ldg(&ps[b]);
+                            hit = dist2(p.x - pa.x, p.y - pa.y, p.z - pa.z) < reach2;
+                        }
+                        const unsigned in = __ballot_sync(0xffffffffu, hit);
+                        const uint32_t e = at + __popc(in & lanemask_lt());
+                        if (hit && e < A.hcap) row[(e >> 2) * 128 + (e & 3u)] = b;
+                        at += __popc(in);
+                    }
+                    if (lane < 3 && at + lane < ((at + 3u) & ~3u) && at + lane < A.hcap)
+                        row[((at + lane) >> 2) * 128 + ((at + lane) & 3u)] = A.none;
+                    if (lane == j) found = at;
+                    __syncwarp();
                 }
             }
-        }
-        if (lane < own) A.hcount[first + lane] = found > A.hcap ? kListOverflow : (uint16_t)found;
-        if (A.over) {
-            const unsigned full = __ballot_sync(0xffffffffu, lane < own && found > A.hcap);
-            if (full && lane == 0) atomicAdd(A.over, (uint32_t)__popc(full));
+            if (lane < own) A.hcount[base + lane] = found > A.hcap ? kListOverflow : (uint16_t)found;
+            if (A.over) {
+                const unsigned full = __ballot_sync(0xffffffffu, lane < own && found > A.hcap);
+                if (full && lane == 0) atomicAdd(A.over, (uint32_t)__popc(full));
+            }
         }
     }
     if (!kFirst && count_use) report();
@@ -549,6 +652,7 @@ RowArgs row_args(const StepView &s) {
     A.ps_grid = s.ps_grid;
     A.moved = s.moved;
     A.lasting = s.lasting;
+    A.inv_h = 1.f / s.ph.h;
     A.skin = kRowSkin * s.ph.h;
     const float reach = (s.ph.h + A.skin) * 1.00001f;
     A.skin_r2 = reach * reach;
@@ -639,11 +743,15 @@ cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaS
     return s.ph.fast_root ? velocity_as<true>(s, ps, st, between) : velocity_as<false>(s, ps, st, between);
 }
 
-// Particles of a group: small scenes have too few cells to fill the GPU, and the ref
-// profile's constants clump the fluid into few crowded ones, so a cell's particles go to
-// several warps.
+// Particles of a group.  A cell's setup is shared by the particles of its group, but small
+// scenes have too few cells to fill the GPU, and the ref profile's constants clump the fluid
+// into few crowded ones, so a cell's particles go to several warps.  us a step, groups that
+// end at multiples of 4 / 8 / 16 / 256: baseline 4 k 144 / 147 / 152 / 152, 14 k 163 / 158 /
+// 159 / 158, 50 k 235 / 227 / 223 / 222, 110 k 311 / 295 / 285 / 276; ref 14 k - / 441 / 471
+// / -, 50 k - / 594 / 589 / -, 262 k - / 1511 / 1472 / -.
 uint32_t row_group_mask(int profile, uint64_t n) {
-    return n < 24000 ? 3u : profile == FGB_PROFILE_REF ? 7u : 31u;
+    if (profile == FGB_PROFILE_REF) return n < 65536 ? 7u : 15u;
+    return n < 8000 ? 3u : 255u;
 }
 
 }  // namespace fgb

@@ -101,3 +101,23 @@ def test_row_ends(profile, n):
 def test_rows_asked_for_ahead(n):
     # at either side of the size from which the passes prefetch their rows
     _same(capi.PROFILE_BASELINE, [_cloud(n, 36, n, obstacles=11)], 3)
+
+
+@pytest.mark.parametrize("profile", PROFILES)
+@pytest.mark.parametrize("n", [7999, 8001, 65535, 65537])
+def test_group_sizes(profile, n):
+    _same(profile, [_cloud(n, 10 if n < 10000 else 20, n)], 3)
+
+
+@pytest.mark.parametrize("profile", PROFILES)
+@pytest.mark.parametrize("first", [False, True])
+def test_particles_far_from_their_cell(profile, first):
+    # outside the grid, where the edge cells hold them at any distance; beyond 16 bits; not a
+    # number; and (crowded) pushed across several cells by the first correction
+    made, crowd = _cloud(6000, 8, 11), _cloud(2000, 2, 12, speed=300.0)
+    p = made[0]["position"].reshape(-1, 3)
+    at = slice(0, 40) if first else slice(5000, 5040)
+    p[at] = np.linspace(-3.0, 4.0, 120, dtype=np.float32).reshape(40, 3)
+    p[at.start + 40] = (1e30, 0.1, 0.1)
+    p[at.start + 41] = (np.nan, 0.2, 0.2)
+    _same(profile, [made, crowd], 3)
