@@ -61,6 +61,8 @@ struct RowArgs {
     const float4 *ps_grid;       // the grid positions
     uint32_t *moved;             // largest movement in a cell since then (float bits), at its first particle
     uint8_t *lasting;            // per group: its rows are the first search's, with the skin
+    uint32_t *stale;             // first particles of the groups that a later search goes through
+    uint32_t *stale_count;
     float inv_h;
     float skin, skin_r2;         // the skin, and (h + skin)^2
     const RowPolicy *policy;     // per scene, of the step before; policy_next of this one
@@ -75,6 +77,7 @@ __device__ __forceinline__ uint4 *row_of(const RowArgs &A, uint32_t a) {
 
 constexpr uint32_t kCellBlock = 128, kCellWarps = kCellBlock / 32;
 constexpr uint32_t kFetchFrom = 400000;   // particles from which the passes ask for their rows ahead
+constexpr uint32_t kListFrom = 100000;    // particles from which stale groups are listed first
 constexpr float kRowSkin = 0.1f;          // the skin of rows that last, in h
 constexpr uint32_t kHeldAll = 256;        // candidates a warp holds at a time
 constexpr uint32_t kList = 4;             // particles whose hits are collected before they are written
@@ -172,16 +175,94 @@ struct Pairs {
 // before its sign is settled add 2 * 2^-11 (it stays within 2): below 0.0086 in all.
 constexpr float kHalfReach = 2.f, kHalfMargin = 0.0087f;
 
-// kFirst: the step's first search (the grid positions); else a later one, which leaves the
-// groups whose rows still last.
-template <bool kFirst>
+enum Search {
+    kFirstSearch,  // the step's first one (the grid positions): all groups
+    kLaterSearch,  // leaves the groups whose rows still last
+    kStaleSearch,  // goes through the groups that k_stale_groups listed
+};
+
+// The groups whose rows do not last for the next search, by a thread each.
+//
+// Where most rows last a search comes down to this question, and a warp that asks it of one
+// group at a time mostly waits.  A calm search of 1 M particles takes 34 us with this list
+// and 60 without (steps of 1.43 and 1.54 ms; at step 100, where no row lasts, 2.12 and
+// 2.13); 262 k 461 and 484 us a step, 110 k 271 and 276, 50 k 228 and 219, 14 k 181 and 162:
+// hence kListFrom.  With the ref profile's constants hardly any row lasts (262 k 1480 and
+// 1466): its searches ask as they go.  L1 lookups bound it, 54 scattered ones a group.
+__global__ void __launch_bounds__(128, 8) k_stale_groups(RowArgs A, uint32_t n_scenes, int count_use) {
+    const uint32_t groups = *A.group_count, lane = threadIdx.x & 31u;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t c0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < groups; c0 += stride) {
+        const uint32_t c = c0 + lane;
+        bool stale = false, lasts = false;
+        uint32_t first = 0, scene = 0, own = 0;
+        if (c < groups) {
+            first = A.groups[c];
+            lasts = A.lasting[c] != 0;
+            stale = !lasts;
+        }
+        if (lasts || (count_use && c < groups)) {
+            const uint32_t key = A.keys[first], m = morton_of(key, A.mbits);
+            scene = scene_of(key, A.mbits);
+            const SceneDev &S = A.scenes[scene];
+            const uint32_t end = min(__ldg(&A.cells[S.table_base + m]).y, (first | A.group_mask) + 1);
+            own = end > first ? end - first : 0u;
+            if (lasts) {
+                uint32_t most = 0, mine = 0;
+#pragma unroll 1
+                for (int dz = -1; dz <= 1; ++dz) {
+                    uint2 range[9];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        uint32_t cell;
+                        range[k] = make_uint2(0, 0);
+                        if (neighbour_cell(S, m, k % 3 - 1, k / 3 - 1, dz, cell)) range[k] = __ldg(&A.cells[cell]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        const uint32_t moved = range[k].y > range[k].x ? __ldg(&A.moved[range[k].x]) : 0u;
+                        most = max(most, moved);
+                        if (k == 4 && dz == 0) mine = moved;
+                    }
+                }
+                stale = !(__uint_as_float(mine) + __uint_as_float(most) <= A.skin);
+                if (stale) A.lasting[c] = 0;
+            }
+        }
+        const unsigned list = __ballot_sync(0xffffffffu, stale);
+        if (list) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(A.stale_count, (uint32_t)__popc(list));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(list & lanemask_lt());
+            if (stale) A.stale[at] = first;
+        }
+        if (count_use) {  // particles asked and those that use their rows, a scene at a time
+            unsigned rest = __ballot_sync(0xffffffffu, own != 0);
+            while (rest) {
+                const uint32_t s0 = __shfl_sync(0xffffffffu, scene, __ffs(rest) - 1);
+                const bool in = own != 0 && scene == s0;
+                const uint32_t asked = __reduce_add_sync(0xffffffffu, in ? own : 0u),
+                               used = __reduce_add_sync(0xffffffffu, in && !stale ? own : 0u);
+                if (lane == 0) {
+                    atomicAdd(&A.policy_next[s0].asked, asked);
+                    if (used) atomicAdd(&A.policy_next[s0].used, used);
+                }
+                rest &= ~__ballot_sync(0xffffffffu, in);
+            }
+        }
+    }
+}
+
+template <Search kSearch>
 __global__ void __launch_bounds__(kCellBlock, 7)
     k_cell_rows(RowArgs A, const float4 *__restrict__ ps, float r2max, uint32_t n_scenes, int count_use) {
+    constexpr bool kFirst = kSearch == kFirstSearch;
     __shared__ CellShared s_warp[kCellWarps];
     const uint32_t lane = threadIdx.x & 31u;
     CellShared &sh = s_warp[threadIdx.x >> 5];
     const uint32_t lists = (uint32_t)__cvta_generic_to_shared(sh.hits);
-    const uint32_t warps = gridDim.x * kCellWarps, groups = *A.group_count;
+    const uint32_t *list = kSearch == kStaleSearch ? A.stale : A.groups;
+    const uint32_t warps = gridDim.x * kCellWarps, groups = kSearch == kStaleSearch ? *A.stale_count : *A.group_count;
     if (kFirst && blockIdx.x == 0)
         for (uint32_t k = threadIdx.x; k < n_scenes; k += kCellBlock) A.policy_next[k] = decide(A.policy[k]);
     // the lane's neighbour cell: x fastest; lanes 27 to 31 have none
@@ -196,7 +277,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
         asked = used = 0;
     };
     for (uint32_t c = blockIdx.x * kCellWarps + (threadIdx.x >> 5); c < groups; c += warps) {
-        const uint32_t first = A.groups[c], key = A.keys[first], scene = scene_of(key, A.mbits);
+        const uint32_t first = list[c], key = A.keys[first], scene = scene_of(key, A.mbits);
         const SceneDev &S = A.scenes[scene];
         uint32_t cell;
         uint2 range = make_uint2(0, 0);
@@ -208,7 +289,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
             const bool keep = decide(A.policy[scene]).keep != 0;
             if (keep) reach2 = A.skin_r2;
             if (lane == 0) A.lasting[c] = keep ? 1 : 0;
-        } else {
+        } else if (kSearch == kLaterSearch) {
             const bool lasts = A.lasting[c] != 0;
             const uint32_t m = count ? __ldg(&A.moved[from]) : 0u;
             const float bound = __uint_as_float(__shfl_sync(0xffffffffu, m, 13)) +
@@ -381,7 +462,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
             }
         }
     }
-    if (!kFirst && count_use) report();
+    if (kSearch == kLaterSearch && count_use) report();
 }
 
 // The 27-cell walk, for rows that overflowed.
@@ -652,6 +733,8 @@ RowArgs row_args(const StepView &s) {
     A.ps_grid = s.ps_grid;
     A.moved = s.moved;
     A.lasting = s.lasting;
+    A.stale = s.stale;
+    A.stale_count = nullptr;
     A.inv_h = 1.f / s.ph.h;
     A.skin = kRowSkin * s.ph.h;
     const float reach = (s.ph.h + A.skin) * 1.00001f;
@@ -681,13 +764,21 @@ cudaError_t rows_of(const StepView &s, const float4 *ps, uint32_t pass, cudaStre
     cudaError_t e;
     if (pass == 0) {
         if (s.over) A.over = s.over + 1;  // counted once a step
-        e = resident_grid(k_cell_rows<true>, s, kCellBlock, &grid);
+        e = resident_grid(k_cell_rows<kFirstSearch>, s, kCellBlock, &grid);
         if (e != cudaSuccess) return e;
-        k_cell_rows<true><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, 0);
+        k_cell_rows<kFirstSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, 0);
+    } else if (s.ph.profile == FGB_PROFILE_REF || s.n < kListFrom) {
+        e = resident_grid(k_cell_rows<kLaterSearch>, s, kCellBlock, &grid);
+        if (e != cudaSuccess) return e;
+        k_cell_rows<kLaterSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, pass == 1);
     } else {
-        e = resident_grid(k_cell_rows<false>, s, kCellBlock, &grid);
+        A.stale_count = s.group_count + pass;  // one a pass, zeroed with the groups' number
+        e = resident_grid(k_stale_groups, s, 128, &grid);
         if (e != cudaSuccess) return e;
-        k_cell_rows<false><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, pass == 1);
+        k_stale_groups<<<grid, 128, 0, st>>>(A, s.n_scenes, pass == 1);
+        e = resident_grid(k_cell_rows<kStaleSearch>, s, kCellBlock, &grid);
+        if (e != cudaSuccess) return e;
+        k_cell_rows<kStaleSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, 0);
     }
     return cudaGetLastError();
 }

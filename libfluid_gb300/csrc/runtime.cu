@@ -592,6 +592,7 @@ struct fgb_batch {
     uint32_t cell_hits = 96;  // entries of a hit row of rows.cu
     uint32_t group_mask = 31;
     Dev<uint32_t> groups, group_count, moved;
+    Dev<uint32_t> stale;  // per search, the first particles of the groups it goes through
     Dev<uint8_t> lasting;
     Dev<RowPolicy> row_policy[2];  // by the state set a step reads
     Dev<float> lambda, density;
@@ -725,6 +726,7 @@ struct fgb_batch {
         s.group_count = group_count.p;
         s.group_mask = group_mask;
         s.moved = moved.p;
+        s.stale = stale.p;
         s.lasting = lasting.p;
         s.row_policy = row_policy[c].p;
         s.row_policy_next = row_policy[c ^ 1].p;
@@ -768,7 +770,8 @@ struct fgb_batch {
                      "step: clear tile counters");
         FGB_CUDA(cudaMemsetAsync(mass_range.p, 0xff, 2 * sizeof(uint32_t), st), "step: clear mass range");
         if (cell_rows)
-            FGB_CUDA(cudaMemsetAsync(group_count.p, 0, sizeof(uint32_t), st), "step: clear group count");
+            FGB_CUDA(cudaMemsetAsync(group_count.p, 0, group_count.n * sizeof(uint32_t), st),
+                     "step: clear group counts");
         if (s.cap && cellmax.p)
             FGB_CUDA(cudaMemsetAsync(cellmax.p, 0, cells_n * sizeof(uint32_t), st), "step: clear cellmax");
         launch_reorder_cells(s, st);
@@ -1256,7 +1259,8 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
         FGB_CUDA(b->groups.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->lasting.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->moved.alloc(cap), "batch alloc groups");
-        FGB_CUDA(b->group_count.alloc(1), "batch alloc groups");
+        FGB_CUDA(b->stale.alloc(cap), "batch alloc groups");
+        FGB_CUDA(b->group_count.alloc(2 + b->iterations), "batch alloc groups");
         int rc = b->alloc_cell_rows(cap);
         if (rc) return rc;
     }

@@ -121,3 +121,10 @@ def test_particles_far_from_their_cell(profile, first):
     p[at.start + 40] = (1e30, 0.1, 0.1)
     p[at.start + 41] = (np.nan, 0.2, 0.2)
     _same(profile, [made, crowd], 3)
+
+
+@pytest.mark.parametrize("n", [99999, 100001])
+def test_stale_groups_listed_first(n):
+    # at either side of the size from which a later search lists its groups first, calm and not
+    _same(capi.PROFILE_BASELINE, [_cloud(n, 24, n, obstacles=13, speed=0.2)], 6)
+    _same(capi.PROFILE_BASELINE, [_cloud(n - 700, 24, n), _cloud(700, 5, n, speed=30.0)], 4)
