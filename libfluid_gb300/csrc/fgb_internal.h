@@ -22,7 +22,11 @@ uint64_t radix_scratch_bytes(uint64_t n);
 int radix_passes(uint32_t key_bits);
 cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
                              uint32_t *vals_out, uint64_t n, uint32_t key_bits, void *scratch,
-                             uint64_t scratch_bytes, cudaStream_t stream, uint32_t *err, uint64_t *launches);
+                             uint64_t scratch_bytes, cudaStream_t stream, uint32_t *err, uint64_t *launches,
+                             const uint32_t *counted);
+// What a sort with `counted` (the digits' counts of its keys, digit_counts.cuh) asks to be
+// zero before it: `words` from the returned address.
+uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t *words);
 
 // Copy a device error-flag word to *flags and clear it, after the work queued on
 // stream (synchronises the stream; allocates nothing).
@@ -64,6 +68,16 @@ struct StepView {
     uint32_t *keys_in, *vals_in, *keys_sorted, *vals_sorted;
     uint2 *cells;
     uint64_t cells_n;
+    // the table holds the cells of the last step's keys (0) or of the last surface's (1):
+    // whoever builds the next grid empties those cells alone
+    uint32_t *cells_of;
+    const uint32_t *surface_keys;
+    // counts of the step's key digits, and those of the next step (zeroed by this one)
+    uint32_t *digits, *digits_next;
+    int sort_passes;
+    uint32_t *sort_state;  // zeroed with them (radix_state)
+    uint64_t sort_state_n;
+    uint32_t group_counts;  // words at group_count
     float4 *ps_a, *ps_b;
     float *lambda, *density;
     // the lambda pass's p* with lambda in w (the delta pass's neighbour reads; null: off)

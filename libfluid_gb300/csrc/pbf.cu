@@ -17,6 +17,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "digit_counts.cuh"
 #include "fgb_internal.h"
 #include "pbf_sums.cuh"
 
@@ -71,19 +72,76 @@ __device__ __forceinline__ void for_neighbours(const SceneDev &S, const uint2 *_
     for_neighbour_cells(S, cells, (int)compact10(m), (int)compact10(m >> 1), (int)compact10(m >> 2), f);
 }
 
-__global__ void k_predict_keys(const SceneDev *__restrict__ scenes, const WellDev *__restrict__ wells, Phys ph,
-                               uint32_t n, uint32_t mbits, const uint32_t *__restrict__ keys_prev,
-                               const float4 *__restrict__ x, const float4 *__restrict__ v,
-                               const int32_t *__restrict__ type, uint32_t *__restrict__ keys_out,
-                               uint32_t *__restrict__ vals_out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// The cells that the table holds, for the kernel that begins the next grid to empty.  Only
+// a few of a table's cells are occupied: to clear it all takes a step of 1 M particles (134
+// MB) 20 us, these stores and the digit counts 10.
+struct OldCells {
+    uint2 *cells;
+    uint64_t cells_n;
+    const uint32_t *step_keys, *surface_keys, *of;
+
+    __device__ __forceinline__ const uint32_t *keys() const { return *of ? surface_keys : step_keys; }
+    // the cell that particle i of the old grid begins
+    __device__ __forceinline__ void clear(const SceneDev *scenes, uint32_t mbits, const uint32_t *k, uint32_t i) const {
+        const uint32_t key = k[i];
+        if (i > 0 && k[i - 1] == key) return;
+        const uint64_t c = (uint64_t)scenes[scene_of(key, mbits)].table_base + morton_of(key, mbits);
+        if (c < cells_n) cells[c] = make_uint2(0u, 0u);
+    }
+};
+
+OldCells old_cells(const StepView &s) {
+    return OldCells{s.cells, s.cells_n, s.keys_prev, s.surface_keys, s.cells_of};
+}
+
+// What a step finds at its beginning, set by its first kernel: counters at zero, and the
+// sort's.  (As a memset each, and with a kernel each to count the digits and to sum the
+// counts, a step of 4096 particles took 144 us, 134 now; one of 14 k 159 and 150.)
+struct StepBegin {
+    uint32_t *mass_range, *over, *group_count, *digits_next, *sort_state;
+    uint32_t group_counts;
+    uint64_t sort_state_n;
+
+    __device__ __forceinline__ void run() const {
+        const uint64_t t = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+        for (uint64_t i = t; i < sort_state_n; i += all) sort_state[i] = 0;
+        for (uint64_t i = t; i < kMaxPasses * kRadix; i += all) digits_next[i] = 0;
+        for (uint64_t i = t; group_count && i < group_counts; i += all) group_count[i] = 0;
+        if (t < 2) {
+            mass_range[t] = 0xffffffffu;
+            if (over) over[t] = 0;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(256)
+    k_predict_keys(const SceneDev *__restrict__ scenes, const WellDev *__restrict__ wells, Phys ph, uint32_t n,
+                   uint32_t mbits, const uint32_t *__restrict__ keys_prev, const float4 *__restrict__ x,
+                   const float4 *__restrict__ v, const int32_t *__restrict__ type, uint32_t *__restrict__ keys_out,
+                   uint32_t *__restrict__ vals_out, OldCells old, StepBegin begin, uint32_t *__restrict__ digits,
+                   int passes) {
+    __shared__ DigitCounts counts;
+    counts.clear();
+    begin.run();
+    const uint32_t *old_keys = old.keys();
+    __syncthreads();
+    // a CTA's particles in a row: their keys share the high digits, and the CTA has few
+    // counts to give
+    const uint32_t share = ((n + gridDim.x - 1) / gridDim.x + 255u) & ~255u, from = blockIdx.x * share;
+    const uint32_t to = from < n ? min(n - from, share) + from : 0u;
+    for (uint32_t i = from + threadIdx.x; i < to; i += blockDim.x) {
         const uint32_t s = scene_of(keys_prev[i], mbits);
         const SceneDev &S = scenes[s];
         const float3 p = predict(ph, S, wells, type[i], x[i], v[i]);
         const uint32_t m = cell_key(S, ph.h, p.x, p.y, p.z);
-        keys_out[i] = (mbits >= 32 ? 0u : (s << mbits)) | m;
+        const uint32_t key = (mbits >= 32 ? 0u : (s << mbits)) | m;
+        keys_out[i] = key;
         vals_out[i] = i;
+        old.clear(scenes, mbits, old_keys, i);
+        counts.add(key, passes);
     }
+    __syncthreads();
+    counts.give(digits, passes);
 }
 
 // Gather the state into sorted order, recompute p* there (same bits as
@@ -97,47 +155,57 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
                                 uint32_t *__restrict__ col1, uint32_t *__restrict__ slot1,
                                 float4 *__restrict__ ps, uint2 *__restrict__ cells, uint64_t cells_n,
                                 uint32_t *err, uint32_t *mass_range, uint32_t *__restrict__ groups,
-                                uint32_t *group_count, uint32_t group_mask) {
+                                uint32_t *group_count, uint32_t group_mask, uint32_t *cells_of) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *cells_of = 0;
     // the smallest mass's bits and the complement of the largest's, both by atomicMin
     // (one pair per CTA); the masses are all equal when range[0] == ~range[1]
-    __shared__ uint32_t s_lo, s_hi;
+    __shared__ uint32_t s_lo, s_hi, s_groups, s_at;
     if (threadIdx.x == 0) s_lo = s_hi = 0xffffffffu;
     __syncthreads();
     uint32_t lo = 0xffffffffu, hi = 0xffffffffu;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t j = vals[i];
-        const uint32_t key = keys[i];
-        const uint32_t s = scene_of(key, mbits);
-        const SceneDev &S = scenes[s];
-        const float4 xj = x0[j], vj = v0[j];
-        const int32_t tj = type0[j];
-        const float3 p = predict(ph, S, wells, tj, xj, vj);
-        x1[i] = xj;
-        v1[i] = vj;
-        type1[i] = tj;
-        col1[i] = col0[j];
-        slot1[i] = slot0[j];
-        ps[i] = make_float4(p.x, p.y, p.z, xj.w);
-        lo = min(lo, __float_as_uint(xj.w));
-        hi = min(hi, ~__float_as_uint(xj.w));
-        if (groups) {  // list the groups of each cell's particles, one atomic a warp
-            const bool start = (i & group_mask) == 0 || keys[i - 1] != key;
-            const unsigned m = __activemask(), b = __ballot_sync(m, start);
-            if (b) {
-                const int leader = __ffs(m) - 1;
-                uint32_t at = 0;
-                if ((int)(threadIdx.x & 31u) == leader) at = atomicAdd(group_count, (uint32_t)__popc(b));
-                at = __shfl_sync(m, at, leader);
-                if (start) groups[at + __popc(b & lanemask_lt())] = i;
+    for (uint32_t from = blockIdx.x * blockDim.x; from < n; from += gridDim.x * blockDim.x) {
+        const uint32_t i = from + threadIdx.x;
+        bool start = false;  // of a group
+        if (i < n) {
+            const uint32_t j = vals[i];
+            const uint32_t key = keys[i];
+            const uint32_t s = scene_of(key, mbits);
+            const SceneDev &S = scenes[s];
+            const float4 xj = x0[j], vj = v0[j];
+            const int32_t tj = type0[j];
+            const float3 p = predict(ph, S, wells, tj, xj, vj);
+            x1[i] = xj;
+            v1[i] = vj;
+            type1[i] = tj;
+            col1[i] = col0[j];
+            slot1[i] = slot0[j];
+            ps[i] = make_float4(p.x, p.y, p.z, xj.w);
+            lo = min(lo, __float_as_uint(xj.w));
+            hi = min(hi, ~__float_as_uint(xj.w));
+            const bool first = i == 0 || keys[i - 1] != key;
+            start = first || (i & group_mask) == 0;
+            const uint64_t c = (uint64_t)S.table_base + morton_of(key, mbits);
+            if (c >= cells_n) {
+                raise_error(err, ERR_CELL_RANGE);
+            } else {
+                if (first) cells[c].x = i;
+                if (i + 1 == n || keys[i + 1] != key) cells[c].y = i + 1;
             }
         }
-        const uint64_t c = (uint64_t)S.table_base + morton_of(key, mbits);
-        if (c >= cells_n) {
-            raise_error(err, ERR_CELL_RANGE);
-            continue;
+        if (groups) {
+            // list the groups of each cell's particles, by one atomic a CTA (one a warp cost
+            // 8 us of 38 at 1 M particles, and left the list in less order)
+            const unsigned starts = __ballot_sync(0xffffffffu, start);
+            if (threadIdx.x == 0) s_groups = 0;
+            __syncthreads();
+            uint32_t at = 0;
+            if ((threadIdx.x & 31u) == 0 && starts) at = atomicAdd(&s_groups, (uint32_t)__popc(starts));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(starts & lanemask_lt());
+            __syncthreads();
+            if (threadIdx.x == 0) s_at = atomicAdd(group_count, s_groups);
+            __syncthreads();
+            if (start) groups[s_at + at] = i;
         }
-        if (i == 0 || keys[i - 1] != key) cells[c].x = i;
-        if (i + 1 == n || keys[i + 1] != key) cells[c].y = i + 1;
     }
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_min_sync(0xffffffffu, hi);
@@ -980,7 +1048,8 @@ __global__ void k_list_policy(uint32_t *policy, uint32_t n_scenes, uint32_t min_
 // Keys of the current positions (marching-cubes grid).
 __global__ void k_position_keys(const SceneDev *__restrict__ scenes, Phys ph, uint32_t n, uint32_t mbits,
                                 const uint32_t *__restrict__ keys_prev, const float4 *__restrict__ x,
-                                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out) {
+                                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, OldCells old) {
+    const uint32_t *old_keys = old.keys();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t s = scene_of(keys_prev[i], mbits);
         const SceneDev &S = scenes[s];
@@ -988,6 +1057,7 @@ __global__ void k_position_keys(const SceneDev *__restrict__ scenes, Phys ph, ui
         const uint32_t m = cell_key(S, ph.h, xi.x / S.scale, xi.y / S.scale, xi.z / S.scale);
         keys_out[i] = (mbits >= 32 ? 0u : (s << mbits)) | m;
         vals_out[i] = i;
+        old.clear(scenes, mbits, old_keys, i);
     }
 }
 
@@ -996,7 +1066,9 @@ __global__ void k_gather_positions(const SceneDev *__restrict__ scenes, uint32_t
                                    const float4 *__restrict__ x, const int32_t *__restrict__ type,
                                    const uint32_t *__restrict__ col, float4 *__restrict__ xs,
                                    int32_t *__restrict__ type_s, uint32_t *__restrict__ col_s,
-                                   uint2 *__restrict__ cells, uint64_t cells_n, uint32_t *err) {
+                                   uint2 *__restrict__ cells, uint64_t cells_n, uint32_t *err,
+                                   uint32_t *cells_of) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *cells_of = 1;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t j = vals[i];
         const uint32_t key = keys[i];
@@ -1096,14 +1168,18 @@ void launch_fill_u32(uint32_t *p, uint64_t n, uint32_t value, cudaStream_t st) {
 
 void launch_predict_keys(const StepView &s, cudaStream_t st) {
     k_predict_keys<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.wells, s.ph, s.n, s.mbits, s.keys_prev, s.x0, s.v0,
-                                                     s.type0, s.keys_in, s.vals_in);
+                                                     s.type0, s.keys_in, s.vals_in, old_cells(s),
+                                                     StepBegin{s.mass_range, s.over, s.group_count, s.digits_next,
+                                                               s.sort_state, s.group_counts, s.sort_state_n},
+                                                     s.digits, s.sort_passes);
 }
 
 void launch_reorder_cells(const StepView &s, cudaStream_t st) {
     k_reorder_cells<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.wells, s.ph, s.n, s.mbits, s.keys_sorted,
                                                       s.vals_sorted, s.x0, s.v0, s.type0, s.col0, s.slot0, s.x1,
                                                       s.v1, s.type1, s.col1, s.slot1, s.ps_grid, s.cells, s.cells_n,
-                                                      s.err, s.mass_range, s.groups, s.group_count, s.group_mask);
+                                                      s.err, s.mass_range, s.groups, s.group_count, s.group_mask,
+                                                      s.cells_of);
 }
 
 // Grid and tile counter of one gather launch (slot: its place among the step's
@@ -1197,14 +1273,14 @@ void launch_diffuse(const StepView &s, uint4 *agg, uint32_t *count, cudaStream_t
 
 void launch_position_keys(const StepView &s, const float4 *x, cudaStream_t st) {
     k_position_keys<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.ph, s.n, s.mbits, s.keys_prev, x, s.keys_in,
-                                                      s.vals_in);
+                                                      s.vals_in, old_cells(s));
 }
 
 void launch_gather_positions(const StepView &s, const float4 *x, const int32_t *type, const uint32_t *col,
                              float4 *xs_sorted, int32_t *type_sorted, uint32_t *col_sorted, cudaStream_t st) {
     k_gather_positions<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.n, s.mbits, s.keys_sorted, s.vals_sorted, x,
                                                          type, col, xs_sorted, type_sorted, col_sorted, s.cells,
-                                                         s.cells_n, s.err);
+                                                         s.cells_n, s.err, s.cells_of);
 }
 
 }  // namespace fgb

@@ -36,6 +36,7 @@
 #include <unistd.h>
 
 #include "fast_root.h"
+#include "digit_counts.cuh"
 #include "fgb_internal.h"
 
 namespace fgb {
@@ -593,6 +594,8 @@ struct fgb_batch {
     uint32_t group_mask = 31;
     Dev<uint32_t> groups, group_count, moved;
     Dev<uint32_t> stale;  // per search, the first particles of the groups it goes through
+    Dev<uint32_t> cells_of;   // StepView::cells_of
+    Dev<uint32_t> digits[2];  // counts of the key digits, of the steps that read state set 0 and 1
     Dev<uint8_t> lasting;
     Dev<RowPolicy> row_policy[2];  // by the state set a step reads
     Dev<float> lambda, density;
@@ -606,6 +609,7 @@ struct fgb_batch {
     Dev<uint32_t> err;
     // cell queries: the cell table is the last step's grid until the next upload, edit
     // or surface replaces it
+    bool grid_unknown = true;     // fresh_grid has to run before the next step or surface
     bool query_ok = false;
     Dev<fgb_query> q_dev;
     Dev<uint32_t> q_out;
@@ -681,6 +685,13 @@ struct fgb_batch {
         s.vals_sorted = vals_sorted.p;
         s.cells = cells.p;
         s.cells_n = cells_n;
+        s.cells_of = cells_of.p;
+        s.surface_keys = mc_keys.p;
+        s.digits = digits[c].p;
+        s.digits_next = digits[c ^ 1].p;
+        s.sort_passes = radix_passes(key_bits);
+        s.sort_state = radix_state(n, key_bits, sort_scratch.p, &s.sort_state_n);
+        s.group_counts = (uint32_t)group_count.n;
         s.ps_a = ps[0].p;
         s.ps_b = ps[1].p;
         s.lambda = lambda.p;
@@ -754,24 +765,18 @@ struct fgb_batch {
         StepView s = view(c);
         uint64_t l = 0;
         uint32_t k = 0;
-        if (over.p) FGB_CUDA(cudaMemsetAsync(over.p, 0, 2 * sizeof(uint32_t), st), "step: overflow counters");
         mark(k, st);
         launch_predict_keys(s, st);
         l += 1;
         mark(k, st);
         cudaError_t e = radix_sort_pairs(keys_in.p, vals_in.p, keys_sorted.p, vals_sorted.p, n, key_bits,
-                                         sort_scratch.p, sort_scratch_bytes, st, err.p, &l);
+                                         sort_scratch.p, sort_scratch_bytes, st, err.p, &l, s.digits);
         if (e != cudaSuccess) return fail_cuda(e, "step: radix sort");
         mark(k, st);
         if (io_up) FGB_CUDA(cudaStreamWaitEvent(st, io_up, cudaEventWaitExternal), "step: upload event");
-        FGB_CUDA(cudaMemsetAsync(cells.p, 0, cells_n * sizeof(uint2), st), "step: clear cells");
         if (persistent && !cell_rows)
             FGB_CUDA(cudaMemsetAsync(queue.p, 0, slots_of_step(iterations) * sizeof(uint32_t), st),
                      "step: clear tile counters");
-        FGB_CUDA(cudaMemsetAsync(mass_range.p, 0xff, 2 * sizeof(uint32_t), st), "step: clear mass range");
-        if (cell_rows)
-            FGB_CUDA(cudaMemsetAsync(group_count.p, 0, group_count.n * sizeof(uint32_t), st),
-                     "step: clear group counts");
         if (s.cap && cellmax.p)
             FGB_CUDA(cudaMemsetAsync(cellmax.p, 0, cells_n * sizeof(uint32_t), st), "step: clear cellmax");
         launch_reorder_cells(s, st);
@@ -1067,6 +1072,18 @@ struct fgb_batch {
         return FGB_OK;
     }
 
+    // Where the sorted keys no longer tell which cells the table holds: an empty table, and
+    // the counts that a step leaves for the next one.
+    int fresh_grid() {
+        if (!grid_unknown) return FGB_OK;
+        FGB_CUDA(cudaMemsetAsync(cells.p, 0, cells_n * sizeof(uint2), stream()), "clear cells");
+        FGB_CUDA(cudaMemsetAsync(cells_of.p, 0, sizeof(uint32_t), stream()), "clear cells");
+        for (auto &d : digits)
+            FGB_CUDA(cudaMemsetAsync(d.p, 0, kMaxPasses * kRadix * sizeof(uint32_t), stream()), "clear digit counts");
+        grid_unknown = false;
+        return FGB_OK;
+    }
+
     int step(uint32_t steps) {
         int rc = grow_rows();
         if (rc) return rc;
@@ -1074,6 +1091,10 @@ struct fgb_batch {
         if (rc) return rc;
         if (!graphs_ok) {
             rc = build_graphs();
+            if (rc) return rc;
+        }
+        if (steps) {
+            rc = fresh_grid();
             if (rc) return rc;
         }
         for (uint32_t k = 0; k < steps; ++k) {
@@ -1088,7 +1109,6 @@ struct fgb_batch {
     int ensure_surface() {
         if (surf_ready) return FGB_OK;
         PoolScope scope(&solver->pool);
-        FGB_CUDA(mc_keys.alloc(n), "surface alloc");
         FGB_CUDA(mc_vals.alloc(n), "surface alloc");
         FGB_CUDA(mc_xs.alloc(n), "surface alloc");
         FGB_CUDA(mc_type.alloc(n), "surface alloc");
@@ -1108,6 +1128,7 @@ struct fgb_batch {
     int surface_count(uint32_t b, uint32_t e, uint64_t *tri_total) {
         int rc = sync_tris();  // the scene table (obstacle counts) as of the last upload
         if (!rc) rc = ensure_surface();
+        if (!rc) rc = fresh_grid();
         if (rc) return rc;
         query_ok = false;  // the cell table becomes the grid of the current positions
         cudaStream_t st = stream();
@@ -1116,9 +1137,8 @@ struct fgb_batch {
         launch_position_keys(s, x[cur].p, st);
         launches += 1;
         cudaError_t ce = radix_sort_pairs(keys_in.p, vals_in.p, mc_keys.p, mc_vals.p, n, key_bits, sort_scratch.p,
-                                          sort_scratch_bytes, st, err.p, &launches);
+                                          sort_scratch_bytes, st, err.p, &launches, nullptr);
         if (ce != cudaSuccess) return fail_cuda(ce, "surface: sort");
-        FGB_CUDA(cudaMemsetAsync(cells.p, 0, cells_n * sizeof(uint2), st), "surface: clear cells");
         s.keys_sorted = mc_keys.p;
         s.vals_sorted = mc_vals.p;
         launch_gather_positions(s, x[cur].p, type[cur].p, col[cur].p, mc_xs.p, mc_type.p, mc_col.p, st);
@@ -1252,6 +1272,10 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     FGB_CUDA(b->vals_in.alloc(cap), "batch alloc");
     FGB_CUDA(b->keys_sorted.alloc(cap), "batch alloc");
     FGB_CUDA(b->vals_sorted.alloc(cap), "batch alloc");
+    FGB_CUDA(b->mc_keys.alloc(cap), "batch alloc");  // of the surface; the steps' first kernel may read them
+    b->grid_unknown = true;
+    FGB_CUDA(b->cells_of.alloc(1), "batch alloc");
+    for (auto &d : b->digits) FGB_CUDA(d.alloc(kMaxPasses * kRadix), "batch alloc");
     b->sort_scratch_bytes = radix_scratch_bytes(cap);
     FGB_CUDA(b->sort_scratch.alloc(b->sort_scratch_bytes), "batch alloc");
     FGB_CUDA(b->ps_grid.alloc(cap + 1), "batch alloc");
@@ -1516,15 +1540,14 @@ static int sync_ids(fgb_batch *b) {
 }
 
 // What every upload ends with: the scene table learns whether the scene holds
-// obstacles, and the scene's key prefix is set in case a surface call precedes
-// the first step.
+// obstacles.  (The scene's keys keep its prefix, from the batch's creation on: sorted
+// keys stay in their scenes' segments.)
 static void upload_done(fgb_batch *b, uint32_t k, uint32_t obstacles) {
     b->query_ok = false;
     if (b->h_scenes[k].obstacles != obstacles) {
         b->h_scenes[k].obstacles = obstacles;
         b->tris_dirty = true;  // re-uploads the scene table before the next step
     }
-    launch_fill_u32(b->keys_sorted.p + b->first[k], b->counts[k], b->mbits >= 32 ? 0u : (k << b->mbits), b->stream());
 }
 
 // One kernel reads the caller's arrays and writes the scene segment (ids go to
@@ -1639,7 +1662,6 @@ static int batch_copy_scene(fgb_batch *dst, uint32_t dk, fgb_batch *src, uint32_
         FGB_CUDA(cudaMemcpyAsync(dst->ids_dev.p + fd, src->ids_dev.p + fs, n * sizeof(uint64_t),
                                  cudaMemcpyDeviceToDevice, st),
                  "copy_scene");
-        launch_fill_u32(dst->keys_sorted.p + fd, n, dst->mbits >= 32 ? 0u : (dk << dst->mbits), st);
     }
     if (src->direct && !dst->direct) {  // dst keeps its ids on the host
         dst->ids[dk].assign(n, 0);
@@ -2325,6 +2347,7 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     }
     b->ids_dev.swap(ids1);
     b->cur = cn;
+    b->grid_unknown = true;  // the keys are replaced below, and a set is stepped over
     b->counts = counts;
     b->first = first;
     b->n = n1;
@@ -2452,7 +2475,6 @@ static int advance_direct(fgb_batch *b, const fgb_config *cfg, fgb_particles *xs
     launch_pack_static(in, n, b->col[c].p, b->slot[c].p, b->ids_dev.p, io);
     FGB_CUDA(cudaGetLastError(), "advance: upload kernel");
     FGB_CUDA(cudaEventRecord(b->io_up, io), "advance: upload event");
-    launch_fill_u32(b->keys_sorted.p, n, 0u, st);  // scene 0's key prefix for the prediction
     b->ids[0].clear();
     b->ids_stale[0] = 0;
     // the step's last kernel stores positions and velocities into the caller's arrays
@@ -2560,7 +2582,6 @@ static int advance_records_direct(fgb_batch *b, const fgb_config *cfg, const Hos
                         st);
     FGB_CUDA(cudaGetLastError(), "advance: upload kernel");
     FGB_CUDA(cudaEventRecord(b->io_up, st), "advance: upload event");  // every field is in
-    launch_fill_u32(b->keys_sorted.p, n, 0u, st);  // scene 0's key prefix for the prediction
     b->ids[0].clear();
     b->ids_stale[0] = 0;
     b->query_ok = false;

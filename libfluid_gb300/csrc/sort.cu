@@ -8,25 +8,25 @@
 // Per pass (8-bit digit): each CTA takes the next tile id from an atomic counter,
 // ranks its 4096 keys with warp-level match_any (in index order, hence stable),
 // publishes its per-digit counts, looks back over earlier tiles' published counts
-// (decoupled look-back) to find where its keys start, and scatters.  A pre-pass
-// histograms all digits of all passes at once.  Every look-back wait is bounded.
+// (decoupled look-back) to find where its keys start, and scatters.  The digits of all
+// passes are counted before the first: by a kernel of their own, or by the one that makes
+// the keys (digit_counts.cuh); each tile sums the counts of its pass itself.  Every
+// look-back wait is bounded.
 #include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "digit_counts.cuh"
 #include "fgb_device.cuh"
 #include "fgb_internal.h"
 
 namespace fgb {
 namespace {
 
-constexpr int kRadixBits = 8;
-constexpr int kRadix = 1 << kRadixBits;
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 16;
 constexpr int kTile = kSortThreads * kSortItems;  // 4096 keys per tile
-constexpr int kMaxPasses = 4;
 
 constexpr uint32_t kFlagAggregate = 1u << 30;
 constexpr uint32_t kFlagInclusive = 2u << 30;
@@ -34,46 +34,24 @@ constexpr uint32_t kValueMask = (1u << 30) - 1u;
 
 __global__ void __launch_bounds__(256) k_radix_histogram(const uint32_t *__restrict__ keys, uint32_t n,
                                                          int passes, uint32_t *__restrict__ hist) {
-    __shared__ uint32_t sh[kMaxPasses][kRadix];
-    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) (&sh[0][0])[i] = 0;
+    __shared__ DigitCounts counts;
+    counts.clear();
     __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&sh[p][(k >> (p * kRadixBits)) & (kRadix - 1)], 1u);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        counts.add(keys[i], passes);
     __syncthreads();
-    for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) {
-        uint32_t v = (&sh[0][0])[i];
-        if (v) atomicAdd(&hist[i], v);
-    }
-}
-
-// Exclusive scan of each pass's 256 digit counts (one block per pass).
-__global__ void __launch_bounds__(256) k_radix_offsets(const uint32_t *__restrict__ hist,
-                                                       uint32_t *__restrict__ offsets) {
-    __shared__ uint32_t warp_tot[kSortWarps];
-    const int p = blockIdx.x, d = threadIdx.x, lane = d & 31, w = d >> 5;
-    uint32_t v = hist[p * kRadix + d];
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[w] = x;
-    __syncthreads();
-    uint32_t base = 0;
-    for (int i = 0; i < w; ++i) base += warp_tot[i];
-    offsets[p * kRadix + d] = base + x - v;
+    counts.give(hist, passes);
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
     uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n, int shift,
-    const uint32_t *__restrict__ offsets, uint32_t *status, uint32_t *tile_counter, uint32_t *err,
+    const uint32_t *__restrict__ counts, uint32_t *status, uint32_t *tile_counter, uint32_t *err,
     LookbackCtl ctl) {
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_hist[kSortWarps][kRadix + 1];
     __shared__ uint32_t s_base[kRadix + 1];
+    __shared__ uint32_t s_before[kSortWarps];
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
@@ -91,6 +69,18 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
         v[i] = ok ? vals_in[idx] : 0u;
     }
     const uint32_t lt = lanemask_lt();
+    // the keys with a digit below tid: the counts of the earlier digits
+    uint32_t below = counts[tid];
+    {
+        const uint32_t own = below;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, below, o);
+            if (lane >= o) below += y;
+        }
+        if (lane == 31) s_before[w] = below;
+        below -= own;
+    }
 #pragma unroll
     for (int i = 0; i < kSortItems; ++i) {
         uint32_t idx = base + (uint32_t)i * 32u + (uint32_t)lane;
@@ -141,7 +131,8 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
             }
             if (publish) st_relaxed(my, kFlagInclusive | (excl + run));
         }
-        s_base[d] = offsets[d] + excl;
+        for (int ww = 0; ww < w; ++ww) below += s_before[ww];
+        s_base[d] = below + excl;
     }
     __syncthreads();
 
@@ -162,7 +153,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
 }
 
 struct SortLayout {
-    size_t hist, offsets, counters, status, alt_keys, alt_vals, total;
+    size_t hist, counters, status, alt_keys, alt_vals, total;
     uint32_t tiles;
 };
 
@@ -173,8 +164,6 @@ SortLayout sort_layout(uint64_t n) {
     L.tiles = (uint32_t)((n + kTile - 1) / kTile);
     size_t o = 0;
     L.hist = o;
-    o = align256(o + sizeof(uint32_t) * kMaxPasses * kRadix);
-    L.offsets = o;
     o = align256(o + sizeof(uint32_t) * kMaxPasses * kRadix);
     L.counters = o;
     o = align256(o + sizeof(uint32_t) * kMaxPasses);
@@ -206,42 +195,50 @@ int radix_passes(uint32_t key_bits) {
     return p < 1 ? 1 : p;
 }
 
+uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t *words) {
+    const SortLayout L = sort_layout(n);
+    *words = (L.status - L.counters) / sizeof(uint32_t) + (uint64_t)radix_passes(key_bits) * L.tiles * kRadix;
+    return (uint32_t *)((char *)scratch + L.counters);
+}
+
 cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
                              uint32_t *vals_out, uint64_t n, uint32_t key_bits, void *scratch,
                              uint64_t scratch_bytes, cudaStream_t stream, uint32_t *err,
-                             uint64_t *launches) {
+                             uint64_t *launches, const uint32_t *counted) {
     if (n == 0) return cudaSuccess;
     if (key_bits > 32 || n > (uint64_t)kValueMask) return cudaErrorInvalidValue;
     SortLayout L = sort_layout(n);
     if (scratch_bytes < L.total || scratch == nullptr) return cudaErrorInvalidValue;
     char *s = (char *)scratch;
     uint32_t *hist = (uint32_t *)(s + L.hist);
-    uint32_t *offsets = (uint32_t *)(s + L.offsets);
     uint32_t *counters = (uint32_t *)(s + L.counters);
     uint32_t *status = (uint32_t *)(s + L.status);
     uint32_t *alt_k = (uint32_t *)(s + L.alt_keys);
     uint32_t *alt_v = (uint32_t *)(s + L.alt_vals);
     const int passes = radix_passes(key_bits);
     const LookbackCtl ctl = lookback_ctl();
-    // hist, offsets, counters and the status words of every pass start at zero
-    cudaError_t e = cudaMemsetAsync(s, 0, L.alt_keys, stream);
-    if (e != cudaSuccess) return e;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 1216) blocks = 1216;
-    k_radix_histogram<<<blocks, 256, 0, stream>>>(keys_in, (uint32_t)n, passes, hist);
-    k_radix_offsets<<<passes, 256, 0, stream>>>(hist, offsets);
+    if (!counted) {
+        // hist, counters and the status words of every pass start at zero
+        cudaError_t e = cudaMemsetAsync(s, 0, L.alt_keys, stream);
+        if (e != cudaSuccess) return e;
+        int blocks = (int)((n + 255) / 256);
+        if (blocks > 1216) blocks = 1216;
+        k_radix_histogram<<<blocks, 256, 0, stream>>>(keys_in, (uint32_t)n, passes, hist);
+        counted = hist;
+        if (launches) *launches += 1;
+    }
     const uint32_t *src_k = keys_in, *src_v = vals_in;
     for (int p = 0; p < passes; ++p) {
         bool to_out = ((passes - 1 - p) % 2) == 0;
         uint32_t *dk = to_out ? keys_out : alt_k;
         uint32_t *dv = to_out ? vals_out : alt_v;
         k_onesweep<<<L.tiles, kSortThreads, 0, stream>>>(
-            src_k, src_v, dk, dv, (uint32_t)n, p * kRadixBits, offsets + p * kRadix,
+            src_k, src_v, dk, dv, (uint32_t)n, p * kRadixBits, counted + p * kRadix,
             status + (size_t)p * L.tiles * kRadix, counters + p, err, ctl);
         src_k = dk;
         src_v = dv;
     }
-    if (launches) *launches += 2 + passes;
+    if (launches) *launches += passes;
     return cudaGetLastError();
 }
 
@@ -268,7 +265,7 @@ int fgb_radix_sort_pairs_u32(const uint32_t *d_keys_in, const uint32_t *d_vals_i
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess)
         e = fgb::radix_sort_pairs(d_keys_in, d_vals_in, d_keys_out, d_vals_out, n, key_bits, d_scratch, core, st,
-                                  err, nullptr);
+                                  err, nullptr, nullptr);
     if (e != cudaSuccess) return fgb::fail_cuda(e, "radix sort");
     return FGB_OK;
 }
