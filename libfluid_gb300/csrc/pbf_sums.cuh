@@ -136,6 +136,7 @@ __device__ __forceinline__ Two operator-(const Two &x) { return Two(-x.a, -x.b);
 __device__ __forceinline__ Two fma(const Two &x, const Two &y, const Two &z) {
     return Two(__fmaf_rn(x.a, y.a, z.a), __fmaf_rn(x.b, y.b, z.b));
 }
+__device__ __forceinline__ float fma(float x, float y, float z) { return __fmaf_rn(x, y, z); }
 // r^2 of a pair of neighbours, as dist2
 __device__ __forceinline__ Two dist2(const Two &dx, const Two &dy, const Two &dz) {
     return fma(dx, dx, fma(dy, dy, dz * dz));
@@ -147,7 +148,13 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return y;
 }
 
-// Of a pair of neighbours at squared distances q2 <= h^2: r = sqrt(q2) and
+__device__ __forceinline__ Two rsqrt_approx(const Two &x) { return Two(rsqrt_approx(x.a), rsqrt_approx(x.b)); }
+__device__ __forceinline__ float ieee_root(float x) { return sqrtf(x); }
+__device__ __forceinline__ Two ieee_root(const Two &x) { return Two(sqrtf(x.a), sqrtf(x.b)); }
+__device__ __forceinline__ float ieee_div(float x, float y) { return x / y; }
+__device__ __forceinline__ Two ieee_div(const Two &x, const Two &y) { return Two(x.a / y.a, x.b / y.b); }
+
+// Of a neighbour, or a pair of them (T: float or Two), at squared distances q2 <= h^2: r = sqrt(q2) and
 // s = (h - r)^2 / r, both correctly rounded -- the bits of sqrtf and of the division.
 //
 // kFast (Phys::fast_root): one approximate reciprocal square root y serves both.  A
@@ -162,34 +169,36 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // root and quotient take about 30 with their range checks.
 // Below q2 = 1e-30 (only there does the approximation leave the normal range) r is
 // meaningless; its users drop s below eps_r2.
-template <bool kFast>
-__device__ __forceinline__ void root_and_spiky(const Phys &ph, const Two &q2, Two &r, Two &s) {
+template <bool kFast, class T>
+__device__ __forceinline__ void root_and_spiky(const Phys &ph, const T &q2, T &r, T &s) {
     if constexpr (kFast) {
-        const Two y(rsqrt_approx(q2.lo()), rsqrt_approx(q2.hi()));
-        const Two g = q2 * y;
-        r = fma(fma(-g, g, q2), y * Two(0.5f), g);
-        const Two hr = Two(ph.h) - r, a = hr * hr, nr = -r;
-        const Two inv = fma(fma(nr, y, Two(1.f)), y, y);
-        const Two w = a * inv;
+        const T y = rsqrt_approx(q2);
+        const T g = q2 * y;
+        r = fma(fma(-g, g, q2), y * T(0.5f), g);
+        const T hr = T(ph.h) - r, a = hr * hr, nr = -r;
+        const T inv = fma(fma(nr, y, T(1.f)), y, y);
+        const T w = a * inv;
         s = fma(fma(nr, w, a), inv, w);
     } else {
-        const float r0 = sqrtf(q2.lo()), r1 = sqrtf(q2.hi());
-        const float h0 = ph.h - r0, h1 = ph.h - r1;
-        r = Two(r0, r1);
-        s = Two((h0 * h0) / r0, (h1 * h1) / r1);
+        r = ieee_root(q2);
+        const T hr = T(ph.h) - r;
+        s = ieee_div(hr * hr, r);
     }
 }
 
 // a / c of a pair, correctly rounded, for a constant c with inv_c = 1 / c correctly rounded.
 // kFast: Markstein's correction again; a is zero or within 2^+-90 (else the division).
-template <bool kFast>
-__device__ __forceinline__ Two over_const(const Two &a, float c, float inv_c) {
+template <bool kFast, class T>
+__device__ __forceinline__ T over_const(const T &a, float c, float inv_c) {
     if constexpr (kFast) {
-        const Two w = a * Two(inv_c);
-        return fma(fma(Two(-c), w, a), Two(inv_c), w);
+        const T w = a * T(inv_c);
+        return fma(fma(T(-c), w, a), T(inv_c), w);
     }
-    return Two(a.lo() / c, a.hi() / c);
+    return ieee_div(a, T(c));
 }
+
+// The sums add their neighbours' terms with `add2`, two neighbours a thread, or from where
+// `terms` of one neighbour each have left them (rows.cu: a particle's four lanes).
 
 // Density and constraint gradients of one particle (oclsph_kernel.h:305-346).
 template <int PROFILE>
@@ -231,25 +240,47 @@ struct LambdaSum {
         }
     }
 
-    // two neighbours in order; r^2 above h^2 (a staged point at infinity) adds nothing
+    // a neighbour's (or two neighbours') share.  baseline: w = t^3, s = m (h - r)^2 / r, ss = s^2
+    // and the difference; ref: w its density, x, y, z the gradient's share but for 1 / rho0
+    template <class T>
+    struct Terms {
+        T q2, w, s, ss, x, y, z;
+    };
+    template <bool kFast, class T>
+    static __device__ __forceinline__ Terms<T> terms(const Phys &ph, const float4 &pa, const T &bx, const T &by,
+                                                     const T &bz, const T &mb) {
+        Terms<T> o;
+        const T dx = T(pa.x) - bx, dy = T(pa.y) - by, dz = T(pa.z) - bz;
+        T r, s;
+        if (PROFILE == kRef) {
+            o.q2 = (dx * dx + dy * dy) + dz * dz;
+            root_and_spiky<kFast>(ph, o.q2, r, s);
+            const T t = T(ph.hh) - r * r, sc = T(ph.spikyf) * s;
+            o.w = T(ph.poly6f) * (t * t * t);
+            o.x = dx * sc, o.y = dy * sc, o.z = dz * sc;
+        } else {
+            o.q2 = dist2(dx, dy, dz);
+            root_and_spiky<kFast>(ph, o.q2, r, s);
+            const T t = T(ph.hh) - o.q2;
+            o.w = t * t * t;
+            o.s = mb * s;
+            o.ss = o.s * o.s;
+            o.x = dx, o.y = dy, o.z = dz;
+        }
+        return o;
+    }
+
+    // two neighbours in order; r^2 above h^2 (a point at infinity) adds nothing
     template <bool kFast>
     __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, const Two &bx, const Two &by, const Two &bz,
                                          const Two &mb) {
-        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
-        Two r, s;
+        const Terms<Two> t = terms<kFast>(ph, pa, bx, by, bz, mb);
         if (PROFILE == kRef) {
-            const Two q2 = (dx * dx + dy * dy) + dz * dz;
-            root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - r * r, w = Two(ph.poly6f) * (t * t * t);
-            const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;
-            one<kFast>(ph, pa, q2.lo(), w.lo(), kx.lo(), ky.lo(), kz.lo());
-            one<kFast>(ph, pa, q2.hi(), w.hi(), kx.hi(), ky.hi(), kz.hi());
+            one<kFast>(ph, pa, t.q2.lo(), t.w.lo(), t.x.lo(), t.y.lo(), t.z.lo());
+            one<kFast>(ph, pa, t.q2.hi(), t.w.hi(), t.x.hi(), t.y.hi(), t.z.hi());
         } else {
-            const Two q2 = dist2(dx, dy, dz);
-            root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - q2, w = t * t * t, sc = mb * s, ss = sc * sc;
-            one(ph, q2.lo(), mb.lo(), w.lo(), sc.lo(), ss.lo(), dx.lo(), dy.lo(), dz.lo());
-            one(ph, q2.hi(), mb.hi(), w.hi(), sc.hi(), ss.hi(), dx.hi(), dy.hi(), dz.hi());
+            one(ph, t.q2.lo(), mb.lo(), t.w.lo(), t.s.lo(), t.ss.lo(), t.x.lo(), t.y.lo(), t.z.lo());
+            one(ph, t.q2.hi(), mb.hi(), t.w.hi(), t.s.hi(), t.ss.hi(), t.x.hi(), t.y.hi(), t.z.hi());
         }
     }
     __device__ __forceinline__ void one(const Phys &ph, float q2, float m, float w, float sc, float ss, float dx,
@@ -268,9 +299,7 @@ struct LambdaSum {
     __device__ __forceinline__ void one(const Phys &ph, const float4 &pa, float q2, float w, float kx, float ky,
                                         float kz) {
         if (!(q2 <= ph.hh_le)) return;
-        // on top of each other, at fast_root's h: r^2 vanishes beside h^2 (and the fast root
-        // of r^2 below 1e-30 is meaningless)
-        if (kFast && q2 < ph.eps_r2) w = ph.poly6f * (ph.hh * ph.hh * ph.hh);
+        if (kFast && q2 < ph.eps_r2) w = on_top(ph);
         rho = __fmaf_rn(pa.w, w, rho);
         if (q2 >= ph.eps_r2) {
             gx = __fmaf_rn(kx, ph.inv_rho0, gx);
@@ -278,6 +307,10 @@ struct LambdaSum {
             gz = __fmaf_rn(kz, ph.inv_rho0, gz);
         }
     }
+
+    // the density of two particles on top of each other, at fast_root's h: r^2 vanishes beside
+    // h^2 (and the fast root of r^2 below 1e-30 is meaningless)
+    static __device__ __forceinline__ float on_top(const Phys &ph) { return ph.poly6f * (ph.hh * ph.hh * ph.hh); }
 
     // lambda, and the density in *dens
     __device__ __forceinline__ float finish(const Phys &ph, float *dens) const {
@@ -341,53 +374,73 @@ struct DeltaSum {
         }
     }
 
+    // a neighbour's (or two neighbours') share: f times (x, y, z)
+    template <class T>
+    struct Terms {
+        T q2, f, x, y, z;
+    };
+    template <bool kFast, class T>
+    static __device__ __forceinline__ Terms<T> terms(const Phys &ph, const float4 &pa, float la, const T &bx,
+                                                     const T &by, const T &bz, const T &lb, const T &mb) {
+        Terms<T> o;
+        const T dx = T(pa.x) - bx, dy = T(pa.y) - by, dz = T(pa.z) - bz;
+        T r, s;
+        if (PROFILE == kRef) {
+            o.q2 = (dx * dx + dy * dy) + dz * dz;
+            root_and_spiky<kFast>(ph, o.q2, r, s);
+            const T t = T(ph.hh) - r * r, w = T(ph.poly6f) * (t * t * t);
+            const T c = T(-ph.corr_k) * corr<kFast>(ph, over_const<kFast>(w, ph.corr_ref, ph.inv_corr_ref));
+            const T sum = (T(la) + lb) + c;
+            o.f = over_const<kFast>(sum, ph.rho0, ph.inv_rho0);
+            // outside over_const's range (a sum that cancelled, or one that ran away)
+            if (kFast && out_of_range(ph, o.q2, sum)) o.f = ieee_div(sum, T(ph.rho0));
+            const T sc = T(ph.spikyf) * s;
+            o.x = dx * sc, o.y = dy * sc, o.z = dz * sc;
+        } else {
+            o.q2 = dist2(dx, dy, dz);
+            root_and_spiky<kFast>(ph, o.q2, r, s);
+            const T t = T(ph.hh) - o.q2;
+            const T c = T(-ph.corr_k) * corr<kFast>(ph, (t * t * t) * T(ph.inv_corr_wdq));
+            o.f = mb * s * ((T(la) + lb) + c);
+            o.x = dx, o.y = dy, o.z = dz;
+        }
+        return o;
+    }
+    static __device__ __forceinline__ bool in_range(const Phys &ph, float q2) {
+        return q2 <= (PROFILE == kRef ? ph.hh_le : ph.hh) && q2 >= ph.eps_r2;
+    }
+    static __device__ __forceinline__ bool out_of_range(const Phys &ph, float q2, float sum) {
+        return q2 <= ph.hh_le && !(fabsf(sum) > 1e-27f && fabsf(sum) < 1e27f);
+    }
+    static __device__ __forceinline__ bool out_of_range(const Phys &ph, const Two &q2, const Two &sum) {
+        return out_of_range(ph, q2.lo(), sum.lo()) || out_of_range(ph, q2.hi(), sum.hi());
+    }
+
     // two neighbours in order, their lambdas in lb
     template <bool kFast>
     __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, float la, const Two &bx, const Two &by,
                                          const Two &bz, const Two &lb, const Two &mb) {
-        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
-        Two r, s, k;
-        if (PROFILE == kRef) {
-            const Two q2 = (dx * dx + dy * dy) + dz * dz;
-            root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - r * r, w = Two(ph.poly6f) * (t * t * t);
-            const Two c =
-                Two(-ph.corr_k) * corr<kFast>(ph, over_const<kFast>(w, ph.corr_ref, ph.inv_corr_ref));
-            const Two sum = (Two(la) + lb) + c;
-            Two f = over_const<kFast>(sum, ph.rho0, ph.inv_rho0);
-            if (kFast) {
-                // outside over_const's range (a sum that cancelled, or one that ran away)
-                const float s0 = fabsf(sum.lo()), s1 = fabsf(sum.hi());
-                if ((q2.lo() <= ph.hh_le && !(s0 > 1e-27f && s0 < 1e27f)) ||
-                    (q2.hi() <= ph.hh_le && !(s1 > 1e-27f && s1 < 1e27f)))
-                    f = Two(sum.lo() / ph.rho0, sum.hi() / ph.rho0);
-            }
-            const Two sc = Two(ph.spikyf) * s, kx = dx * sc, ky = dy * sc, kz = dz * sc;
-            if (q2.lo() <= ph.hh_le && q2.lo() >= ph.eps_r2) move_by(f.lo(), kx.lo(), ky.lo(), kz.lo());
-            if (q2.hi() <= ph.hh_le && q2.hi() >= ph.eps_r2) move_by(f.hi(), kx.hi(), ky.hi(), kz.hi());
-        } else {
-            const Two q2 = dist2(dx, dy, dz);
-            root_and_spiky<kFast>(ph, q2, r, s);
-            const Two t = Two(ph.hh) - q2;
-            const Two c = Two(-ph.corr_k) * corr<kFast>(ph, (t * t * t) * Two(ph.inv_corr_wdq));
-            const Two sc = mb * s * ((Two(la) + lb) + c);
-            if (q2.lo() <= ph.hh && q2.lo() >= ph.eps_r2) move_by(sc.lo(), dx.lo(), dy.lo(), dz.lo());
-            if (q2.hi() <= ph.hh && q2.hi() >= ph.eps_r2) move_by(sc.hi(), dx.hi(), dy.hi(), dz.hi());
-        }
+        const Terms<Two> t = terms<kFast>(ph, pa, la, bx, by, bz, lb, mb);
+        if (in_range(ph, t.q2.lo())) move_by(t.f.lo(), t.x.lo(), t.y.lo(), t.z.lo());
+        if (in_range(ph, t.q2.hi())) move_by(t.f.hi(), t.x.hi(), t.y.hi(), t.z.hi());
     }
     __device__ __forceinline__ void move_by(float f, float kx, float ky, float kz) {
         px = __fmaf_rn(kx, f, px);
         py = __fmaf_rn(ky, f, py);
         pz = __fmaf_rn(kz, f, pz);
     }
-    // corr_pow of a pair (fast_root asks for the fourth power)
-    template <bool kFast>
-    static __device__ __forceinline__ Two corr(const Phys &ph, const Two &ratio) {
+    // corr_pow (fast_root asks for the fourth power)
+    template <bool kFast, class T>
+    static __device__ __forceinline__ T corr(const Phys &ph, const T &ratio) {
         if constexpr (kFast) {
-            const Two r2 = ratio * ratio;
+            const T r2 = ratio * ratio;
             return r2 * r2;
         }
-        return Two(corr_pow(ratio.lo(), ph.corr_n), corr_pow(ratio.hi(), ph.corr_n));
+        return power(ratio, ph.corr_n);
+    }
+    static __device__ __forceinline__ float power(float ratio, float n) { return corr_pow(ratio, n); }
+    static __device__ __forceinline__ Two power(const Two &ratio, float n) {
+        return Two(corr_pow(ratio.lo(), n), corr_pow(ratio.hi(), n));
     }
 
     // The corrected p* after the colliders and the bounds (solver units) in q[3], and
@@ -480,21 +533,37 @@ struct VorticitySum {
         }
     }
 
-    // two neighbours in order, at velocities (ux, uy, uz)
+    // a neighbour's (or two neighbours') share, at velocities (ux, uy, uz): mw times (vx, vy, vz)
+    // and s times (cx, cy, cz)
+    template <class T>
+    struct Terms {
+        T q2, mw, vx, vy, vz, s, cx, cy, cz;
+    };
+    template <bool kFast, class T>
+    static __device__ __forceinline__ Terms<T> terms(const Phys &ph, const float4 &pa, const float4 &va, const T &bx,
+                                                     const T &by, const T &bz, const T &mb, const T &ux, const T &uy,
+                                                     const T &uz) {
+        Terms<T> o;
+        const T dx = T(pa.x) - bx, dy = T(pa.y) - by, dz = T(pa.z) - bz;
+        o.q2 = dist2(dx, dy, dz);
+        T r, s;
+        root_and_spiky<kFast>(ph, o.q2, r, s);
+        o.vx = ux - T(va.x), o.vy = uy - T(va.y), o.vz = uz - T(va.z);
+        const T t = T(ph.hh) - o.q2;
+        o.mw = mb * (t * t * t);
+        o.s = mb * s;
+        o.cx = o.vy * dz - o.vz * dy, o.cy = o.vz * dx - o.vx * dz, o.cz = o.vx * dy - o.vy * dx;
+        return o;
+    }
+
+    // two neighbours in order
     template <bool kFast>
     __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, const float4 &va, const Two &bx,
                                          const Two &by, const Two &bz, const Two &mb, const Two &ux, const Two &uy,
                                          const Two &uz) {
-        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
-        const Two q2 = dist2(dx, dy, dz);
-        Two r, s;
-        root_and_spiky<kFast>(ph, q2, r, s);
-        const Two vx = ux - Two(va.x), vy = uy - Two(va.y), vz = uz - Two(va.z);
-        const Two t = Two(ph.hh) - q2, mw = mb * (t * t * t), sc = mb * s;
-        const Two cx = vy * dz - vz * dy, cy = vz * dx - vx * dz,
-                  cz = vx * dy - vy * dx;
-        one(ph, q2.lo(), mw.lo(), vx.lo(), vy.lo(), vz.lo(), sc.lo(), cx.lo(), cy.lo(), cz.lo());
-        one(ph, q2.hi(), mw.hi(), vx.hi(), vy.hi(), vz.hi(), sc.hi(), cx.hi(), cy.hi(), cz.hi());
+        const Terms<Two> t = terms<kFast>(ph, pa, va, bx, by, bz, mb, ux, uy, uz);
+        one(ph, t.q2.lo(), t.mw.lo(), t.vx.lo(), t.vy.lo(), t.vz.lo(), t.s.lo(), t.cx.lo(), t.cy.lo(), t.cz.lo());
+        one(ph, t.q2.hi(), t.mw.hi(), t.vx.hi(), t.vy.hi(), t.vz.hi(), t.s.hi(), t.cx.hi(), t.cy.hi(), t.cz.hi());
     }
     __device__ __forceinline__ void one(const Phys &ph, float q2, float mw, float vx, float vy, float vz, float sc,
                                         float cx, float cy, float cz) {
@@ -547,17 +616,31 @@ struct ApplySum {
         e[2] = __fmaf_rn(sc, d[2], e[2]);
     }
 
-    // two neighbours in order, their |omega| in ob
+    // a neighbour's (or two neighbours') share, |omega| in ob: f times (x, y, z)
+    template <class T>
+    struct Terms {
+        T q2, f, x, y, z;
+    };
+    template <bool kFast, class T>
+    static __device__ __forceinline__ Terms<T> terms(const Phys &ph, const float4 &pa, float oa, const T &bx,
+                                                     const T &by, const T &bz, const T &ob, const T &mb) {
+        Terms<T> o;
+        o.x = T(pa.x) - bx, o.y = T(pa.y) - by, o.z = T(pa.z) - bz;
+        o.q2 = dist2(o.x, o.y, o.z);
+        T r, s;
+        root_and_spiky<kFast>(ph, o.q2, r, s);
+        o.f = mb * s * (ob - T(oa));
+        return o;
+    }
+    static __device__ __forceinline__ bool in_range(const Phys &ph, float q2) { return q2 <= ph.hh && q2 >= ph.eps_r2; }
+
+    // two neighbours in order
     template <bool kFast>
     __device__ __forceinline__ void add2(const Phys &ph, const float4 &pa, float oa, const Two &bx, const Two &by,
                                          const Two &bz, const Two &ob, const Two &mb) {
-        const Two dx = Two(pa.x) - bx, dy = Two(pa.y) - by, dz = Two(pa.z) - bz;
-        const Two q2 = dist2(dx, dy, dz);
-        Two r, s;
-        root_and_spiky<kFast>(ph, q2, r, s);
-        const Two sc = mb * s * (ob - Two(oa));
-        if (q2.lo() <= ph.hh && q2.lo() >= ph.eps_r2) one(sc.lo(), dx.lo(), dy.lo(), dz.lo());
-        if (q2.hi() <= ph.hh && q2.hi() >= ph.eps_r2) one(sc.hi(), dx.hi(), dy.hi(), dz.hi());
+        const Terms<Two> t = terms<kFast>(ph, pa, oa, bx, by, bz, ob, mb);
+        if (in_range(ph, t.q2.lo())) one(t.f.lo(), t.x.lo(), t.y.lo(), t.z.lo());
+        if (in_range(ph, t.q2.hi())) one(t.f.hi(), t.x.hi(), t.y.hi(), t.z.hi());
     }
     __device__ __forceinline__ void one(float sc, float dx, float dy, float dz) {
         e[0] = __fmaf_rn(sc, dx, e[0]);

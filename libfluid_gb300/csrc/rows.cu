@@ -78,6 +78,7 @@ __device__ __forceinline__ uint4 *row_of(const RowArgs &A, uint32_t a) {
 constexpr uint32_t kCellBlock = 128, kCellWarps = kCellBlock / 32;
 constexpr uint32_t kFetchFrom = 400000;   // particles from which the passes ask for their rows ahead
 constexpr uint32_t kListFrom = 100000;    // particles from which stale groups are listed first
+constexpr uint32_t kQuadsTo = 24000, kQuadsToRef = 45000;  // particles below which one has four lanes
 constexpr float kRowSkin = 0.1f;          // the skin of rows that last, in h
 constexpr uint32_t kHeldAll = 256;        // candidates a warp holds at a time
 constexpr uint32_t kList = 4;             // particles whose hits are collected before they are written
@@ -186,7 +187,7 @@ enum Search {
 // Where most rows last a search comes down to this question, and a warp that asks it of one
 // group at a time mostly waits.  A calm search of 1 M particles takes 34 us with this list
 // and 60 without (steps of 1.43 and 1.54 ms; at step 100, where no row lasts, 2.12 and
-// 2.13); 262 k 461 and 484 us a step, 110 k 271 and 276, 50 k 228 and 219, 14 k 181 and 162:
+// 2.13); 262 k 461 and 484 us a step, 110 k 271 and 276, 64 k 228 and 219, 14 k 181 and 162:
 // hence kListFrom.  With the ref profile's constants hardly any row lasts (262 k 1480 and
 // 1466): its searches ask as they go.  L1 lookups bound it, 54 scattered ones a group.
 __global__ void __launch_bounds__(128, 8) k_stale_groups(RowArgs A, uint32_t n_scenes, int count_use) {
@@ -542,19 +543,46 @@ __global__ void __launch_bounds__(128, 8)
 }
 
 // Keep the cell's largest movement since the grid was built: lanes of one cell (their
-// particles are consecutive) settle theirs first.  All lanes take part.
+// particles are consecutive, every kStride lanes) settle theirs first.  All lanes take part.
+template <int kStride>
 __device__ __forceinline__ void keep_moved(const RowArgs &A, bool have, uint32_t cell_start, float moved) {
     uint32_t m = have ? __float_as_uint(moved) : 0u;
     if (have && !(moved == moved)) m = 0x7f800000u;  // not a number: the bound has to fail
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t where = have ? cell_start : 0xffffffffu;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
+    for (int d = kStride; d < 32; d <<= 1) {
         const uint32_t o = __shfl_down_sync(0xffffffffu, m, d), w = __shfl_down_sync(0xffffffffu, where, d);
         if (lane + d < 32 && w == where) m = max(m, o);
     }
-    const uint32_t left = __shfl_up_sync(0xffffffffu, where, 1);
-    if (have && (lane == 0 || left != where) && m) atomicMax(&A.moved[where], m);
+    const uint32_t left = __shfl_up_sync(0xffffffffu, where, kStride);
+    if (have && (lane < kStride || left != where) && m) atomicMax(&A.moved[where], m);
+}
+
+// The end of a particle's delta pass: its new position, after the step's last correction also
+// its velocity; how far it is from its grid position, and where its cell begins.
+template <int PROFILE>
+__device__ __forceinline__ float finish_delta(const RowArgs &A, const SceneDev &S, const DeltaSum<PROFILE> &sum,
+                                              uint32_t a, uint32_t key, const float4 &pa, float4 *__restrict__ ps_out,
+                                              float4 *__restrict__ x, float4 *__restrict__ v, int last,
+                                              float4 *__restrict__ pv, const HostParticlesOut *__restrict__ hout,
+                                              uint32_t &cell_start) {
+    const Phys &ph = A.ph;
+    float4 va;
+    float q[3], vel[3];
+    sum.move(ph, S, A.tris, pa, a, v, q, va, vel);
+    ps_out[a] = make_float4(q[0], q[1], q[2], pa.w);
+    if (last) {
+        const float4 now = finalise<PROFILE>(ph, S, a, q, va, vel, x, v, hout);
+        if (PROFILE != kRef) {
+            pv[2 * (size_t)a] = make_float4(q[0], q[1], q[2], pa.w);
+            pv[2 * (size_t)a + 1] = now;
+        }
+    }
+    const float4 g = __ldg(&A.ps_grid[a]);
+    const float ex = q[0] - g.x, ey = q[1] - g.y, ez = q[2] - g.z;
+    cell_start = __ldg(&A.cells[S.table_base + morton_of(key, A.mbits)]).x;
+    return sqrtf(ex * ex + ey * ey + ez * ez);
 }
 
 template <int PROFILE, bool kFast>
@@ -594,23 +622,9 @@ __global__ void __launch_bounds__(128, 8)
                 const float4 p = __ldg(&plam[b]);
                 sum.add(ph, pa, la, p.x, p.y, p.z, [&] { return p.w; }, __ldg(&ps_in[b]).w);
             });
-        float4 va;
-        float q[3], vel[3];
-        sum.move(ph, S, A.tris, pa, a, v, q, va, vel);
-        ps_out[a] = make_float4(q[0], q[1], q[2], pa.w);
-        if (last) {
-            const float4 now = finalise<PROFILE>(ph, S, a, q, va, vel, x, v, hout);
-            if (PROFILE != kRef) {
-                pv[2 * (size_t)a] = make_float4(q[0], q[1], q[2], pa.w);
-                pv[2 * (size_t)a + 1] = now;
-            }
-        }
-        const float4 g = __ldg(&A.ps_grid[a]);
-        const float ex = q[0] - g.x, ey = q[1] - g.y, ez = q[2] - g.z;
-        moved = sqrtf(ex * ex + ey * ey + ez * ez);
-        cell_start = __ldg(&A.cells[S.table_base + morton_of(key, A.mbits)]).x;
+        moved = finish_delta<PROFILE>(A, S, sum, a, key, pa, ps_out, x, v, last, pv, hout, cell_start);
     }
-    if (PROFILE != kRef || !last) keep_moved(A, fluid, cell_start, moved);  // a search follows
+    if (PROFILE != kRef || !last) keep_moved<1>(A, fluid, cell_start, moved);  // a search follows
 }
 
 // Pass A of the velocity terms: fluid neighbours only, which rows do not tell apart.  The
@@ -710,6 +724,282 @@ __global__ void __launch_bounds__(128, 8)
     sum.finish(ph, S, a, pa, oa, vx, v, x, hout);
 }
 
+// ---------------------------------------------------------------- four lanes a particle
+//
+// The same passes for small scenes.  A thread that goes through a row
+// alone waits for one operation after another where a scheduler holds a warp or two, and a
+// warp of 32 particles for its longest row; with four lanes a particle there are four times
+// the warps, each lane forms the terms of every fourth entry, and they meet in shared memory,
+// where lane 0 to 2 adds up one component, in the row's order, and lane 3 what remains.
+// A step with a thread a particle / four lanes: baseline 4 k 133 / 115 us, 14 k 150 / 135,
+// 33 k 179 / 183, 64 k 211 / 260; ref profile 14 k 430 / 342, 33 k 605 / 565, 64 k 578 / 616:
+// a warp of lanes adds 68 instructions for four entries of eight particles where 160 did for
+// those of 32, so it only pays where warps are few (kQuadsTo, kQuadsToRef).
+
+constexpr uint32_t kQuadPitch = 40;  // floats: eight lanes' reads of four values touch all banks once
+
+template <int kValues>
+struct QuadBuffer {
+    float v[2][kValues][kQuadPitch];  // by turns: one barrier an iteration
+};
+
+// A particle's row by its four lanes: fetch(b) gives an entry's data, terms(b, data, v, in, near)
+// its terms and whether it is within range and not on top of the particle, add(v, at, in, near)
+// takes four entries' terms: those of value k at v[k][at ..], bit e of in and near for the e-th.
+// All lanes of a warp take part; count is 0 for those without a row.
+template <int kValues, class Fetch, class Terms, class Add>
+__device__ __forceinline__ void for_quads(const RowArgs &A, QuadBuffer<kValues> &buffer, uint32_t a, uint32_t count,
+                                          Fetch &&fetch, Terms &&terms, Add &&add) {
+    const uint32_t lane = threadIdx.x & 31u, at = lane & 28u, quads = (count + 3) >> 2;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, quads);
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(row_of(A, a)) + (lane & 3u);
+    auto entry = [&](uint32_t i) { return i < quads ? __ldg(row + i * 128) : A.none; };
+    uint32_t b = entry(0), next = entry(1);
+    auto data = fetch(b);
+    for (uint32_t i = 0; i < most; ++i) {
+        const uint32_t this_b = b;
+        const auto this_data = data;
+        b = next;
+        data = fetch(b);
+        next = entry(i + 2);
+        float v[kValues];
+        bool in, near;
+        terms(this_b, this_data, v, in, near);
+        float(&to)[kValues][kQuadPitch] = buffer.v[i & 1u];
+#pragma unroll
+        for (int k = 0; k < kValues; ++k) to[k][lane] = v[k];
+        const unsigned ins = __ballot_sync(0xffffffffu, in) >> at, nears = __ballot_sync(0xffffffffu, near) >> at;
+        __syncwarp();
+        add(to, at, ins, nears);
+    }
+}
+
+// acc += f x for the entries whose bit is set, in order
+__device__ __forceinline__ void add_four(float &acc, const float4 &f, const float4 &x, unsigned bits) {
+    if (bits & 1u) acc = __fmaf_rn(f.x, x.x, acc);
+    if (bits & 2u) acc = __fmaf_rn(f.y, x.y, acc);
+    if (bits & 4u) acc = __fmaf_rn(f.z, x.z, acc);
+    if (bits & 8u) acc = __fmaf_rn(f.w, x.w, acc);
+}
+__device__ __forceinline__ float4 four(const float (&v)[kQuadPitch], uint32_t at) {
+    return *reinterpret_cast<const float4 *>(&v[at]);
+}
+// the value of the quad's lane k
+__device__ __forceinline__ float of_lane(float v, int k) { return __shfl_sync(0xffffffffu, v, k, 4); }
+
+template <int PROFILE, bool kFast>
+__global__ void __launch_bounds__(128)
+    k_quad_lambda(RowArgs A, const float4 *__restrict__ ps, float *__restrict__ lambda, float *__restrict__ density,
+                  float4 *__restrict__ plam) {
+    constexpr bool kR = PROFILE == kRef;
+    __shared__ alignas(16) QuadBuffer<kR ? 4 : 8> s_buffer[4];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, part = threadIdx.x & 3u;
+    const bool own = (t >> 2) < A.n;
+    const uint32_t a = own ? t >> 2 : A.n - 1;
+    const Phys &ph = A.ph;
+    const float4 pa = ps[a];
+    const bool fluid = own && A.type[a] != FGB_TYPE_OBSTACLE;
+    const uint32_t count = fluid ? A.hcount[a] : 0u;
+    float first = 0.f, second = 0.f;  // the lane's sums
+    const float hh = kR ? ph.hh_le : ph.hh;
+    for_quads(
+        A, s_buffer[threadIdx.x >> 5], a, count == kListOverflow ? 0u : count, [&](uint32_t b) { return __ldg(&ps[b]); },
+        [&](uint32_t, const float4 &p, float *v, bool &in, bool &near) {
+            const auto o = LambdaSum<PROFILE>::template terms<kFast>(ph, pa, p.x, p.y, p.z, p.w);
+            in = o.q2 <= hh;
+            near = o.q2 >= ph.eps_r2;
+            v[0] = o.x, v[1] = o.y, v[2] = o.z, v[3] = o.w;
+            if (kR) {
+                if (kFast && !near) v[3] = LambdaSum<PROFILE>::on_top(ph);
+            } else {
+                v[4] = o.s, v[5] = p.w, v[6] = o.ss, v[7] = o.q2;
+            }
+        },
+        [&](const auto &v, uint32_t at, unsigned in, unsigned near) {
+            near &= in;
+            const float4 x = four(v[part], at);
+            if constexpr (kR) {
+                const float f = part < 3 ? ph.inv_rho0 : pa.w;
+                add_four(first, make_float4(f, f, f, f), x, part < 3 ? near : in);
+            } else {
+                add_four(first, four(v[part < 3 ? 4 : 5], at), x, part < 3 ? near : in);
+                add_four(second, four(v[6], at), four(v[7], at), near);
+            }
+        });
+    LambdaSum<PROFILE> sum;
+    sum.gx = of_lane(first, 0), sum.gy = of_lane(first, 1), sum.gz = of_lane(first, 2);
+    sum.rho = of_lane(first, 3), sum.g2 = second;  // second is the same in all four
+    if (!own || part) return;
+    float lam = 0.f, dens = 0.f;
+    if (fluid) {
+        if (count == kListOverflow)
+            walk_cells(A, A.scenes[scene_of(A.keys[a], A.mbits)], A.keys[a], [&](uint32_t b) {
+                const float4 p = __ldg(&ps[b]);
+                sum.add(ph, pa, p.x, p.y, p.z, p.w);
+            });
+        lam = sum.finish(ph, &dens);
+    }
+    lambda[a] = lam;
+    density[a] = dens;
+    plam[a] = make_float4(pa.x, pa.y, pa.z, lam);
+    A.moved[a] = 0;  // before the delta pass that follows
+}
+
+template <int PROFILE, bool kFast>
+__global__ void __launch_bounds__(128)
+    k_quad_delta(RowArgs A, const float4 *__restrict__ ps_in, const float4 *__restrict__ plam,
+                 float4 *__restrict__ ps_out, float4 *__restrict__ x, float4 *__restrict__ v, int last,
+                 float4 *__restrict__ pv, const HostParticlesOut *__restrict__ hout) {
+    __shared__ alignas(16) QuadBuffer<4> s_buffer[4];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, part = threadIdx.x & 3u;
+    const bool own = (t >> 2) < A.n;
+    const uint32_t a = own ? t >> 2 : A.n - 1;
+    const Phys &ph = A.ph;
+    const bool equal = PROFILE == kRef || A.mass_range[0] == ~A.mass_range[1];
+    const float mass = __uint_as_float(A.mass_range[0]);
+    const float4 pa = ps_in[a];
+    const float la = __ldg(&plam[a]).w;
+    const bool fluid = own && A.type[a] != FGB_TYPE_OBSTACLE;
+    const uint32_t count = fluid ? A.hcount[a] : 0u;
+    float first = 0.f;
+    for_quads(
+        A, s_buffer[threadIdx.x >> 5], a, count == kListOverflow ? 0u : count,
+        [&](uint32_t b) { return __ldg(&plam[b]); },
+        [&](uint32_t b, const float4 &p, float *o, bool &in, bool &near) {
+            const float m = equal ? mass : __ldg(&ps_in[b]).w;
+            const auto terms = DeltaSum<PROFILE>::template terms<kFast>(ph, pa, la, p.x, p.y, p.z, p.w, m);
+            in = near = DeltaSum<PROFILE>::in_range(ph, terms.q2);
+            o[0] = terms.x, o[1] = terms.y, o[2] = terms.z, o[3] = terms.f;
+        },
+        [&](const auto &o, uint32_t at, unsigned in, unsigned) {
+            add_four(first, four(o[part < 3 ? part : 2], at), four(o[3], at), in);
+        });
+    DeltaSum<PROFILE> sum;
+    sum.px = of_lane(first, 0), sum.py = of_lane(first, 1), sum.pz = of_lane(first, 2);
+    const bool leads = own && part == 0;
+    uint32_t cell_start = 0;
+    float moved = 0.f;
+    if (leads && !fluid) {
+        ps_out[a] = ps_in[a];
+        if (PROFILE != kRef && last) pv[2 * (size_t)a] = ps_in[a], pv[2 * (size_t)a + 1] = v[a];
+        if (PROFILE == kRef && last) store_host_motion(hout, a, x[a], v[a]);
+    }
+    if (leads && fluid) {
+        const uint32_t key = A.keys[a];
+        const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
+        if (count == kListOverflow)
+            walk_cells(A, S, key, [&](uint32_t b) {
+                const float4 p = __ldg(&plam[b]);
+                sum.add(ph, pa, la, p.x, p.y, p.z, [&] { return p.w; }, __ldg(&ps_in[b]).w);
+            });
+        moved = finish_delta<PROFILE>(A, S, sum, a, key, pa, ps_out, x, v, last, pv, hout, cell_start);
+    }
+    if (PROFILE != kRef || !last) keep_moved<4>(A, leads && fluid, cell_start, moved);  // a search follows
+}
+
+template <bool kFast>
+__global__ void __launch_bounds__(128)
+    k_quad_vorticity(RowArgs A, const float4 *__restrict__ pv, float4 *__restrict__ omega, float4 *__restrict__ pom,
+                     float4 *__restrict__ vx) {
+    __shared__ alignas(16) QuadBuffer<8> s_buffer[4];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, part = threadIdx.x & 3u;
+    const bool own = (t >> 2) < A.n;
+    const uint32_t a = own ? t >> 2 : A.n - 1;
+    const Phys &ph = A.ph;
+    float4 pa, va;
+    load_two(pv + 2 * (size_t)a, pa, va);
+    const bool fluid = own && A.type[a] != FGB_TYPE_OBSTACLE;
+    const uint32_t key = A.keys[a], count = fluid ? A.hcount[a] : 0u;
+    const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
+    const bool obstacles = S.obstacles != 0;
+    float first = 0.f, second = 0.f;
+    struct Both {
+        float4 p, u;
+    };
+    for_quads(
+        A, s_buffer[threadIdx.x >> 5], a, count == kListOverflow ? 0u : count,
+        [&](uint32_t b) {
+            Both o;
+            load_two(pv + 2 * (size_t)b, o.p, o.u);
+            return o;
+        },
+        [&](uint32_t b, const Both &n, float *o, bool &in, bool &near) {
+            const auto terms = VorticitySum::terms<kFast>(ph, pa, va, n.p.x, n.p.y, n.p.z, n.p.w, n.u.x, n.u.y, n.u.z);
+            in = terms.q2 <= ph.hh && !(obstacles && __ldg(&A.type[b]) == FGB_TYPE_OBSTACLE);
+            near = terms.q2 >= ph.eps_r2;
+            o[0] = terms.vx, o[1] = terms.vy, o[2] = terms.vz, o[3] = terms.mw;
+            o[4] = terms.cx, o[5] = terms.cy, o[6] = terms.cz, o[7] = terms.s;
+        },
+        [&](const auto &o, uint32_t at, unsigned in, unsigned near) {
+            const uint32_t k = part < 3 ? part : 2;
+            add_four(first, four(o[3], at), four(o[k], at), in);
+            add_four(second, four(o[7], at), four(o[4 + k], at), in & near);
+        });
+    VorticitySum sum;
+    for (int k = 0; k < 3; ++k) sum.xs[k] = of_lane(first, k), sum.o[k] = of_lane(second, k);
+    if (!own || part) return;
+    if (!fluid) {
+        omega[a] = make_float4(0.f, 0.f, 0.f, 0.f);
+        vx[a] = va;
+        pom[a] = make_float4(pa.x, pa.y, pa.z, 0.f);
+        return;
+    }
+    if (count == kListOverflow)
+        walk_cells(A, S, key, [&](uint32_t b) {
+            if (obstacles && __ldg(&A.type[b]) == FGB_TYPE_OBSTACLE) return;
+            const float4 p = __ldg(&pv[2 * (size_t)b]);
+            sum.add(ph, pa, va, p.x, p.y, p.z, p.w, [&] { return __ldg(&pv[2 * (size_t)b + 1]); });
+        });
+    sum.finish(ph, a, pa, va, omega, pom, vx);
+}
+
+template <bool kFast>
+__global__ void __launch_bounds__(128)
+    k_quad_apply(RowArgs A, const float4 *__restrict__ ps, const float4 *__restrict__ omega,
+                 const float4 *__restrict__ pom, const float4 *__restrict__ vx, float4 *__restrict__ v,
+                 float4 *__restrict__ x, const HostParticlesOut *__restrict__ hout) {
+    __shared__ alignas(16) QuadBuffer<4> s_buffer[4];
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, part = threadIdx.x & 3u;
+    const bool own = (t >> 2) < A.n;
+    const uint32_t a = own ? t >> 2 : A.n - 1;
+    const Phys &ph = A.ph;
+    const bool equal = A.mass_range[0] == ~A.mass_range[1];
+    const float mass = __uint_as_float(A.mass_range[0]);
+    const uint32_t key = A.keys[a];
+    const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
+    const bool obstacles = S.obstacles != 0;
+    const float4 pa = ps[a], oa = omega[a];
+    const bool fluid = own && A.type[a] != FGB_TYPE_OBSTACLE;
+    const uint32_t count = fluid ? A.hcount[a] : 0u;
+    float first = 0.f;
+    for_quads(
+        A, s_buffer[threadIdx.x >> 5], a, count == kListOverflow ? 0u : count,
+        [&](uint32_t b) { return __ldg(&pom[b]); },
+        [&](uint32_t b, const float4 &p, float *o, bool &in, bool &near) {
+            const float m = equal ? mass : __ldg(&ps[b]).w;
+            const auto terms = ApplySum::terms<kFast>(ph, pa, oa.w, p.x, p.y, p.z, p.w, m);
+            in = near = ApplySum::in_range(ph, terms.q2) && !(obstacles && __ldg(&A.type[b]) == FGB_TYPE_OBSTACLE);
+            o[0] = terms.x, o[1] = terms.y, o[2] = terms.z, o[3] = terms.f;
+        },
+        [&](const auto &o, uint32_t at, unsigned in, unsigned) {
+            add_four(first, four(o[3], at), four(o[part < 3 ? part : 2], at), in);
+        });
+    ApplySum sum;
+    for (int k = 0; k < 3; ++k) sum.e[k] = of_lane(first, k);
+    if (!own || part) return;
+    if (!fluid) {
+        store_host_motion(hout, a, x[a], v[a]);
+        return;
+    }
+    if (count == kListOverflow)
+        walk_cells(A, S, key, [&](uint32_t b) {
+            if (obstacles && __ldg(&A.type[b]) == FGB_TYPE_OBSTACLE) return;
+            const float4 p = __ldg(&pom[b]);
+            sum.add(ph, pa, oa.w, p.x, p.y, p.z, [&] { return p.w; }, __ldg(&ps[b]).w);
+        });
+    sum.finish(ph, S, a, pa, oa, vx, v, x, hout);
+}
+
 RowArgs row_args(const StepView &s) {
     RowArgs A;
     A.scenes = s.scenes;
@@ -784,19 +1074,30 @@ cudaError_t rows_of(const StepView &s, const float4 *ps, uint32_t pass, cudaStre
 }
 
 inline unsigned row_grid(const StepView &s) { return (s.n + 127) / 128; }
+inline unsigned quad_grid(const StepView &s) { return (unsigned)(((uint64_t)s.n + 31) / 32); }
+
+// Whether the passes give a particle four lanes.
+inline bool by_quads(const StepView &s) { return s.n < (s.ph.profile == FGB_PROFILE_REF ? kQuadsToRef : kQuadsTo); }
 
 template <int PROFILE, bool kFast>
 cudaError_t lambda_as(const StepView &s, const float4 *ps, int iteration, cudaStream_t st) {
     cudaError_t e = rows_of(s, ps, (uint32_t)iteration, st);
     if (e != cudaSuccess) return e;
-    k_row_lambda<PROFILE, kFast><<<row_grid(s), 128, 0, st>>>(row_args(s), ps, s.lambda, s.density, s.plam);
+    if (by_quads(s))
+        k_quad_lambda<PROFILE, kFast><<<quad_grid(s), 128, 0, st>>>(row_args(s), ps, s.lambda, s.density, s.plam);
+    else
+        k_row_lambda<PROFILE, kFast><<<row_grid(s), 128, 0, st>>>(row_args(s), ps, s.lambda, s.density, s.plam);
     return cudaGetLastError();
 }
 
 template <int PROFILE, bool kFast>
 cudaError_t delta_as(const StepView &s, const float4 *ps_in, float4 *ps_out, bool last, cudaStream_t st) {
-    k_row_delta<PROFILE, kFast><<<row_grid(s), 128, 0, st>>>(row_args(s), ps_in, s.plam, ps_out, s.x1, s.v1,
-                                                                  last ? 1 : 0, s.pv, s.hout);
+    if (by_quads(s))
+        k_quad_delta<PROFILE, kFast><<<quad_grid(s), 128, 0, st>>>(row_args(s), ps_in, s.plam, ps_out, s.x1, s.v1,
+                                                                   last ? 1 : 0, s.pv, s.hout);
+    else
+        k_row_delta<PROFILE, kFast><<<row_grid(s), 128, 0, st>>>(row_args(s), ps_in, s.plam, ps_out, s.x1, s.v1,
+                                                                 last ? 1 : 0, s.pv, s.hout);
     return cudaGetLastError();
 }
 
@@ -805,9 +1106,16 @@ cudaError_t velocity_as(const StepView &s, const float4 *ps, cudaStream_t st, co
     cudaError_t e = rows_of(s, ps, s.iterations, st);
     if (e != cudaSuccess) return e;
     const RowArgs A = row_args(s);
-    k_row_vorticity<kFast><<<row_grid(s), 128, 0, st>>>(A, s.pv, s.omega, s.pom, s.vx);
+    const bool quads = by_quads(s);
+    if (quads)
+        k_quad_vorticity<kFast><<<quad_grid(s), 128, 0, st>>>(A, s.pv, s.omega, s.pom, s.vx);
+    else
+        k_row_vorticity<kFast><<<row_grid(s), 128, 0, st>>>(A, s.pv, s.omega, s.pom, s.vx);
     if (between) between();
-    k_row_apply<kFast><<<row_grid(s), 128, 0, st>>>(A, ps, s.omega, s.pom, s.vx, s.v1, s.x1, s.hout);
+    if (quads)
+        k_quad_apply<kFast><<<quad_grid(s), 128, 0, st>>>(A, ps, s.omega, s.pom, s.vx, s.v1, s.x1, s.hout);
+    else
+        k_row_apply<kFast><<<row_grid(s), 128, 0, st>>>(A, ps, s.omega, s.pom, s.vx, s.v1, s.x1, s.hout);
     return cudaGetLastError();
 }
 
@@ -838,8 +1146,8 @@ cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaS
 // scenes have too few cells to fill the GPU, and the ref profile's constants clump the fluid
 // into few crowded ones, so a cell's particles go to several warps.  us a step, groups that
 // end at multiples of 4 / 8 / 16 / 256: baseline 4 k 144 / 147 / 152 / 152, 14 k 163 / 158 /
-// 159 / 158, 50 k 235 / 227 / 223 / 222, 110 k 311 / 295 / 285 / 276; ref 14 k - / 441 / 471
-// / -, 50 k - / 594 / 589 / -, 262 k - / 1511 / 1472 / -.
+// 159 / 158, 64 k 235 / 227 / 223 / 222, 110 k 311 / 295 / 285 / 276; ref 14 k - / 441 / 471
+// / -, 64 k - / 594 / 589 / -, 262 k - / 1511 / 1472 / -.
 uint32_t row_group_mask(int profile, uint64_t n) {
     if (profile == FGB_PROFILE_REF) return n < 65536 ? 7u : 15u;
     return n < 8000 ? 3u : 255u;

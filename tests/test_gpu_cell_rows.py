@@ -128,3 +128,11 @@ def test_stale_groups_listed_first(n):
     # at either side of the size from which a later search lists its groups first, calm and not
     _same(capi.PROFILE_BASELINE, [_cloud(n, 24, n, obstacles=13, speed=0.2)], 6)
     _same(capi.PROFILE_BASELINE, [_cloud(n - 700, 24, n), _cloud(700, 5, n, speed=30.0)], 4)
+
+
+@pytest.mark.parametrize("profile", PROFILES)
+@pytest.mark.parametrize("n", [23997, 24003, 44998, 45001])
+@pytest.mark.parametrize("h,masses,obstacles", [(0.1, False, 0), (0.1, True, 9), (1.0, True, 9)])
+def test_four_lanes_or_one(profile, n, h, masses, obstacles):
+    # at either side of the sizes below which a particle has four lanes, in both forms of the root
+    _same(profile, [_cloud(n - 500, 15, n, h, masses, obstacles), _cloud(500, 1, 1, h, masses)], 3, h)
