@@ -270,6 +270,9 @@ void launch_unpack_static(const HostParticlesOut &out, uint64_t n, const float4 
 // vertex welding of device-resident triangles (weld.cu)
 int weld_device(const fgb_mesh_triangle *d_tris, uint64_t n_tris, uint32_t *d_index, float *d_vertices,
                 uint64_t *n_vertices, cudaStream_t st);
+void weld_release();
+// Host pages that the host has not touched yet, made ready for a copy into them (runtime.cu).
+void ready_output(void *p, size_t bytes);
 
 // marching cubes (mc.cu)
 struct SurfaceView {

@@ -1198,17 +1198,76 @@ struct fgb_batch {
     }
 };
 
+// Freed mesh buffers, for the next mesh: at most kMeshKeep bytes until a solver is destroyed.
+// A mesh a frame otherwise finds its pages new every time, and a copy into new pages takes
+// 1 to 3 ms where one into used pages takes 28 us (36 k triangles).
+static constexpr uint64_t kMeshKeep = 64ull << 20;
+struct MeshBuffers {
+    struct Buffer {
+        fgb_mesh_triangle *p;
+        uint64_t capacity;
+    };
+    std::mutex mutex;
+    std::vector<Buffer> kept;
+    uint64_t bytes = 0;
+
+    // the smallest that holds `count`, unless it is much too large ({null, 0}: none)
+    Buffer take(uint64_t count) {
+        std::lock_guard<std::mutex> lock(mutex);
+        size_t best = kept.size();
+        for (size_t i = 0; i < kept.size(); ++i)
+            if (kept[i].capacity >= count && kept[i].capacity / 8 <= count &&
+                (best == kept.size() || kept[i].capacity < kept[best].capacity))
+                best = i;
+        if (best == kept.size()) return {nullptr, 0};
+        const Buffer b = kept[best];
+        kept.erase(kept.begin() + (long)best);
+        bytes -= b.capacity * sizeof(fgb_mesh_triangle);
+        return b;
+    }
+    void give(fgb_mesh_triangle *p, uint64_t capacity) {
+        const uint64_t size = capacity * sizeof(fgb_mesh_triangle);
+        {
+            std::lock_guard<std::mutex> lock(mutex);
+            if (capacity && capacity <= kMeshKeep / sizeof(fgb_mesh_triangle) && bytes + size <= kMeshKeep) {
+                kept.push_back({p, capacity});
+                bytes += size;
+                return;
+            }
+        }
+        free(p);
+    }
+    void release() {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (const Buffer &b : kept) free(b.p);
+        kept.clear();
+        bytes = 0;
+    }
+};
+static MeshBuffers &mesh_buffers() {
+    static MeshBuffers *b = new MeshBuffers;  // never destroyed: meshes may be freed at exit
+    return *b;
+}
+
 static int mesh_assign(fgb_mesh *m, const fgb_mesh_triangle *dev, uint64_t count, cudaStream_t st) {
     if (!m) return FGB_OK;
     if (count > m->capacity || !m->triangles) {
         free(m->triangles);
-        m->triangles = (fgb_mesh_triangle *)malloc(std::max<uint64_t>(count, 1) * sizeof(fgb_mesh_triangle));
+        const MeshBuffers::Buffer kept = mesh_buffers().take(std::max<uint64_t>(count, 1));
+        m->triangles = kept.p;
+        m->capacity = kept.capacity;
         if (!m->triangles) {
-            m->capacity = 0;
-            m->n = 0;
-            return fail(FGB_ERR_OOM, "mesh: host allocation failed");
+            // room for a mesh that grows a little from frame to frame
+            const uint64_t room = std::max<uint64_t>(count + count / 8, 1);
+            m->triangles = (fgb_mesh_triangle *)malloc(room * sizeof(fgb_mesh_triangle));
+            if (!m->triangles) {
+                m->capacity = 0;
+                m->n = 0;
+                return fail(FGB_ERR_OOM, "mesh: host allocation failed");
+            }
+            m->capacity = room;
+            prefault_outputs({{m->triangles, count * sizeof(fgb_mesh_triangle)}});
         }
-        m->capacity = std::max<uint64_t>(count, 1);
     }
     m->n = count;
     if (count)
@@ -1912,6 +1971,8 @@ int fgb_destroy(fgb_solver *s) {
         cudaStreamDestroy(s->own);
     }
     delete s;
+    weld_release();
+    mesh_buffers().release();
     return FGB_OK;
 }
 
@@ -2048,6 +2109,8 @@ int fgb_batch_surface_all(fgb_batch *b, uint64_t *counts) {
 
 extern "C++" {
 namespace fgb {
+void ready_output(void *p, size_t bytes) { prefault_outputs({{p, bytes}}); }
+
 int batch_resident(fgb_batch *b, uint32_t k, ResidentScene *out) {
     if (!b || !out || k >= b->n_scenes) return fail(FGB_ERR_INVALID, "resident scene: bad argument");
     int rc = sync_ids(b);
@@ -2711,7 +2774,7 @@ int fgb_host_ready_pages(void *p, size_t bytes, int keep_contents, uint64_t *tou
 
 void fgb_mesh_free(fgb_mesh *m) {
     if (!m) return;
-    free(m->triangles);
+    if (m->triangles) mesh_buffers().give(m->triangles, m->capacity);
     m->triangles = nullptr;
     m->n = 0;
     m->capacity = 0;

@@ -59,3 +59,42 @@ def test_steps_surfaces_and_uploads_in_any_order(profile, n):
             _check(solver, batch, 0, cfg)
     batch.close()
     solver.close()
+
+
+def test_mesh_arrays_outlive_their_solver_and_welds_share_their_pool():
+    import gc
+    import threading
+
+    from libfluid_gb300.weld import weld
+
+    solver = SphSolver(params=capi.params(capi.PROFILE_BASELINE, H))
+    parts, cfg = _scene(capi.PROFILE_BASELINE, 4096, 3)
+    batch = Batch(solver, [(parts, cfg)])
+    batch.step(2)
+    mesh = batch.surface(0)
+    want = mesh.copy()
+    view = mesh[5:, :18]
+    again = batch.surface(0)  # another buffer: the first array is not written again
+    again[:] = 0
+    assert mesh.tobytes() == want.tobytes()
+    index, vertices = weld(mesh)
+    seen = []
+
+    def work():
+        for _ in range(5):
+            i, v = weld(want)
+            seen.append(i.tobytes() == index.tobytes() and v.tobytes() == vertices.tobytes())
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == [True] * 20
+    batch.close()
+    solver.close()
+    del mesh, again
+    gc.collect()
+    assert view.tobytes() == want[5:, :18].tobytes()
+    i, v = weld(want)  # after the pool was trimmed
+    assert i.tobytes() == index.tobytes() and v.tobytes() == vertices.tobytes()
