@@ -6,7 +6,7 @@
 
 namespace fgb {
 
-uint64_t scan_u32_scratch_bytes(uint64_t n) { return scan_scratch(n); }
+uint64_t scan_u32_scratch_bytes(uint64_t n) { return scan_scratch_short(n); }
 
 cudaError_t scan_u32(const uint32_t *in, uint32_t *out, uint32_t *total, uint64_t n, void *scratch,
                      uint64_t scratch_bytes, cudaStream_t stream, uint32_t *err, uint64_t *launches) {

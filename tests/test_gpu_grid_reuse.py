@@ -98,3 +98,21 @@ def test_mesh_arrays_outlive_their_solver_and_welds_share_their_pool():
     assert view.tobytes() == want[5:, :18].tobytes()
     i, v = weld(want)  # after the pool was trimmed
     assert i.tobytes() == index.tobytes() and v.tobytes() == vertices.tobytes()
+
+
+@pytest.mark.parametrize("n", [4095, 4097, 32 * 4096, 33 * 4096, 33 * 4096 + 1, 66 * 4096 + 7, 1200007])
+def test_scans_that_look_back_a_warp_at_a_time(n):
+    # around one tile and 32 of them, the most that a warp sees at once
+    import ctypes
+
+    torch = pytest.importorskip("torch")
+    lib = capi.load()
+    x = torch.from_numpy(np.random.default_rng(n).integers(0, 9, n, dtype=np.int32)).cuda()
+    out, total = torch.empty_like(x), torch.zeros(1, dtype=torch.int32, device="cuda")
+    size = lib.fgb_scan_scratch_bytes(n)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    capi.check(lib.fgb_exclusive_scan_u32(x.data_ptr(), out.data_ptr(), total.data_ptr(), n, scratch.data_ptr(),
+                                          size, stream))
+    want = np.cumsum(x.cpu().numpy())
+    assert (out.cpu().numpy()[1:] == want[:-1]).all() and int(out[0]) == 0 and int(total[0]) == want[-1]
