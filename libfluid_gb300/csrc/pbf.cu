@@ -956,17 +956,21 @@ __global__ void __launch_bounds__(256)
 // itself included) and moves toward 1.33x that mean by dt/750, per 8-bit channel,
 // clamped to [8, 255] and truncated.  The channel sums are integers below 2^24, exact
 // in float in any order, so each cell's sums are formed once (k_cell_colours, at the
-// cell's first sorted index) and a particle adds up 27 of them.
-__global__ void k_cell_colours(uint32_t n, const uint32_t *__restrict__ keys, const int32_t *__restrict__ type,
-                               const uint32_t *__restrict__ col, uint4 *__restrict__ agg,
-                               uint32_t *__restrict__ count) {
+// cell's first sorted index) and 27 of them added up for a cell's particles together.
+__global__ void k_cell_colours(const SceneDev *__restrict__ scenes, uint32_t n, uint32_t mbits,
+                               const uint32_t *__restrict__ keys, const uint2 *__restrict__ cells,
+                               const int32_t *__restrict__ type, const uint32_t *__restrict__ col,
+                               uint4 *__restrict__ agg, uint32_t *__restrict__ count) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t key = keys[i];
         if (i > 0 && keys[i - 1] == key) continue;
+        const SceneDev &S = scenes[scene_of(key, mbits)];
+        const uint32_t end = __ldg(&cells[S.table_base + morton_of(key, mbits)]).y;
         uint4 s = make_uint4(0, 0, 0, 0);
         uint32_t c = 0;
-        for (uint32_t j = i; j < n && keys[j] == key; ++j) {
-            if (type[j] == FGB_TYPE_OBSTACLE) continue;
+#pragma unroll 4
+        for (uint32_t j = i; j < end; ++j) {
+            if (S.obstacles && type[j] == FGB_TYPE_OBSTACLE) continue;
             const uint32_t v = col[j];
             s.x += v & 0xffu;
             s.y += (v >> 8) & 0xffu;
@@ -988,34 +992,49 @@ __device__ __forceinline__ uint32_t diffuse_channel(uint32_t own, uint32_t sum, 
     return (uint32_t)o;
 }
 
+// A warp takes 32 particles and, for each cell that they lie in, the sums of its neighbour cells:
+// a lane per cell (the sums are whole numbers, in any order).  With a thread per particle that
+// summed its 27 cells itself, and cell sums that ended where the key changes, the two kernels
+// took 24 us for 14 k particles, 29 for 262 k, 79 for 1 M; now 14, 22 and 58.
 __global__ void k_diffuse(const SceneDev *__restrict__ scenes, uint32_t n, uint32_t mbits,
                           const uint32_t *__restrict__ keys, const uint2 *__restrict__ cells,
                           const int32_t *__restrict__ type, const uint4 *__restrict__ agg,
                           const uint32_t *__restrict__ count, uint32_t *__restrict__ col) {
-    for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        if (type[a] == FGB_TYPE_OBSTACLE) continue;
-        const uint32_t key = keys[a];
-        const SceneDev &S = scenes[scene_of(key, mbits)];
-        const uint32_t m = morton_of(key, mbits);
-        const int cx = (int)compact10(m), cy = (int)compact10(m >> 1), cz = (int)compact10(m >> 2);
-        const uint2 *tbl = cells + S.table_base;
-        uint4 s = make_uint4(0, 0, 0, 0);
-        uint32_t c = 0;
-        for_cell_indices(S, cx, cy, cz, [&](uint32_t k) {
-            const uint2 r = __ldg(&tbl[k]);
-            if (r.x >= r.y) return;
-            const uint4 g = __ldg(&agg[r.x]);
-            s.x += g.x;
-            s.y += g.y;
-            s.z += g.z;
-            s.w += g.w;
-            c += __ldg(&count[r.x]);
-        });
-        const float t = S.dt / 750.f;
-        const float fc = (float)c;
-        const uint32_t v = col[a];
-        col[a] = diffuse_channel(v & 0xffu, s.x, fc, t) | (diffuse_channel((v >> 8) & 0xffu, s.y, fc, t) << 8) |
-                 (diffuse_channel((v >> 16) & 0xffu, s.z, fc, t) << 16) | (diffuse_channel(v >> 24, s.w, fc, t) << 24);
+    const uint32_t lane = threadIdx.x & 31u;
+    const int dz = (int)lane / 9 - 1, dy = (int)lane / 3 % 3 - 1, dx = (int)lane % 3 - 1;
+    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t a = base + lane;
+        const bool in = a < n;
+        const uint32_t key = in ? keys[a] : 0u;
+        const uint32_t left = __shfl_up_sync(0xffffffffu, key, 1);
+        for (unsigned starts = __ballot_sync(0xffffffffu, in && (lane == 0 || left != key)); starts;
+             starts &= starts - 1) {
+            const uint32_t cell = __shfl_sync(0xffffffffu, key, __ffs(starts) - 1);
+            const SceneDev &S = scenes[scene_of(cell, mbits)];
+            const uint32_t m = morton_of(cell, mbits);
+            const uint32_t x = compact10(m) + dx, y = compact10(m >> 1) + dy, z = compact10(m >> 2) + dz;
+            uint4 s = make_uint4(0, 0, 0, 0);
+            uint32_t c = 0;
+            if (lane < 27 && x <= S.ext[0] && y <= S.ext[1] && z <= S.ext[2]) {  // -1 wraps to above
+                const uint2 r = __ldg(&cells[S.table_base + morton3(x, y, z)]);
+                if (r.x < r.y) {
+                    s = __ldg(&agg[r.x]);
+                    c = __ldg(&count[r.x]);
+                }
+            }
+            s.x = __reduce_add_sync(0xffffffffu, s.x);
+            s.y = __reduce_add_sync(0xffffffffu, s.y);
+            s.z = __reduce_add_sync(0xffffffffu, s.z);
+            s.w = __reduce_add_sync(0xffffffffu, s.w);
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (!in || key != cell || type[a] == FGB_TYPE_OBSTACLE) continue;
+            const float t = S.dt / 750.f;
+            const float fc = (float)c;
+            const uint32_t v = col[a];
+            col[a] = diffuse_channel(v & 0xffu, s.x, fc, t) | (diffuse_channel((v >> 8) & 0xffu, s.y, fc, t) << 8) |
+                     (diffuse_channel((v >> 16) & 0xffu, s.z, fc, t) << 16) |
+                     (diffuse_channel(v >> 24, s.w, fc, t) << 24);
+        }
     }
 }
 
@@ -1266,7 +1285,8 @@ void launch_list_policy(const StepView &s, cudaStream_t st) {
 }
 
 void launch_diffuse(const StepView &s, uint4 *agg, uint32_t *count, cudaStream_t st) {
-    k_cell_colours<<<stream_grid(s.n), 256, 0, st>>>(s.n, s.keys_sorted, s.type1, s.col1, agg, count);
+    k_cell_colours<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.n, s.mbits, s.keys_sorted, s.cells, s.type1,
+                                                     s.col1, agg, count);
     k_diffuse<<<stream_grid(s.n), 256, 0, st>>>(s.scenes, s.n, s.mbits, s.keys_sorted, s.cells, s.type1, agg, count,
                                                 s.col1);
 }

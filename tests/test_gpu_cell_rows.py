@@ -136,3 +136,22 @@ def test_stale_groups_listed_first(n):
 def test_four_lanes_or_one(profile, n, h, masses, obstacles):
     # at either side of the sizes below which a particle has four lanes, in both forms of the root
     _same(profile, [_cloud(n - 500, 15, n, h, masses, obstacles), _cloud(500, 1, 1, h, masses)], 3, h)
+
+
+@pytest.mark.parametrize("n,side", [(1, 2), (31, 1), (65, 3), (4097, 7)])
+@pytest.mark.parametrize("obstacles", [0, 3])
+def test_colours_diffuse_as_the_oracle_has_them(n, side, obstacles):
+    from oracle import oracle
+    oracle.build()
+    params = capi.params(capi.PROFILE_REF, 0.1)
+    parts, cfg = _cloud(n, side, n, obstacles=obstacles)
+    parts["colour"][:] = np.random.default_rng(n).integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    want = scenes.copy_particles(parts)
+    solver = SphSolver(params=params)
+    b = Batch(solver, [(parts, cfg)])
+    for _ in range(3):
+        b.step(1)
+        oracle.step(params, cfg, want)
+        assert (b.download(0)["colour"] == want["colour"]).all()
+    b.close()
+    solver.close()
