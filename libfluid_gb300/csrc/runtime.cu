@@ -464,6 +464,7 @@ static constexpr uint32_t kMaxRowCap = 1024;  // Verlet and hit rows, entries pe
 static constexpr uint32_t kPieces = 4;
 
 static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu
+static constexpr uint32_t kCellHitsRef = 256;   // at first, with the ref profile, whose constants clump the fluid
 
 // Autotuner cache key: physics profile and floor(log2(particles)).
 static uint32_t tune_bucket(int32_t profile, uint64_t n) {
@@ -1522,7 +1523,7 @@ static int batch_init(fgb_batch *b) {
             FGB_CUDA(cudaMemcpy(pol.p, init.data(), init.size() * sizeof(RowPolicy), cudaMemcpyHostToDevice),
                      "batch alloc");
         }
-        if (p.profile == FGB_PROFILE_REF) b->cell_hits = 256;  // its constants clump the fluid
+        if (p.profile == FGB_PROFILE_REF) b->cell_hits = kCellHitsRef;
         auto it = s->cell_caps.find(tune_bucket(p.profile, n));
         if (it != s->cell_caps.end()) b->cell_hits = it->second;
     }
@@ -2442,6 +2443,8 @@ int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, 
     uint32_t cap = 96, hits = 64;
     if (const char *e = getenv("FGB_LIST_CAP")) cap = (uint32_t)atoi(e);
     if (const char *e = getenv("FGB_HIT_CAP")) hits = (uint32_t)atoi(e);
+    // the hit rows of rows.cu under the ref profile's constants are longer than both lists
+    if (s->params.profile == FGB_PROFILE_REF && !list_kernels_asked()) hits = kCellHitsRef;
     *bytes = scene_footprint(s->params, *cfg, n, want_mesh != 0, cap + hits);
     return FGB_OK;
 }
