@@ -135,7 +135,8 @@ struct StepView {
     float4 *pv;            // per particle: p* and mass, velocity after the last delta pass
     uint32_t *moved;       // per particle: at a cell's first, the largest movement in the cell
     uint8_t *lasting;      // per group
-    uint32_t *stale;       // room for the groups; their number for the step's k-th search at group_count[k]
+    uint32_t *stale;       // room for the groups; their number for the step's k-th search at group_count[k],
+                           // and at group_count[2 + iterations + k] how many of them warps asked for
     RowPolicy *row_policy, *row_policy_next;  // per scene: of the step before, and of this one
     // null, or [0] warps of the checked passes that ran on their near rows and [1]
     // warps that filtered their candidates instead (accumulated until read)

@@ -63,6 +63,7 @@ struct RowArgs {
     uint8_t *lasting;            // per group: its rows are the first search's, with the skin
     uint32_t *stale;             // first particles of the groups that a later search goes through
     uint32_t *stale_count;
+    uint32_t *taken;             // groups that the search's warps took beyond their first
     float inv_h;
     float skin, skin_r2;         // the skin, and (h + skin)^2
     const RowPolicy *policy;     // per scene, of the step before; policy_next of this one
@@ -277,7 +278,22 @@ __global__ void __launch_bounds__(kCellBlock, 7)
         }
         asked = used = 0;
     };
-    for (uint32_t c = blockIdx.x * kCellWarps + (threadIdx.x >> 5); c < groups; c += warps) {
+    // The group after this one, asked for before this one is worked on: by turns where there are
+    // few, else whichever is left, as groups' work differs with the flow (and by an order of
+    // magnitude where the ref profile's fluid clumps).  By turns / by demand: 262 k ref 1.46 /
+    // 1.41 ms a step, later 2.17 / 2.07; 1 M 2.05 / 2.02 and 2.09 / 2.06; for a few groups a warp
+    // the counter costs a small scene 2 us a search.
+    const bool by_demand = groups > 2 * warps;
+    auto after = [&](uint32_t c) {
+        if (!by_demand) return c + warps;
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(A.taken, 1u);
+        return warps + k;  // in lane 0
+    };
+    uint32_t next;
+    for (uint32_t c = blockIdx.x * kCellWarps + (threadIdx.x >> 5); c < groups;
+         c = __shfl_sync(0xffffffffu, next, 0)) {
+        next = after(c);
         const uint32_t first = list[c], key = A.keys[first], scene = scene_of(key, A.mbits);
         const SceneDev &S = A.scenes[scene];
         uint32_t cell;
@@ -1025,6 +1041,7 @@ RowArgs row_args(const StepView &s) {
     A.lasting = s.lasting;
     A.stale = s.stale;
     A.stale_count = nullptr;
+    A.taken = nullptr;
     A.inv_h = 1.f / s.ph.h;
     A.skin = kRowSkin * s.ph.h;
     const float reach = (s.ph.h + A.skin) * 1.00001f;
@@ -1052,6 +1069,7 @@ cudaError_t rows_of(const StepView &s, const float4 *ps, uint32_t pass, cudaStre
     const float r2max = (s.ph.profile == FGB_PROFILE_REF ? s.ph.hh_le : s.ph.hh) * 1.000002f;
     unsigned grid = 1;
     cudaError_t e;
+    A.taken = s.group_count + 2 + s.iterations + pass;
     if (pass == 0) {
         if (s.over) A.over = s.over + 1;  // counted once a step
         e = resident_grid(k_cell_rows<kFirstSearch>, s, kCellBlock, &grid);

@@ -1344,7 +1344,7 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
         FGB_CUDA(b->lasting.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->moved.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->stale.alloc(cap), "batch alloc groups");
-        FGB_CUDA(b->group_count.alloc(2 + b->iterations), "batch alloc groups");
+        FGB_CUDA(b->group_count.alloc(2 * (2 + b->iterations)), "batch alloc groups");
         int rc = b->alloc_cell_rows(cap);
         if (rc) return rc;
     }
