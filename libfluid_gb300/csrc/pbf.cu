@@ -96,7 +96,7 @@ OldCells old_cells(const StepView &s) {
 
 // What a step finds at its beginning, set by its first kernel: counters at zero, and the
 // sort's.  (As a memset each, and with a kernel each to count the digits and to sum the
-// counts, a step of 4096 particles took 144 us, 134 now; one of 14 k 159 and 150.)
+// counts, a step of 4096 particles took 144 us, 134 without them; one of 14 k 159 and 150.)
 struct StepBegin {
     uint32_t *mass_range, *over, *group_count, *digits_next, *sort_state;
     uint32_t group_counts;

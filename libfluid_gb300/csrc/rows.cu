@@ -15,8 +15,8 @@
 // straight to their lanes), 21 went to a cell's setup, 34 to its candidates, 120 to the
 // particle: 36 tests, 27 appends, 10 the running sum, 12 the writing of its row.  In 32 bits
 // with a ballot for every 32 candidates it took 222.  The first lambda stage (search and
-// sums) of the 1 M dam break at steps 5, 30 and 100: 357, 387 and 357 us before, 319, 334
-// and 323 now.
+// sums) of the 1 M dam break at steps 5, 30 and 100: 357, 387 and 357 us before, 318, 328
+// and 319 now.
 //
 // Rows that last.  The step's first search keeps every candidate within h plus a skin of
 // the grid positions.  Such a row holds every neighbour within h, in order, while no
@@ -1075,7 +1075,7 @@ cudaError_t rows_of(const StepView &s, const float4 *ps, uint32_t pass, cudaStre
         e = resident_grid(k_cell_rows<kFirstSearch>, s, kCellBlock, &grid);
         if (e != cudaSuccess) return e;
         k_cell_rows<kFirstSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, 0);
-    } else if (s.ph.profile == FGB_PROFILE_REF || s.n < kListFrom) {
+    } else if (row_later_search_launches(s.ph.profile, s.n) == 1) {
         e = resident_grid(k_cell_rows<kLaterSearch>, s, kCellBlock, &grid);
         if (e != cudaSuccess) return e;
         k_cell_rows<kLaterSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, pass == 1);
@@ -1158,6 +1158,10 @@ cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_
 cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaStream_t st,
                                        const std::function<void()> &between) {
     return s.ph.fast_root ? velocity_as<true>(s, ps, st, between) : velocity_as<false>(s, ps, st, between);
+}
+
+uint32_t row_later_search_launches(int profile, uint64_t n) {
+    return profile == FGB_PROFILE_REF || n < kListFrom ? 1u : 2u;
 }
 
 // Particles of a group.  A cell's setup is shared by the particles of its group, but small

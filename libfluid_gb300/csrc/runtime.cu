@@ -797,7 +797,7 @@ struct fgb_batch {
                 mark(k, st);
                 FGB_CUDA(launch_row_delta(s, pin, pout, it + 1 == iterations, st), "step: delta rows");
                 mark(k, st);
-                l += 3;
+                l += 2 + (it ? row_later_search_launches(ph.profile, n) : 1);
                 pin = pout;
                 continue;
             }
@@ -820,7 +820,7 @@ struct fgb_batch {
             else
                 launch_velocity_terms(s, pin, st, [&] { mark(k, st); });
             mark(k, st);
-            l += cell_rows ? 3 : 2;
+            l += 2 + (cell_rows ? row_later_search_launches(ph.profile, n) : 0);
         }
         if (s.list_policy && s.cap) {
             launch_list_policy(s, st);
@@ -1335,6 +1335,7 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     FGB_CUDA(b->keys_sorted.alloc(cap), "batch alloc");
     FGB_CUDA(b->vals_sorted.alloc(cap), "batch alloc");
     FGB_CUDA(b->mc_keys.alloc(cap), "batch alloc");  // of the surface; the steps' first kernel may read them
+    FGB_CUDA(cudaMemsetAsync(b->mc_keys.p, 0, cap * sizeof(uint32_t), b->stream()), "batch alloc");
     b->grid_unknown = true;
     FGB_CUDA(b->cells_of.alloc(1), "batch alloc");
     for (auto &d : b->digits) FGB_CUDA(d.alloc(kMaxPasses * kRadix), "batch alloc");
@@ -1601,15 +1602,23 @@ static int sync_ids(fgb_batch *b) {
     return FGB_OK;
 }
 
+// A scene of several gets its key prefix back (a sort whose wait gave up may have left it
+// another's); the keys then no longer tell which cells the table holds.
+static void scene_prefix(fgb_batch *b, uint32_t k) {
+    if (b->n_scenes == 1) return;  // every key is of scene 0
+    launch_fill_u32(b->keys_sorted.p + b->first[k], b->counts[k], b->mbits >= 32 ? 0u : (k << b->mbits), b->stream());
+    b->grid_unknown = true;
+}
+
 // What every upload ends with: the scene table learns whether the scene holds
-// obstacles.  (The scene's keys keep its prefix, from the batch's creation on: sorted
-// keys stay in their scenes' segments.)
+// obstacles.
 static void upload_done(fgb_batch *b, uint32_t k, uint32_t obstacles) {
     b->query_ok = false;
     if (b->h_scenes[k].obstacles != obstacles) {
         b->h_scenes[k].obstacles = obstacles;
         b->tris_dirty = true;  // re-uploads the scene table before the next step
     }
+    scene_prefix(b, k);
 }
 
 // One kernel reads the caller's arrays and writes the scene segment (ids go to
@@ -1724,6 +1733,7 @@ static int batch_copy_scene(fgb_batch *dst, uint32_t dk, fgb_batch *src, uint32_
         FGB_CUDA(cudaMemcpyAsync(dst->ids_dev.p + fd, src->ids_dev.p + fs, n * sizeof(uint64_t),
                                  cudaMemcpyDeviceToDevice, st),
                  "copy_scene");
+        scene_prefix(dst, dk);
     }
     if (src->direct && !dst->direct) {  // dst keeps its ids on the host
         dst->ids[dk].assign(n, 0);
