@@ -235,7 +235,8 @@ int fgb_batch_error_flags(fgb_batch *b, uint32_t *flags);
  * over the steps since the last call, which clears them: [0] warps that ran on their
  * near rows, [1] warps that filtered their candidates instead, and among the particles
  * of later lambda passes that filtered, [2] those whose Verlet list held and [3] those
- * that walked their 27 cells.  Writes min(n, 4) values, zeros without FGB_ROW_STATS.
+ * that walked their 27 cells.  (FGB_ROW_STATS asks for the list kernels, whose passes
+ * these are.)  Writes min(n, 4) values, zeros without FGB_ROW_STATS.
  * Synchronous. */
 int fgb_batch_row_stats(fgb_batch *b, uint32_t *stats, uint32_t n);
 /* Number of kernels this batch launched since creation (for accounting). */
@@ -245,7 +246,9 @@ uint64_t fgb_batch_launch_count(const fgb_batch *b);
  * (predict, sort, reorder, lambda/delta per iteration, vorticity, vorticity apply);
  * fgb_batch_stage_times returns the last step's per-stage milliseconds. */
 int fgb_batch_set_timing(fgb_batch *b, int on);
-/* Autotuner: runs the batch's next steps under each candidate launch shape (gather
+/* Autotuner: runs the batch's next steps under each candidate launch shape of the list
+ * kernels, which a list setting in the environment asks for (the row kernels, used
+ * otherwise, choose theirs by the scene's size: there the trials are plain steps) (gather
  * CTA size 64, 128, 256 at the current Verlet skin, then skins 0.1-0.3 h at the best
  * size, then persistent tile queues of 1 and 2 particles per thread, then near rows
  * with and without Verlet lists in turn (five trials); steps_per_trial steps each, the
@@ -276,6 +279,7 @@ int fgb_batch_stage_times(fgb_batch *b, float *ms, uint32_t max, uint32_t *count
 #define FGB_PROBE_DENSITY     5 /* f32 density of the last solver iteration */
 #define FGB_PROBE_LATTICE     6 /* f32x4 MC lattice (value, normal) of the last surface call */
 #define FGB_PROBE_CUBE_CASES  7 /* u8 MC case index per cube of the last surface call */
+/* 8, 9, 10 and 11 are of the list kernels; 0xffff, 0, 0 and 0 on the row kernels */
 #define FGB_PROBE_LIST_COUNT  8 /* u16 neighbour-list length per particle (0xffff: overflow) */
 #define FGB_PROBE_LIST_VALID  9 /* u8 per particle: 1 if its list served the last vorticity pass */
 #define FGB_PROBE_DISPLACEMENT 10 /* f32 distance moved since the grid was built (last delta) */
