@@ -19,6 +19,7 @@ uint32_t scene_morton_bits(const fgb_solver *s, const fgb_config *cfg);
 
 // radix sort (sort.cu)
 uint64_t radix_scratch_bytes(uint64_t n);
+uint64_t radix_scratch_bytes_short(uint64_t n);  // with which sorts of up to n keys take short tiles
 int radix_passes(uint32_t key_bits);
 cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
                              uint32_t *vals_out, uint64_t n, uint32_t key_bits, void *scratch,
@@ -26,7 +27,7 @@ cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, u
                              const uint32_t *counted);
 // What a sort with `counted` (the digits' counts of its keys, digit_counts.cuh) asks to be
 // zero before it: `words` from the returned address.
-uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t *words);
+uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t scratch_bytes, uint64_t *words);
 
 // Copy a device error-flag word to *flags and clear it, after the work queued on
 // stream (synchronises the stream; allocates nothing).

@@ -708,7 +708,7 @@ struct fgb_batch {
         s.digits = digits[c].p;
         s.digits_next = digits[c ^ 1].p;
         s.sort_passes = radix_passes(key_bits);
-        s.sort_state = radix_state(n, key_bits, sort_scratch.p, &s.sort_state_n);
+        s.sort_state = radix_state(n, key_bits, sort_scratch.p, sort_scratch_bytes, &s.sort_state_n);
         s.group_counts = (uint32_t)group_count.n;
         s.ps_a = ps[0].p;
         s.ps_b = ps[1].p;
@@ -1358,7 +1358,7 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     b->grid_unknown = true;
     FGB_CUDA(b->cells_of.alloc(1), "batch alloc");
     for (auto &d : b->digits) FGB_CUDA(d.alloc(kMaxPasses * kRadix), "batch alloc");
-    b->sort_scratch_bytes = radix_scratch_bytes(cap);
+    b->sort_scratch_bytes = radix_scratch_bytes_short(cap);
     FGB_CUDA(b->sort_scratch.alloc(b->sort_scratch_bytes), "batch alloc");
     FGB_CUDA(b->ps_grid.alloc(cap + 1), "batch alloc");
     if (b->cell_rows) {

@@ -6,12 +6,13 @@
 // every sum over it) is a deterministic function of the input.
 //
 // Per pass (8-bit digit): each CTA takes the next tile id from an atomic counter,
-// ranks its 4096 keys with warp-level match_any (in index order, hence stable),
+// ranks its 4096 keys (1024 in a short sort) with warp-level match_any (in index order, hence stable),
 // publishes its per-digit counts, looks back over earlier tiles' published counts
 // (decoupled look-back) to find where its keys start, and scatters.  The digits of all
 // passes are counted before the first: by a kernel of their own, or by the one that makes
 // the keys (digit_counts.cuh); each tile sums the counts of its pass itself.  Every
 // look-back wait is bounded.
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -25,8 +26,11 @@ namespace {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
-constexpr int kTile = kSortThreads * kSortItems;  // 4096 keys per tile
+// Keys a thread takes.  A short sort waits for its few tiles' ranking, key after key: a pass
+// over 4 k or 14 k keys takes 2 us less with 4 than with 16; from 64 k keys on they are equal,
+// and for 1 M, where more tiles are more to look back over, 16 take 14 us and 4 take 19.
+constexpr int kSortItems = 16, kShortItems = 4;
+constexpr uint64_t kShortSort = 32768;  // keys below which a sort is short
 
 constexpr uint32_t kFlagAggregate = 1u << 30;
 constexpr uint32_t kFlagInclusive = 2u << 30;
@@ -43,6 +47,7 @@ __global__ void __launch_bounds__(256) k_radix_histogram(const uint32_t *__restr
     counts.give(hist, passes);
 }
 
+template <int kItems>
 __global__ void __launch_bounds__(kSortThreads) k_onesweep(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
     uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n, int shift,
@@ -58,11 +63,11 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
     for (int i = tid; i < kSortWarps * (kRadix + 1); i += kSortThreads) (&s_hist[0][0])[i] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
-    const uint32_t base = tile * (uint32_t)kTile + (uint32_t)w * 32u * kSortItems;
+    const uint32_t base = tile * (uint32_t)(kSortThreads * kItems) + (uint32_t)w * 32u * kItems;
 
-    uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
+    uint32_t k[kItems], v[kItems], rank[kItems];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < kItems; ++i) {
         uint32_t idx = base + (uint32_t)i * 32u + (uint32_t)lane;
         bool ok = idx < n;
         k[i] = ok ? keys_in[idx] : 0u;
@@ -82,7 +87,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
         below -= own;
     }
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < kItems; ++i) {
         uint32_t idx = base + (uint32_t)i * 32u + (uint32_t)lane;
         uint32_t d = idx < n ? ((k[i] >> shift) & (kRadix - 1)) : (uint32_t)kRadix;
         uint32_t peers = __match_any_sync(0xffffffffu, d);
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep(
     __syncthreads();
 
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
+    for (int i = 0; i < kItems; ++i) {
         uint32_t idx = base + (uint32_t)i * 32u + (uint32_t)lane;
         if (idx < n) {
             uint32_t d = (k[i] >> shift) & (kRadix - 1);
@@ -159,9 +164,10 @@ struct SortLayout {
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-SortLayout sort_layout(uint64_t n) {
+SortLayout sort_layout(uint64_t n, int items = kSortItems) {
     SortLayout L;
-    L.tiles = (uint32_t)((n + kTile - 1) / kTile);
+    const uint64_t tile = (uint64_t)kSortThreads * items;
+    L.tiles = (uint32_t)((n + tile - 1) / tile);
     size_t o = 0;
     L.hist = o;
     o = align256(o + sizeof(uint32_t) * kMaxPasses * kRadix);
@@ -190,13 +196,22 @@ LookbackCtl lookback_ctl() {
 
 uint64_t radix_scratch_bytes(uint64_t n) { return sort_layout(n).total; }
 
+uint64_t radix_scratch_bytes_short(uint64_t n) {
+    return std::max(sort_layout(n).total, sort_layout(std::min(n, kShortSort), kShortItems).total);
+}
+
+// Whether a sort of n keys in a scratch of that size takes the short tiles.
+static bool short_sort(uint64_t n, uint64_t scratch_bytes) {
+    return n < kShortSort && scratch_bytes >= sort_layout(n, kShortItems).total;
+}
+
 int radix_passes(uint32_t key_bits) {
     int p = (int)((key_bits + kRadixBits - 1) / kRadixBits);
     return p < 1 ? 1 : p;
 }
 
-uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t *words) {
-    const SortLayout L = sort_layout(n);
+uint32_t *radix_state(uint64_t n, uint32_t key_bits, void *scratch, uint64_t scratch_bytes, uint64_t *words) {
+    const SortLayout L = sort_layout(n, short_sort(n, scratch_bytes) ? kShortItems : kSortItems);
     *words = (L.status - L.counters) / sizeof(uint32_t) + (uint64_t)radix_passes(key_bits) * L.tiles * kRadix;
     return (uint32_t *)((char *)scratch + L.counters);
 }
@@ -207,7 +222,8 @@ cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, u
                              uint64_t *launches, const uint32_t *counted) {
     if (n == 0) return cudaSuccess;
     if (key_bits > 32 || n > (uint64_t)kValueMask) return cudaErrorInvalidValue;
-    SortLayout L = sort_layout(n);
+    const bool brief = short_sort(n, scratch_bytes);
+    SortLayout L = sort_layout(n, brief ? kShortItems : kSortItems);
     if (scratch_bytes < L.total || scratch == nullptr) return cudaErrorInvalidValue;
     char *s = (char *)scratch;
     uint32_t *hist = (uint32_t *)(s + L.hist);
@@ -232,7 +248,8 @@ cudaError_t radix_sort_pairs(const uint32_t *keys_in, const uint32_t *vals_in, u
         bool to_out = ((passes - 1 - p) % 2) == 0;
         uint32_t *dk = to_out ? keys_out : alt_k;
         uint32_t *dv = to_out ? vals_out : alt_v;
-        k_onesweep<<<L.tiles, kSortThreads, 0, stream>>>(
+        auto kernel = brief ? k_onesweep<kShortItems> : k_onesweep<kSortItems>;
+        kernel<<<L.tiles, kSortThreads, 0, stream>>>(
             src_k, src_v, dk, dv, (uint32_t)n, p * kRadixBits, counted + p * kRadix,
             status + (size_t)p * L.tiles * kRadix, counters + p, err, ctl);
         src_k = dk;

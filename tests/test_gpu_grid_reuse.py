@@ -116,3 +116,23 @@ def test_scans_that_look_back_a_warp_at_a_time(n):
                                           size, stream))
     want = np.cumsum(x.cpu().numpy())
     assert (out.cpu().numpy()[1:] == want[:-1]).all() and int(out[0]) == 0 and int(total[0]) == want[-1]
+
+
+@pytest.mark.parametrize("n", [1023, 1025, 5000, 32767, 32768])
+def test_steps_on_short_sorts_order_as_the_oracle(n):
+    # around a short sort's tile, and the size from which tiles are longer
+    from oracle import oracle
+    oracle.build()
+    params = capi.params(capi.PROFILE_BASELINE, H)
+    parts, cfg = scenes.cube_scene(32768, 7)
+    keep = np.sort(np.random.default_rng(n).permutation(32768)[:n])
+    parts = {f: (v.reshape(32768, -1)[keep].ravel() if len(v) != n else v).copy() for f, v in parts.items()}
+    solver = SphSolver(params=params)
+    b = Batch(solver, [(scenes.copy_particles(parts), cfg)])
+    for _ in range(3):
+        b.step(1)
+        pr = oracle.step(params, cfg, parts, probe=True)
+        assert (b.probe(capi.PROBE_KEYS, np.uint32) == np.sort(b.probe(capi.PROBE_KEYS, np.uint32))).all()
+        assert (b.download(0)["id"] == parts["id"]).all()
+    b.close()
+    solver.close()
