@@ -2076,7 +2076,7 @@ int fgb_batch_set_colliders(fgb_batch *b, uint32_t scene, const fgb_triangle *tr
 int fgb_batch_step(fgb_batch *b, uint32_t steps) {
     if (!b) return fail(FGB_ERR_INVALID, "step: null batch");
     if (b->n == 0) return FGB_OK;
-    // flags raised by steps that have finished (copied by their graphs): the state is
+    // flags raised by steps that have finished (k_report): the state is
     // suspect, so nothing more is queued until fgb_batch_error_flags clears them
     int rc = flags_status(b->st_flags.p[0], "step");
     if (rc) return rc;
