@@ -104,8 +104,8 @@ struct Pools {
     std::map<int, cudaMemPool_t> of_device;
 };
 Pools &pools() {
-    static Pools p;
-    return p;
+    static Pools *p = new Pools;  // never destroyed: solvers may be at exit
+    return *p;
 }
 
 // The current device's pool (null: it has none).
