@@ -1089,13 +1089,17 @@ struct fgb_batch {
     }
 
     // Where the sorted keys no longer tell which cells the table holds: an empty table, and
-    // the counts that a step leaves for the next one.
+    // the counts that a step leaves for the next one.  The sort's scratch too, whose parts lie
+    // where the particles' number puts them: a sort whose wait gave up leaves entries unwritten,
+    // and what its next pass finds there has to be a key and an index of this batch, as every
+    // later kernel takes it for one.
     int fresh_grid() {
         if (!grid_unknown) return FGB_OK;
         FGB_CUDA(cudaMemsetAsync(cells.p, 0, cells_n * sizeof(uint2), stream()), "clear cells");
         FGB_CUDA(cudaMemsetAsync(cells_of.p, 0, sizeof(uint32_t), stream()), "clear cells");
         for (auto &d : digits)
             FGB_CUDA(cudaMemsetAsync(d.p, 0, kMaxPasses * kRadix * sizeof(uint32_t), stream()), "clear digit counts");
+        FGB_CUDA(cudaMemsetAsync(sort_scratch.p, 0, sort_scratch_bytes, stream()), "clear sort scratch");
         grid_unknown = false;
         return FGB_OK;
     }
@@ -1132,6 +1136,7 @@ struct fgb_batch {
         if (surf_ready) return FGB_OK;
         PoolScope scope(&solver->pool);
         FGB_CUDA(mc_vals.alloc(n), "surface alloc");
+        FGB_CUDA(cudaMemsetAsync(mc_vals.p, 0, mc_vals.n * sizeof(uint32_t), stream()), "surface alloc");  // as vals_sorted
         FGB_CUDA(mc_xs.alloc(n), "surface alloc");
         FGB_CUDA(mc_type.alloc(n), "surface alloc");
         FGB_CUDA(mc_col.alloc(n), "surface alloc");
@@ -1353,6 +1358,8 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     FGB_CUDA(b->vals_in.alloc(cap), "batch alloc");
     FGB_CUDA(b->keys_sorted.alloc(cap), "batch alloc");
     FGB_CUDA(b->vals_sorted.alloc(cap), "batch alloc");
+    // indices of some particle where a sort leaves them unwritten (fresh_grid)
+    FGB_CUDA(cudaMemsetAsync(b->vals_sorted.p, 0, cap * sizeof(uint32_t), b->stream()), "batch alloc");
     FGB_CUDA(b->mc_keys.alloc(cap), "batch alloc");  // of the surface; the steps' first kernel may read them
     FGB_CUDA(cudaMemsetAsync(b->mc_keys.p, 0, cap * sizeof(uint32_t), b->stream()), "batch alloc");
     b->grid_unknown = true;
@@ -1624,7 +1631,7 @@ static int sync_ids(fgb_batch *b) {
 // A scene of several gets its key prefix back (a sort whose wait gave up may have left it
 // another's); the keys then no longer tell which cells the table holds.
 static void scene_prefix(fgb_batch *b, uint32_t k) {
-    if (b->n_scenes == 1) return;  // every key is of scene 0
+    if (b->n_scenes == 1) return;  // every key is of scene 0, after such a sort as well (fresh_grid)
     launch_fill_u32(b->keys_sorted.p + b->first[k], b->counts[k], b->mbits >= 32 ? 0u : (k << b->mbits), b->stream());
     b->grid_unknown = true;
 }
