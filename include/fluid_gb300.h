@@ -450,6 +450,9 @@ int fgb_scan_noalloc_error(void *cuda_stream, uint32_t *flags);
  * while the hook is set keeps it.  fgb_test_lookback_fault(0xffffffff, 0) restores
  * the defaults.  Process-wide; not for production use. */
 int fgb_test_lookback_fault(uint32_t skip_tile, uint32_t spin_limit);
+/* Test hook: device blocks of more than `bytes` bytes are refused, as by a device that
+ * has no memory for them (0: none are).  Process-wide; existing blocks stay. */
+int fgb_test_alloc_limit(uint64_t bytes);
 
 /* ---- packed record streams (the reference demo's memory-mapped result files) --
  * Replaces strucures::writeParticles / writeTriangles (samples/structures.hpp:

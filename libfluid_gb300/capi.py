@@ -313,6 +313,7 @@ _SIGS = {
     "fgb_scan_error": (ctypes.c_int, [c_void_p, ctypes.c_uint64, c_void_p, P(ctypes.c_uint32)]),
     "fgb_scan_noalloc_error": (ctypes.c_int, [c_void_p, P(ctypes.c_uint32)]),
     "fgb_test_lookback_fault": (ctypes.c_int, [ctypes.c_uint32, ctypes.c_uint32]),
+    "fgb_test_alloc_limit": (ctypes.c_int, [ctypes.c_uint64]),
     "fgb_host_ready_pages": (ctypes.c_int, [c_void_p, ctypes.c_size_t, ctypes.c_int, P(ctypes.c_uint64)]),
     "fgb_advance_records": (ctypes.c_int, [c_void_p, P(Config), P(Records), P(Triangle), ctypes.c_size_t, P(Query),
                                            ctypes.c_size_t, P(QueryResult), P(ctypes.c_size_t), P(Mesh)]),

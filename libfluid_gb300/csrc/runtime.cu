@@ -93,6 +93,14 @@ __global__ void k_scene_first_triangles(const SceneDev *__restrict__ scenes, uin
     }
 }
 
+// Blocks larger than this are refused, as if the device had no room (fgb_test_alloc_limit;
+// 0: none are).
+std::atomic<uint64_t> g_alloc_limit{0};
+bool alloc_refused(size_t bytes) {
+    const uint64_t limit = g_alloc_limit.load(std::memory_order_relaxed);
+    return limit && bytes > limit;
+}
+
 // Device blocks of one solver's batches, kept for reuse instead of freed.  Every
 // batch of a solver queues its work on the solver's stream, so a block handed back
 // while kernels that use it are still queued can go to the next allocation of the
@@ -114,6 +122,10 @@ class DevPool {
     }
     void *get(size_t bytes, cudaError_t *e) {
         const size_t c = size_class(bytes);
+        if (alloc_refused(bytes)) {
+            *e = cudaErrorMemoryAllocation;
+            return nullptr;
+        }
         {
             std::lock_guard<std::mutex> lk(mu_);
             auto it = free_.find(c);
@@ -481,6 +493,7 @@ static constexpr uint32_t kMaxRowCap = 1024;  // Verlet and hit rows, entries pe
 static constexpr uint32_t kPieces = 4;
 
 static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu
+static constexpr uint32_t kLeastCellHits = 16;  // where memory is short
 static constexpr uint32_t kCellHitsRef = 256;   // at first, with the ref profile, whose constants clump the fluid
 
 // Autotuner cache key: physics profile and floor(log2(particles)).
@@ -557,8 +570,9 @@ struct fgb_batch {
     // velocities straight into the caller's arrays, named per frame in hout_dev
     bool advance_io = false;
     Dev<HostParticlesOut> hout_dev;
-    // rows that overflowed in each step's build pass, reported to st_over at the end of
-    // the step; grow_rows() enlarges the capacities when more than 1% did
+    // rows that overflowed in each step's build pass, reported to st_over at the end of a
+    // call's steps; grow_rows() enlarges the capacities by them
+    bool rows_full = false;  // there was no memory for longer rows: they do not grow any more
     // over[2..3]: near-row statistics of the checked passes (FGB_ROW_STATS=1), kept
     // on the device across steps until fgb_batch_row_stats reads and clears them
     Dev<uint32_t> over;
@@ -997,6 +1011,7 @@ struct fgb_batch {
 
     int build_graphs() {
         cudaStream_t st = stream();
+        if (cell_rows && !hlist.p) return fail(FGB_ERR_OOM, "step: the batch has no hit rows");
         for (int c = 0; c < 2; ++c) {
             cudaGraph_t g = nullptr;
             FGB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture begin");
@@ -1029,47 +1044,61 @@ struct fgb_batch {
         return FGB_OK;
     }
 
-    // Rows that overflow send their particles' passes back to the 27-cell walk; when
-    // more than 1% of a step's particles overflowed (dense, compressed scenes: the
-    // ref profile's constants clump the fluid to ~200-400 neighbours within h), the
-    // capacity grows by half (at most 1024) and the solver remembers it for the
-    // bucket.  The counts arrive in st_over from steps already run.
+    // Rows that overflow send their particles' passes back to the 27-cell walk, which gives
+    // the same sums later.  So the capacity grows by half, and the solver remembers it for the
+    // bucket: on the list kernels (dense, compressed scenes: the ref profile's constants clump
+    // the fluid to ~200-400 neighbours within h) when more than 1% of a step's particles
+    // overflowed, to at most kMaxRowCap entries; on the row kernels when more than n / 50000
+    // did, to at most kMaxCellHits.  The counts arrive in st_over from steps already run.
+    // Longer rows come beside the present ones or not at all: without memory for both the
+    // batch keeps what it has and asks no more.
     int grow_rows() {
-        if (!st_over.p) return FGB_OK;
-        const uint64_t lim = std::max<uint64_t>(n / 100, 1);
+        if (!st_over.p || rows_full) return FGB_OK;
+        const uint64_t lim = std::max<uint64_t>(n / 100, 1), rows = capacity ? capacity : n;
         if (cell_rows) {
             // a row that overflowed holds up its warp's other rows, by 27 cells of a clump:
             // hardly any may.  (Up to n / 5000 of them made steps of 110 k particles with the
             // ref profile 1.58 ms instead of 0.94, of 1 M 5.27 instead of 4.62.)
             if (st_over.p[1] <= n / 50000 || cell_hits >= kMaxCellHits) return FGB_OK;
             FGB_CUDA(cudaStreamSynchronize(stream()), "grow hit rows sync");
-            cell_hits = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 3) & ~3u);
             st_over.p[0] = st_over.p[1] = 0;
-            drop_graphs();
+            const uint32_t more = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 3) & ~3u);
+            rows_full = !replace_rows(hlist, rows_of(rows) * more);
+            if (rows_full) return FGB_OK;
+            cell_hits = more;
             solver->cell_caps[tune_bucket(solver->params.profile, n)] = cell_hits;
-            return alloc_cell_rows(capacity ? capacity : n);
+            drop_graphs();
+            return no_rows(rows);
         }
         const bool gl = list_cap && st_over.p[0] > lim && list_cap < kMaxRowCap;
         const bool gh = hit_cap && st_over.p[1] > lim && hit_cap < kMaxRowCap;
         if (!gl && !gh) return FGB_OK;
         // copies queued by earlier steps would report the old capacities
         FGB_CUDA(cudaStreamSynchronize(stream()), "grow rows sync");
-        PoolScope scope(&solver->pool);
-        const uint64_t rows = capacity ? capacity : n;
-        if (gl) {
-            list_cap = std::min<uint32_t>(kMaxRowCap, (list_cap * 3 / 2 + 3u) & ~3u);
-            FGB_CUDA(nlist.alloc(rows * list_cap), "grow neighbour lists");
-        }
-        if (gh) {
-            hit_cap = std::min<uint32_t>(kMaxRowCap, (hit_cap * 3 / 2 + 3u) & ~3u);
-            FGB_CUDA(hlist.alloc(rows * hit_cap), "grow hit lists");
-        }
         st_over.p[0] = st_over.p[1] = 0;
-        for (auto &g : graph)
-            if (g) cudaGraphExecDestroy(g), g = nullptr;
-        graphs_ok = false;
+        auto grow = [&](Dev<uint32_t> &list, uint32_t &entries) {
+            const uint32_t more = std::min<uint32_t>(kMaxRowCap, (entries * 3 / 2 + 3u) & ~3u);
+            if (!replace_rows(list, rows * more)) return false;
+            entries = more;
+            drop_graphs();
+            return true;
+        };
+        if (gl && !grow(nlist, list_cap)) rows_full = true;
+        if (gh && !grow(hlist, hit_cap)) rows_full = true;
         solver->caps[tune_bucket(solver->params.profile, n)] = fgb_solver::Caps{list_cap, hit_cap};
         return FGB_OK;
+    }
+
+    // `words` words in place of a list's block, unless there is no memory for them beside it.
+    bool replace_rows(Dev<uint32_t> &list, uint64_t words) {
+        PoolScope scope(&solver->pool);
+        Dev<uint32_t> next;
+        if (next.alloc(words) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        list.swap(next);
+        return true;
     }
 
     void drop_graphs() {
@@ -1078,14 +1107,28 @@ struct fgb_batch {
         graphs_ok = false;
     }
 
-    // The hit rows of rows.cu for cap particles, interleaved by 32 of them.  Every row
-    // starts as overflowed: one that a step did not write is never read.
-    int alloc_cell_rows(uint64_t cap) {
-        PoolScope scope(&solver->pool);
-        FGB_CUDA(hlist.alloc((cap + 31) / 32 * 32 * cell_hits), "hit rows");
-        FGB_CUDA(hcount.alloc(cap), "hit rows");
+    // The hit rows of rows.cu, interleaved by 32 particles of them.
+    static uint64_t rows_of(uint64_t particles) { return (particles + 31) / 32 * 32; }
+
+    // Every row starts as overflowed: one that a step did not write is never read.
+    int no_rows(uint64_t cap) {
         FGB_CUDA(cudaMemsetAsync(hcount.p, 0xff, cap * sizeof(uint16_t), stream()), "hit rows");
         return FGB_OK;
+    }
+
+    // For cap particles rows of cell_hits entries, or shorter ones where there is no memory
+    // for them (particles whose neighbours do not fit walk their cells).
+    int alloc_cell_rows(uint64_t cap) {
+        PoolScope scope(&solver->pool);
+        FGB_CUDA(hcount.alloc(cap), "hit rows");
+        hlist.release();
+        rows_full = false;
+        while (!replace_rows(hlist, rows_of(cap) * cell_hits)) {
+            if (cell_hits <= kLeastCellHits) return fail(FGB_ERR_OOM, "hit rows: out of device memory");
+            cell_hits = std::max(kLeastCellHits, cell_hits / 2 & ~3u);
+            rows_full = true;
+        }
+        return no_rows(cap);
     }
 
     // Where the sorted keys no longer tell which cells the table holds: an empty table, and
@@ -1374,8 +1417,6 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
         FGB_CUDA(b->moved.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->stale.alloc(cap), "batch alloc groups");
         FGB_CUDA(b->group_count.alloc(2 * (2 + b->iterations)), "batch alloc groups");
-        int rc = b->alloc_cell_rows(cap);
-        if (rc) return rc;
     }
     if (!b->cell_rows && b->list_cap) {
         FGB_CUDA(b->cellmax.alloc(std::max<uint64_t>(b->cells_n, 1)), "batch alloc");
@@ -1401,6 +1442,10 @@ static int alloc_step_arrays(fgb_batch *b, uint64_t cap) {
     } else {
         FGB_CUDA(b->colour_sums.alloc(cap), "batch alloc");
         FGB_CUDA(b->colour_count.alloc(cap), "batch alloc");
+    }
+    if (b->cell_rows) {  // last: rows take what the other arrays leave
+        int rc = b->alloc_cell_rows(cap);
+        if (rc) return rc;
     }
     cudaStream_t st = b->stream();
     if (b->cell_rows) {  // the far entry: infinity, out of every pass's range
@@ -2800,6 +2845,13 @@ int fgb_batch_query(fgb_batch *b, uint32_t scene, const fgb_query *queries, size
     if (!b || !n_results || scene >= b->n_scenes || (n && (!queries || !results)))
         return fail(FGB_ERR_INVALID, "query: bad argument");
     return batch_query(b, scene, queries, n, results, n_results);
+}
+
+// Refuse device blocks above `bytes` (0: none), as a device without memory for them does:
+// for tests of what a refusal leaves.
+int fgb_test_alloc_limit(uint64_t bytes) {
+    g_alloc_limit.store(bytes, std::memory_order_relaxed);
+    return FGB_OK;
 }
 
 int fgb_host_ready_pages(void *p, size_t bytes, int keep_contents, uint64_t *touched) {
