@@ -39,6 +39,7 @@ def _crowd(n, seed=1):
 def _steps(batch):
     for steps in CALLS:
         batch.step(steps)
+        batch.sync()  # what overflowed is known at the next call
     got = batch.download(0)
     assert batch.error_flags() == 0
     return got
