@@ -333,7 +333,8 @@ typedef struct fgb_drain {
 int fgb_batch_sources_drains(fgb_batch *b, uint32_t scene, const fgb_source *sources, uint32_t n_sources,
                              const fgb_drain *drains, uint32_t n_drains, uint64_t *count);
 /* Device bytes one scene of n particles occupies in a batch (with its surface
- * buffers when want_mesh); used for admission against an HBM budget. */
+ * buffers when want_mesh); used for admission against an HBM budget.  Rows of
+ * neighbours count as long as this solver's batches of that size have grown them. */
 int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, int want_mesh, uint64_t *bytes);
 
 /* ---- serving: a resident request loop with continuous batching ---------- */

@@ -493,8 +493,9 @@ static constexpr uint32_t kMaxRowCap = 1024;  // Verlet and hit rows, entries pe
 static constexpr uint32_t kPieces = 4;
 
 static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu
+static constexpr uint32_t kCellWords = 16;      // words a particle beside its hit row
 static constexpr uint32_t kLeastCellHits = 16;  // where memory is short
-static constexpr uint32_t kCellHitsRef = 256;   // at first, with the ref profile, whose constants clump the fluid
+static constexpr uint32_t kCellHits = 96, kCellHitsRef = 256;  // at first; the ref profile's constants clump the fluid
 
 // Autotuner cache key: physics profile and floor(log2(particles)).
 static uint32_t tune_bucket(int32_t profile, uint64_t n) {
@@ -526,7 +527,15 @@ struct fgb_solver {
         uint32_t list, hit;
     };
     std::map<uint32_t, Caps> caps;
-    std::map<uint32_t, uint32_t> cell_caps;  // the same for the hit rows of rows.cu
+    // the same for the hit rows of rows.cu, per log2 n (0: not grown); a server's callers read
+    // them for a footprint while its batches grow
+    std::atomic<uint32_t> cell_caps[64] = {};
+    std::atomic<uint32_t> &cell_cap(uint64_t n) { return cell_caps[tune_bucket(params.profile, n) % 64u]; }
+    // entries of a new batch's rows
+    uint32_t first_cell_hits(uint64_t n) {
+        const uint32_t grown = cell_cap(n).load();
+        return grown ? grown : params.profile == FGB_PROFILE_REF ? kCellHitsRef : kCellHits;
+    }
     fgb_batch *cached = nullptr;  // single-scene batch behind fgb_advance
     uint64_t cached_n = 0;
     fgb_config cached_cfg{};
@@ -621,7 +630,7 @@ struct fgb_batch {
     // the gathers run on hit rows from one warp per cell (rows.cu), else on the list
     // kernels (pbf.cu)
     bool cell_rows = false;
-    uint32_t cell_hits = 96;  // entries of a hit row of rows.cu
+    uint32_t cell_hits = kCellHits;  // entries of a hit row of rows.cu
     uint32_t group_mask = 31;
     Dev<uint32_t> groups, group_count, moved;
     Dev<uint32_t> stale;  // per search, the first particles of the groups it goes through
@@ -1066,7 +1075,7 @@ struct fgb_batch {
             rows_full = !replace_rows(hlist, rows_of(rows) * more);
             if (rows_full) return FGB_OK;
             cell_hits = more;
-            solver->cell_caps[tune_bucket(solver->params.profile, n)] = cell_hits;
+            solver->cell_cap(n) = cell_hits;
             drop_graphs();
             return no_rows(rows);
         }
@@ -1597,9 +1606,7 @@ static int batch_init(fgb_batch *b) {
             FGB_CUDA(cudaMemcpy(pol.p, init.data(), init.size() * sizeof(RowPolicy), cudaMemcpyHostToDevice),
                      "batch alloc");
         }
-        if (p.profile == FGB_PROFILE_REF) b->cell_hits = kCellHitsRef;
-        auto it = s->cell_caps.find(tune_bucket(p.profile, n));
-        if (it != s->cell_caps.end()) b->cell_hits = it->second;
+        b->cell_hits = s->first_cell_hits(n);
     }
     int rc = alloc_step_arrays(b, n);
     if (rc) return rc;
@@ -2526,9 +2533,12 @@ int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, 
     uint32_t cap = 96, hits = 64;
     if (const char *e = getenv("FGB_LIST_CAP")) cap = (uint32_t)atoi(e);
     if (const char *e = getenv("FGB_HIT_CAP")) hits = (uint32_t)atoi(e);
-    // the hit rows of rows.cu under the ref profile's constants are longer than both lists
-    if (s->params.profile == FGB_PROFILE_REF && !list_kernels_asked()) hits = kCellHitsRef;
-    *bytes = scene_footprint(s->params, *cfg, n, want_mesh != 0, cap + hits);
+    // rows.cu: the hit rows as long as the solver's batches of that size have them, and what
+    // goes with them (the groups' arrays, the records of position and velocity)
+    uint32_t words = cap + hits;
+    if (!list_kernels_asked())
+        words = std::max(words, const_cast<fgb_solver *>(s)->first_cell_hits(n) + kCellWords);
+    *bytes = scene_footprint(s->params, *cfg, n, want_mesh != 0, words);
     return FGB_OK;
 }
 
