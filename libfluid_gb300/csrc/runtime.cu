@@ -492,7 +492,7 @@ static constexpr uint64_t kPieceMin = 1u << 18;
 static constexpr uint32_t kMaxRowCap = 1024;  // Verlet and hit rows, entries per particle
 static constexpr uint32_t kPieces = 4;
 
-static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu
+static constexpr uint32_t kMaxCellHits = 4096;  // entries of a hit row of rows.cu (grow_rows)
 static constexpr uint32_t kCellWords = 16;      // words a particle beside its hit row
 static constexpr uint32_t kLeastCellHits = 16;  // where memory is short
 static constexpr uint32_t kCellHits = 96, kCellHitsRef = 256;  // at first; the ref profile's constants clump the fluid
@@ -1058,9 +1058,11 @@ struct fgb_batch {
     // bucket: on the list kernels (dense, compressed scenes: the ref profile's constants clump
     // the fluid to ~200-400 neighbours within h) when more than 1% of a step's particles
     // overflowed, to at most kMaxRowCap entries; on the row kernels when more than n / 50000
-    // did, to at most kMaxCellHits.  The counts arrive in st_over from steps already run.
-    // Longer rows come beside the present ones or not at all: without memory for both the
-    // batch keeps what it has and asks no more.
+    // did, to at most kMaxRowCap entries as well, or kMaxCellHits where it is more than 1%:
+    // all particles' rows have one length, which a single clump shall not set.  The counts
+    // arrive in st_over from steps already run.  Longer rows come beside the present ones, in
+    // at most half of the memory that the device has free, or not at all: the batch then keeps
+    // what it has and asks no more.
     int grow_rows() {
         if (!st_over.p || rows_full) return FGB_OK;
         const uint64_t lim = std::max<uint64_t>(n / 100, 1), rows = capacity ? capacity : n;
@@ -1068,11 +1070,15 @@ struct fgb_batch {
             // a row that overflowed holds up its warp's other rows, by 27 cells of a clump:
             // hardly any may.  (Up to n / 5000 of them made steps of 110 k particles with the
             // ref profile 1.58 ms instead of 0.94, of 1 M 5.27 instead of 4.62.)
-            if (st_over.p[1] <= n / 50000 || cell_hits >= kMaxCellHits) return FGB_OK;
+            const uint32_t most = st_over.p[1] > lim ? kMaxCellHits : kMaxRowCap;
+            if (st_over.p[1] <= n / 50000 || cell_hits >= most) return FGB_OK;
             FGB_CUDA(cudaStreamSynchronize(stream()), "grow hit rows sync");
             st_over.p[0] = st_over.p[1] = 0;
-            const uint32_t more = std::min<uint32_t>(kMaxCellHits, (cell_hits * 3 / 2 + 3) & ~3u);
-            rows_full = !replace_rows(hlist, rows_of(rows) * more);
+            const uint32_t more = std::min<uint32_t>(most, (cell_hits * 3 / 2 + 3) & ~3u);
+            size_t free_bytes = 0, all_bytes = 0;
+            FGB_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes), "grow hit rows");
+            rows_full = rows_of(rows) * more * sizeof(uint32_t) > free_bytes / 2 ||
+                        !replace_rows(hlist, rows_of(rows) * more);
             if (rows_full) return FGB_OK;
             cell_hits = more;
             solver->cell_cap(n) = cell_hits;

@@ -49,3 +49,30 @@ def test_footprints_count_the_rows_at_hand(profile, words, rest):
     assert _per_particle(solver, cfg, 200000) == before  # another size class
     batch.close()
     solver.close()
+
+
+def test_a_clump_does_not_set_the_rows_of_a_large_scene():
+    """Four clumps of 6000 obstacles among 262 k particles: far fewer than one in a hundred have
+    more than 1024 neighbours, and those walk their cells."""
+    solver = SphSolver(params=capi.params(capi.PROFILE_BASELINE, 0.1))
+    rng = np.random.default_rng(5)
+    side, clumps, each = 64, 4, 6000
+    calm = scenes.block((side, side, side), (0.0, 0.0, 0.0), 5)
+    n = side ** 3 + clumps * each
+    parts = scenes.block((n, 1, 1), (0.0, 0.0, 0.0), 5)
+    pos = parts["position"].reshape(-1, 3)
+    pos[: side ** 3] = calm["position"].reshape(-1, 3)
+    for k in range(clumps):
+        at = slice(side ** 3 + k * each, side ** 3 + (k + 1) * each)
+        pos[at] = 1.0 + 0.3 * k + 0.12 * (rng.random((each, 3)).astype(np.float32) - np.float32(0.5))
+        parts["type"][at] = capi.TYPE_OBSTACLE
+    e = side * scenes.SPACING
+    cfg = scenes.config((0.0, 0.0, 0.0), (e, e, e))
+    batch = Batch(solver, [(parts, cfg)])
+    for _ in range(14):
+        batch.step(1)
+        batch.sync()
+    words = (_per_particle(solver, cfg, n - 2000) - 242) / 4 - 16
+    assert words == 1024
+    batch.close()
+    solver.close()
