@@ -340,7 +340,8 @@ int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, 
 /* ---- serving: a resident request loop with continuous batching ---------- */
 /* A worker thread admits requests in arrival order while the sum of their device
  * footprints (fgb_scene_footprint) stays within half the budget (a membership
- * change briefly holds two batches) and keeps admitted scenes resident.  Resident
+ * change briefly holds two batches) and keeps admitted scenes resident.  Rows of
+ * neighbours that grow beyond the footprints grow into what that leaves, no further.  Resident
  * scenes are packed into groups of at most tick_particles particles; a tick
  * advances one group by one batched step, the groups taken round robin.  Finished
  * scenes optionally get a surface; their final state waits on the host for

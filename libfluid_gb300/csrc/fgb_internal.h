@@ -17,6 +17,14 @@ int fail_cuda(cudaError_t e, const char *where);
 // Morton key bits of one scene's grid under a solver's h (runtime.cu).
 uint32_t scene_morton_bits(const fgb_solver *s, const fgb_config *cfg);
 
+// A server's budget (serve.cu, runtime.cu).  fgb_scene_footprint, and the bytes of it that are for
+// the scene's rows of neighbours; the most that the rows of a batch may take from now on, when it
+// is made and as it steps; what a batch's rows take.
+int scene_footprint_rows(const fgb_solver *s, const fgb_config *cfg, uint64_t n, bool mesh, uint64_t *bytes,
+                         uint64_t *rows);
+void limit_rows(fgb_solver *s, uint64_t bytes);
+uint64_t batch_row_bytes(const fgb_batch *b);
+
 // radix sort (sort.cu)
 uint64_t radix_scratch_bytes(uint64_t n);
 uint64_t radix_scratch_bytes_short(uint64_t n);  // with which sorts of up to n keys take short tiles

@@ -531,6 +531,7 @@ struct fgb_solver {
     // them for a footprint while its batches grow
     std::atomic<uint32_t> cell_caps[64] = {};
     std::atomic<uint32_t> &cell_cap(uint64_t n) { return cell_caps[tune_bucket(params.profile, n) % 64u]; }
+    uint64_t row_limit = UINT64_MAX;  // bytes of one batch's hit rows (a server's budget: limit_rows)
     // entries of a new batch's rows
     uint32_t first_cell_hits(uint64_t n) {
         const uint32_t grown = cell_cap(n).load();
@@ -1072,9 +1073,10 @@ struct fgb_batch {
             // ref profile 1.58 ms instead of 0.94, of 1 M 5.27 instead of 4.62.)
             const uint32_t most = st_over.p[1] > lim ? kMaxCellHits : kMaxRowCap;
             if (st_over.p[1] <= n / 50000 || cell_hits >= most) return FGB_OK;
+            const uint32_t more = std::min<uint32_t>(most, (cell_hits * 3 / 2 + 3) & ~3u);
+            if (rows_of(rows) * more * sizeof(uint32_t) > solver->row_limit) return FGB_OK;
             FGB_CUDA(cudaStreamSynchronize(stream()), "grow hit rows sync");
             st_over.p[0] = st_over.p[1] = 0;
-            const uint32_t more = std::min<uint32_t>(most, (cell_hits * 3 / 2 + 3) & ~3u);
             size_t free_bytes = 0, all_bytes = 0;
             FGB_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes), "grow hit rows");
             rows_full = rows_of(rows) * more * sizeof(uint32_t) > free_bytes / 2 ||
@@ -1613,6 +1615,8 @@ static int batch_init(fgb_batch *b) {
                      "batch alloc");
         }
         b->cell_hits = s->first_cell_hits(n);
+        if (fgb_batch::rows_of(n) * b->cell_hits * sizeof(uint32_t) > s->row_limit)
+            b->cell_hits = std::min(b->cell_hits, p.profile == FGB_PROFILE_REF ? kCellHitsRef : kCellHits);
     }
     int rc = alloc_step_arrays(b, n);
     if (rc) return rc;
@@ -2534,18 +2538,40 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     return FGB_OK;
 }
 
-int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, int want_mesh, uint64_t *bytes) {
-    if (!s || !cfg || !bytes) return fail(FGB_ERR_INVALID, "footprint: bad argument");
+extern "C++" {
+namespace fgb {
+// The footprint of a scene, and the bytes of it that its rows of neighbours may take.
+static uint64_t footprint_of(const fgb_solver *s, const fgb_config &cfg, uint64_t n, bool mesh, uint64_t *rows) {
     uint32_t cap = 96, hits = 64;
     if (const char *e = getenv("FGB_LIST_CAP")) cap = (uint32_t)atoi(e);
     if (const char *e = getenv("FGB_HIT_CAP")) hits = (uint32_t)atoi(e);
     // rows.cu: the hit rows as long as the solver's batches of that size have them, and what
     // goes with them (the groups' arrays, the records of position and velocity)
-    uint32_t words = cap + hits;
-    if (!list_kernels_asked())
-        words = std::max(words, const_cast<fgb_solver *>(s)->first_cell_hits(n) + kCellWords);
-    *bytes = scene_footprint(s->params, *cfg, n, want_mesh != 0, words);
+    uint32_t words = cap + hits, beside = 0;
+    if (!list_kernels_asked()) {
+        beside = kCellWords;
+        words = std::max(words, const_cast<fgb_solver *>(s)->first_cell_hits(n) + beside);
+    }
+    *rows = sizeof(uint32_t) * n * (words - beside);
+    return scene_footprint(s->params, cfg, n, mesh, words);
+}
+
+int scene_footprint_rows(const fgb_solver *s, const fgb_config *cfg, uint64_t n, bool mesh, uint64_t *bytes,
+                         uint64_t *rows) {
+    if (!s || !cfg || !bytes || !rows) return fail(FGB_ERR_INVALID, "footprint: bad argument");
+    *bytes = footprint_of(s, *cfg, n, mesh, rows);
     return FGB_OK;
+}
+
+void limit_rows(fgb_solver *s, uint64_t bytes) { s->row_limit = bytes; }
+
+uint64_t batch_row_bytes(const fgb_batch *b) { return (b->nlist.n + b->hlist.n) * sizeof(uint32_t); }
+}  // namespace fgb
+}  // extern "C++"
+
+int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, int want_mesh, uint64_t *bytes) {
+    uint64_t rows = 0;
+    return scene_footprint_rows(s, cfg, n, want_mesh != 0, bytes, &rows);
 }
 
 int fgb_batch_grid_info(fgb_batch *b, uint32_t scene, fgb_grid_info *out) {

@@ -19,7 +19,9 @@
 // cubes, their final state is copied to the host, and their memory is released.
 //
 // Budget accounting: rebuilding a group holds its old and new batch at once, so
-// admission keeps the sum of active footprints within half the budget.
+// admission keeps the sum of active footprints within half the budget.  Rows of
+// neighbours that grow beyond the footprints of a group's scenes count as well: they
+// grow into what admission has left, and it waits for what they took.
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -55,7 +57,7 @@ struct Request {
     fgb_config cfg{};
     uint32_t steps = 0, remaining = 0;
     bool want_mesh = false;
-    uint64_t n = 0, footprint = 0;
+    uint64_t n = 0, footprint = 0, rows = 0;  // rows: the part of the footprint for rows of neighbours
     uint32_t mbits = 0;
     std::vector<uint64_t> id;
     std::vector<int32_t> type;
@@ -84,6 +86,14 @@ struct ServeGroup {
     std::vector<Request *> want;    // membership for the next tick
     uint64_t particles = 0;         // of `want`
     uint32_t mbits = 0;             // largest Morton key width in `want`
+
+    uint64_t charged = 0;           // bytes for rows in the footprints of the scenes of `batch`
+
+    // what the batch's rows take beyond that
+    uint64_t beyond() const {
+        const uint64_t have = batch ? fgb::batch_row_bytes(batch) : 0;
+        return have > charged ? have - charged : 0;
+    }
 };
 
 struct fgb_server {
@@ -96,6 +106,7 @@ struct fgb_server {
     std::vector<Request *> live;                         // admitted and still running
     std::map<uint64_t, std::unique_ptr<Request>> requests;
     uint64_t used = 0, next_ticket = 1;
+    uint64_t beyond = 0;  // of all groups: their rows beyond the footprints in `used` (set by the worker)
     bool stop = false;
     double last_submit = -1, gap = -1;  // the last arrival, and its distance from the one before (under mu)
     double t0 = 0;
@@ -131,7 +142,7 @@ struct fgb_server {
             }
             if (opt.one_at_a_time && !live.empty()) break;
             if (live.size() >= opt.max_active) break;
-            if (used + r->footprint > cap_bytes) break;
+            if (used + beyond + r->footprint > cap_bytes) break;
             waiting.pop_front();
             used += r->footprint;
             r->status = FGB_SERVE_ACTIVE;
@@ -140,6 +151,24 @@ struct fgb_server {
             fresh.push_back(r);
         }
         return fresh;
+    }
+
+    // The groups' rows as they are now, into `beyond`; and for a group that is about to step, or
+    // to be made anew of scenes charged with that much: its rows may take what the budget leaves.
+    void count_rows() {
+        uint64_t sum = 0;
+        for (auto &g : groups) sum += g->beyond();
+        std::lock_guard<std::mutex> lk(mu);
+        beyond = sum;
+    }
+    void allow_rows(const ServeGroup &g, uint64_t charged) {
+        uint64_t left = 0;
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            const uint64_t cap_bytes = opt.budget_bytes / 2, taken = used + beyond;
+            left = cap_bytes > taken ? cap_bytes - taken : 0;
+        }
+        fgb::limit_rows(solver, charged + g.beyond() + left);
     }
 
     // Whether r may join a group of `particles` particles, `count` scenes and Morton
@@ -257,13 +286,16 @@ struct fgb_server {
     int rebuild(ServeGroup &g, const std::map<Request *, Home> &where, std::vector<fgb_batch *> &retired) {
         const double r0 = now_s();
         fgb_batch *nb = nullptr;
+        uint64_t charged = 0;
         if (!g.want.empty()) {
             std::vector<uint64_t> counts;
             std::vector<fgb_config> cfgs;
             for (Request *r : g.want) {
                 counts.push_back(r->n);
                 cfgs.push_back(r->cfg);
+                charged += r->rows;
             }
+            allow_rows(g, charged);
             int rc = fgb_batch_create(solver, (uint32_t)g.want.size(), counts.data(), cfgs.data(), &nb);
             if (rc) return rc;
             for (size_t k = 0; k < g.want.size(); ++k) {
@@ -290,6 +322,7 @@ struct fgb_server {
         if (g.batch) retired.push_back(g.batch);
         g.batch = nb;
         g.scenes = g.want;
+        g.charged = charged;
         std::lock_guard<std::mutex> lk(mu);
         rebuilds++;
         rebuild_time += now_s() - r0;
@@ -349,6 +382,7 @@ struct fgb_server {
     // and go home.
     void tick(ServeGroup &g) {
         const uint32_t k = tick_steps(g);
+        allow_rows(g, g.charged);
         const double s0 = now_s();
         int rc = fgb_batch_step(g.batch, k);
         if (!rc) rc = fgb_batch_sync(g.batch);
@@ -454,6 +488,7 @@ struct fgb_server {
             for (auto &g : groups)
                 if (!g->want.empty()) kept.push_back(std::move(g));
             groups.swap(kept);
+            count_rows();
             // round robin over the groups that hold scenes
             ServeGroup *pick = nullptr;
             for (size_t i = 0; i < groups.size() && !pick; ++i) {
@@ -464,10 +499,12 @@ struct fgb_server {
                 }
             }
             if (pick) tick(*pick);
+            count_rows();
         }
         for (auto &g : groups)
             if (g->batch) fgb_batch_destroy(g->batch);
         groups.clear();
+        fgb::limit_rows(solver, UINT64_MAX);
     }
 };
 
@@ -501,7 +538,7 @@ int fgb_serve_submit(fgb_server *sv, const fgb_config *cfg, const fgb_particles 
     r->steps = r->remaining = steps;
     r->want_mesh = want_mesh != 0;
     r->n = xs->n;
-    int rc = fgb_scene_footprint(sv->solver, cfg, xs->n, want_mesh, &r->footprint);
+    int rc = fgb::scene_footprint_rows(sv->solver, cfg, xs->n, want_mesh != 0, &r->footprint, &r->rows);
     if (rc) return rc;
     // Morton bits of the scene's grid: admission keeps scene id + key within 32 bits
     r->mbits = fgb::scene_morton_bits(sv->solver, cfg);
