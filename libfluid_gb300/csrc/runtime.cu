@@ -142,6 +142,7 @@ class DevPool {
             (void)cudaGetLastError();
             trim();
             *e = cudaMalloc(&p, c);
+            if (*e != cudaSuccess) (void)cudaGetLastError();  // the caller's to report, not the next launch's
         }
         return *e == cudaSuccess ? p : nullptr;
     }
@@ -551,6 +552,8 @@ struct fgb_batch {
     std::vector<uint64_t> counts, first;
     uint64_t n = 0;
     uint64_t capacity = 0;  // particles the per-particle arrays hold (>= n)
+    bool lost = false;      // there was no memory for the per-step arrays: no step, surface or edit
+    int usable() const { return lost ? fail(FGB_ERR_OOM, "the batch has no step arrays: out of device memory") : FGB_OK; }
     uint32_t mbits = 0, sbits = 0, key_bits = 0, iterations = 0;
     std::vector<SceneDev> h_scenes;
     Dev<SceneDev> d_scenes;
@@ -1021,7 +1024,6 @@ struct fgb_batch {
 
     int build_graphs() {
         cudaStream_t st = stream();
-        if (cell_rows && !hlist.p) return fail(FGB_ERR_OOM, "step: the batch has no hit rows");
         for (int c = 0; c < 2; ++c) {
             cudaGraph_t g = nullptr;
             FGB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "graph capture begin");
@@ -1043,7 +1045,8 @@ struct fgb_batch {
     // Everything the first step would set up: the scene table and the two step
     // graphs, instantiated and uploaded to the device.
     int prepare() {
-        int rc = sync_tris();
+        int rc = usable();
+        if (!rc) rc = sync_tris();
         if (rc) return rc;
         if (!graphs_ok) {
             rc = build_graphs();
@@ -1165,7 +1168,8 @@ struct fgb_batch {
     }
 
     int step(uint32_t steps) {
-        int rc = grow_rows();
+        int rc = usable();
+        if (!rc) rc = grow_rows();
         if (rc) return rc;
         rc = sync_tris();
         if (rc) return rc;
@@ -1213,7 +1217,8 @@ struct fgb_batch {
 
     // Grid over the current positions, then field + classify + scan for scenes [b, e).
     int surface_count(uint32_t b, uint32_t e, uint64_t *tri_total) {
-        int rc = sync_tris();  // the scene table (obstacle counts) as of the last upload
+        int rc = usable();
+        if (!rc) rc = sync_tris();  // the scene table (obstacle counts) as of the last upload
         if (!rc) rc = ensure_surface();
         if (!rc) rc = fresh_grid();
         if (rc) return rc;
@@ -1690,13 +1695,47 @@ static int sync_ids(fgb_batch *b) {
     return FGB_OK;
 }
 
+// The particles' keys as a new batch has them: nothing but the scene's prefix.
+static void scene_keys(fgb_batch *b, uint32_t k) {
+    if (b->lost) return;
+    launch_fill_u32(b->keys_sorted.p + b->first[k], b->counts[k], b->mbits >= 32 ? 0u : (k << b->mbits), b->stream());
+    b->grid_unknown = true;
+}
+
 // A scene of several gets its key prefix back (a sort whose wait gave up may have left it
 // another's); the keys then no longer tell which cells the table holds.
 static void scene_prefix(fgb_batch *b, uint32_t k) {
     if (b->n_scenes == 1) return;  // every key is of scene 0, after such a sort as well (fresh_grid)
-    launch_fill_u32(b->keys_sorted.p + b->first[k], b->counts[k], b->mbits >= 32 ? 0u : (k << b->mbits), b->stream());
-    b->grid_unknown = true;
+    scene_keys(b, k);
 }
+
+// The arrays of a batch's state set, to take the place of one of its two.
+struct StateSet {
+    Dev<float4> x, v;
+    Dev<int32_t> type;
+    Dev<uint32_t> col, slot;
+    struct Arrays {
+        float4 *x, *v;
+        int32_t *type;
+        uint32_t *col, *slot;
+    };
+    cudaError_t alloc(uint64_t cap) {
+        cudaError_t e = x.alloc(cap);
+        if (e == cudaSuccess) e = v.alloc(cap);
+        if (e == cudaSuccess) e = type.alloc(cap + 1);
+        if (e == cudaSuccess) e = col.alloc(cap);
+        if (e == cudaSuccess) e = slot.alloc(cap);
+        return e;
+    }
+    Arrays arrays() const { return Arrays{x.p, v.p, type.p, col.p, slot.p}; }
+    void swap(fgb_batch *b, int c) {
+        x.swap(b->x[c]);
+        v.swap(b->v[c]);
+        type.swap(b->type[c]);
+        col.swap(b->col[c]);
+        slot.swap(b->slot[c]);
+    }
+};
 
 // What every upload ends with: the scene table learns whether the scene holds
 // obstacles.
@@ -2382,6 +2421,7 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
                              const fgb_drain *drains, uint32_t n_drains, uint64_t *count) {
     if (!b || !count || k >= b->n_scenes) return fail(FGB_ERR_INVALID, "sources_drains: bad argument");
     if ((n_sources && !sources) || (n_drains && !drains)) return fail(FGB_ERR_INVALID, "sources_drains: null array");
+    if (int rc = b->usable()) return rc;
     const fgb_config &c = b->cfg[k];
     PoolScope scope(&b->solver->pool);
     b->query_ok = false;
@@ -2458,20 +2498,18 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
     if (n1 > 0x7fffffffull) return fail(FGB_ERR_CAPACITY, "sources_drains: more than 2^31-1 particles");
     const bool grow = n1 > b->capacity;
     const uint64_t cap = grow ? std::max<uint64_t>(n1, b->capacity + b->capacity / 4) : b->capacity;
-    if (grow) {
-        FGB_CUDA(b->x[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->type[cn].alloc(cap + 1), "sources_drains grow");
-        FGB_CUDA(b->col[cn].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->slot[cn].alloc(cap), "sources_drains grow");
-    }
+    // larger arrays come beside the batch's: without memory for them the batch stays as it is
+    StateSet larger[2];
+    for (int c = 0; grow && c < 2; ++c) FGB_CUDA(larger[c].alloc(cap), "sources_drains grow");
+    const StateSet::Arrays to = grow ? larger[0].arrays()
+                                     : StateSet::Arrays{b->x[cn].p, b->v[cn].p, b->type[cn].p, b->col[cn].p, b->slot[cn].p};
     Dev<uint64_t> ids1;
     FGB_CUDA(ids1.alloc(cap), "sources_drains alloc");
     FGB_CUDA(cudaMemcpyAsync(d_moves.p, moves.data(), b->n_scenes * sizeof(SceneMove), cudaMemcpyHostToDevice, st),
              "sources_drains moves");
     launch_edit_scatter(n0, b->mbits, k, E, b->keys_sorted.p, keep.p, rank.p, d_moves.p, b->x[cs].p, b->v[cs].p,
-                        b->type[cs].p, b->col[cs].p, b->slot[cs].p, b->ids_dev.p, b->x[cn].p, b->v[cn].p,
-                        b->type[cn].p, b->col[cn].p, b->slot[cn].p, ids1.p, st);
+                        b->type[cs].p, b->col[cs].p, b->slot[cs].p, b->ids_dev.p, to.x, to.v, to.type, to.col, to.slot,
+                        ids1.p, st);
     FGB_CUDA(cudaGetLastError(), "sources_drains scatter");
     if (E) {  // the emitted particles, after the scene's survivors
         FGB_CUDA(b->st_x.ensure(E), "sources_drains staging");
@@ -2489,25 +2527,33 @@ int fgb_batch_sources_drains(fgb_batch *b, uint32_t k, const fgb_source *sources
             b->st_ids.p[e] = eid[e];
         }
         const uint64_t d = first[k] + kept_k;
-        FGB_CUDA(cudaMemcpyAsync(b->x[cn].p + d, b->st_x.p, E * sizeof(float4), cudaMemcpyHostToDevice, st), "emit");
-        FGB_CUDA(cudaMemcpyAsync(b->v[cn].p + d, b->st_v.p, E * sizeof(float4), cudaMemcpyHostToDevice, st), "emit");
-        FGB_CUDA(cudaMemcpyAsync(b->type[cn].p + d, b->st_type.p, E * sizeof(int32_t), cudaMemcpyHostToDevice, st),
+        FGB_CUDA(cudaMemcpyAsync(to.x + d, b->st_x.p, E * sizeof(float4), cudaMemcpyHostToDevice, st), "emit");
+        FGB_CUDA(cudaMemcpyAsync(to.v + d, b->st_v.p, E * sizeof(float4), cudaMemcpyHostToDevice, st), "emit");
+        FGB_CUDA(cudaMemcpyAsync(to.type + d, b->st_type.p, E * sizeof(int32_t), cudaMemcpyHostToDevice, st),
                  "emit");
-        FGB_CUDA(cudaMemcpyAsync(b->col[cn].p + d, b->st_col.p, E * sizeof(uint32_t), cudaMemcpyHostToDevice, st),
+        FGB_CUDA(cudaMemcpyAsync(to.col + d, b->st_col.p, E * sizeof(uint32_t), cudaMemcpyHostToDevice, st),
                  "emit");
-        FGB_CUDA(cudaMemcpyAsync(b->slot[cn].p + d, b->st_slot.p, E * sizeof(uint32_t), cudaMemcpyHostToDevice, st),
+        FGB_CUDA(cudaMemcpyAsync(to.slot + d, b->st_slot.p, E * sizeof(uint32_t), cudaMemcpyHostToDevice, st),
                  "emit");
         FGB_CUDA(cudaMemcpyAsync(ids1.p + d, b->st_ids.p, E * sizeof(uint64_t), cudaMemcpyHostToDevice, st), "emit");
     }
     FGB_CUDA(cudaStreamSynchronize(st), "sources_drains sync");
-    if (grow) {  // the old set and the per-step arrays, at the new capacity
-        FGB_CUDA(b->x[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->v[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->type[cs].alloc(cap + 1), "sources_drains grow");
-        FGB_CUDA(b->col[cs].alloc(cap), "sources_drains grow");
-        FGB_CUDA(b->slot[cs].alloc(cap), "sources_drains grow");
+    if (grow) {  // both sets and the per-step arrays, at the new capacity
+        const uint64_t had = b->capacity;
+        const uint32_t had_hits = b->cell_hits;
+        b->drop_graphs();
+        larger[0].swap(b, cn);
+        larger[1].swap(b, cs);
         int rc = alloc_step_arrays(b, cap);
-        if (rc) return rc;
+        if (rc) {  // as before, with the per-step arrays made anew
+            const std::string why = g_last_error;
+            larger[0].swap(b, cn);
+            larger[1].swap(b, cs);
+            b->cell_hits = had_hits;
+            b->lost = alloc_step_arrays(b, had) != FGB_OK;
+            for (uint32_t s = 0; s < b->n_scenes; ++s) scene_keys(b, s);
+            return fail(rc, why.c_str());
+        }
     }
     b->ids_dev.swap(ids1);
     b->cur = cn;
