@@ -345,7 +345,11 @@ int fgb_scene_footprint(const fgb_solver *s, const fgb_config *cfg, uint64_t n, 
  * scenes are packed into groups of at most tick_particles particles; a tick
  * advances one group by one batched step, the groups taken round robin.  Finished
  * scenes optionally get a surface; their final state waits on the host for
- * fgb_serve_fetch.  Every request of one server must use the same iteration count.
+ * fgb_serve_fetch.  Requests that come in a row, each less than 4 ms after the one
+ * before and before a client has learned (poll, fetch, stats, drain) that those are
+ * finished, are taken together: from the third on, one that finds the server idle
+ * waits for its successor, 1.25 times the last gap at most.  A client that waits for
+ * each result before it submits the next request never waits for that.  Every request of one server must use the same iteration count.
  * While a server runs, its solver must not be used for other calls. */
 #define FGB_SERVE_WAITING 0
 #define FGB_SERVE_ACTIVE  1

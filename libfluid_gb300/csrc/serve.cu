@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "fgb_internal.h"
+#include "serve_arrivals.h"
 
 namespace {
 
@@ -65,6 +66,7 @@ struct Request {
     std::vector<uint32_t> col;
     double t_submit = 0, t_admit = -1, t_done = -1;
     int32_t status = FGB_SERVE_WAITING;
+    bool known = false;  // a client has been told that it is finished (fgb_server::unknown)
     uint64_t triangles = 0;
     fgb_mesh mesh{nullptr, 0, 0};
 
@@ -108,7 +110,8 @@ struct fgb_server {
     uint64_t used = 0, next_ticket = 1;
     uint64_t beyond = 0;  // of all groups: their rows beyond the footprints in `used` (set by the worker)
     bool stop = false;
-    double last_submit = -1, gap = -1;  // the last arrival, and its distance from the one before (under mu)
+    fgb::Arrivals arrivals;   // under mu
+    uint64_t unknown = 0;     // requests that no client knows to be finished (under mu)
     double t0 = 0;
     // worker-only state
     std::vector<std::unique_ptr<ServeGroup>> groups;
@@ -441,11 +444,16 @@ struct fgb_server {
         cv.notify_all();
     }
 
-    // Requests this close together are worth stepping together even when each is over
-    // before the next arrives: a lone one waits that long for its successor, where a
-    // rebuild of its own for the successor costs about a third of it.  Requests further
-    // apart never wait.
-    static constexpr double kCloseArrivals = 0.004;
+    // A client learns that r is finished (mu held).
+    void learn(Request &r) {
+        if (r.known || r.status == FGB_SERVE_WAITING || r.status == FGB_SERVE_ACTIVE) return;
+        r.known = true;
+        --unknown;
+    }
+    void learn_all() {
+        if (!unknown) return;
+        for (auto &r : requests) learn(*r.second);
+    }
 
     void run() {
         cudaSetDevice(device);
@@ -455,11 +463,11 @@ struct fgb_server {
                 std::unique_lock<std::mutex> lk(mu);
                 cv.wait(lk, [&] { return stop || !waiting.empty() || !live.empty(); });
                 if (stop) break;
-                if (!opt.one_at_a_time && live.empty() && waiting.size() == 1 && gap >= 0 && gap < kCloseArrivals) {
-                    const double left = waiting.front()->t_submit + 1.25 * gap - t();
-                    if (left > 0)
-                        cv.wait_for(lk, std::chrono::duration<double>(left),
-                                    [&] { return stop || waiting.size() > 1; });
+                if (!opt.one_at_a_time && live.empty() && waiting.size() == 1) {
+                    const double left = arrivals.wait_until() - t();
+                    if (left > 0 && !cv.wait_for(lk, std::chrono::duration<double>(left),
+                                                 [&] { return stop || waiting.size() > 1; }))
+                        arrivals.in_vain();
                     if (stop) break;
                 }
                 fresh = admit();
@@ -555,8 +563,8 @@ int fgb_serve_submit(fgb_server *sv, const fgb_config *cfg, const fgb_particles 
     std::lock_guard<std::mutex> lk(sv->mu);
     r->ticket = sv->next_ticket++;
     r->t_submit = sv->t();
-    if (sv->last_submit >= 0) sv->gap = r->t_submit - sv->last_submit;
-    sv->last_submit = r->t_submit;
+    sv->arrivals.arrived(r->t_submit, sv->unknown == 0);
+    sv->unknown++;
     *ticket = r->ticket;
     sv->waiting.push_back(r.get());
     sv->requests[r->ticket] = std::move(r);
@@ -569,7 +577,8 @@ int fgb_serve_poll(fgb_server *sv, uint64_t ticket, fgb_serve_result *out) {
     std::lock_guard<std::mutex> lk(sv->mu);
     auto it = sv->requests.find(ticket);
     if (it == sv->requests.end()) return fail(FGB_ERR_INVALID, "serve_poll: unknown ticket");
-    const Request &r = *it->second;
+    Request &r = *it->second;
+    sv->learn(r);
     out->ticket = r.ticket;
     out->n = r.n;
     out->steps = r.steps;
@@ -590,6 +599,7 @@ int fgb_serve_fetch(fgb_server *sv, uint64_t ticket, fgb_particles *xs, fgb_mesh
         if (it == sv->requests.end()) return fail(FGB_ERR_INVALID, "serve_fetch: unknown ticket");
         const int32_t st = it->second->status;
         if (st == FGB_SERVE_WAITING || st == FGB_SERVE_ACTIVE) return fail(FGB_ERR_INVALID, "serve_fetch: not done");
+        sv->learn(*it->second);
         r = std::move(it->second);
         sv->requests.erase(it);
     }
@@ -614,6 +624,7 @@ int fgb_serve_fetch(fgb_server *sv, uint64_t ticket, fgb_particles *xs, fgb_mesh
 int fgb_serve_get_stats(fgb_server *sv, fgb_serve_stats *out) {
     if (!sv || !out) return fail(FGB_ERR_INVALID, "serve_stats: null argument");
     std::lock_guard<std::mutex> lk(sv->mu);
+    sv->learn_all();
     out->ticks = sv->ticks;
     out->particle_steps = sv->particle_steps;
     out->completed = sv->completed;
@@ -676,6 +687,7 @@ int fgb_serve_drain(fgb_server *sv, double timeout_seconds) {
     const bool ok = sv->cv.wait_for(lk, std::chrono::duration<double>(timeout_seconds),
                                     [&] { return sv->waiting.empty() && sv->live.empty(); });
     if (!ok) return fail(FGB_ERR_TIMEOUT, "serve_drain: requests still pending at the timeout");
+    sv->learn_all();
     return FGB_OK;
 }
 
