@@ -80,6 +80,13 @@ def profiled(kernel, workload, key="dram_bytes_per_launch"):
     return None
 
 
+def _tuned(batch):
+    """The autotuner's choice, or None on the row kernels, where it chooses nothing (its steps
+    still grow the rows that the solver's next batches start with)."""
+    result = batch.autotune(3)
+    return None if batch.row_kernels() else result
+
+
 SMS, SCHEDULERS_PER_SM = 152, 4
 
 
@@ -341,7 +348,7 @@ def bench_large(params, steps=20, warmup=3, tune=True):
     tuned = None
     if tune:
         t = Batch(solver, [(scenes.copy_particles(parts), cfg)])
-        tuned = t.autotune(3)
+        tuned = _tuned(t)
         t.close()
     batch = Batch(solver, [(parts, cfg)])
     batch.set_timing(True)
@@ -625,7 +632,7 @@ def run_ours(args):
     # autotune on a copy of the scene (so the timed steps stay steps 5-55 of the
     # dam break); the solver caches the launch shape for this size bucket
     tuner = Batch(solver, [(scenes.copy_particles(parts), cfg)])
-    tuned = tuner.autotune(3) if not args.no_tune else None
+    tuned = _tuned(tuner) if not args.no_tune else None
     tuner.close()
     batch = Batch(solver, [(parts, cfg)])
     direct_io = batch.host_io_direct()
@@ -683,7 +690,7 @@ def run_ours(args):
     peak, peak_kind = measured_peaks()
     # the summary's figures for the configuration the autotuner chose (near rows with
     # or without Verlet lists)
-    with_lists = tuned is None or bool(tuned.verlet)
+    with_lists = not batch.row_kernels() and (tuned is None or bool(tuned.verlet))
     suffix = "_with_lists" if with_lists else ""
     traffic = profiled(dom, "dam_break_1m", "dram_bytes_per_launch" + suffix)
     # the FP32-issue ceiling of the same kernel: its warp instructions per launch
@@ -704,7 +711,7 @@ def run_ours(args):
     e2e_steps = args.steps
     host = scenes.copy_particles(parts)
     e2e_solver = SphSolver(params=params)
-    if tuned is not None:
+    if not args.no_tune:
         t = Batch(e2e_solver, [(scenes.copy_particles(parts), cfg)])
         t.autotune(3)
         t.close()

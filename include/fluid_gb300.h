@@ -246,22 +246,26 @@ uint64_t fgb_batch_launch_count(const fgb_batch *b);
  * (predict, sort, reorder, lambda/delta per iteration, vorticity, vorticity apply);
  * fgb_batch_stage_times returns the last step's per-stage milliseconds. */
 int fgb_batch_set_timing(fgb_batch *b, int on);
-/* Autotuner: runs the batch's next steps under each candidate launch shape of the list
- * kernels, which a list setting in the environment asks for (the row kernels, used
- * otherwise, choose theirs by the scene's size: there the trials are plain steps) (gather
- * CTA size 64, 128, 256 at the current Verlet skin, then skins 0.1-0.3 h at the best
- * size, then persistent tile queues of 1 and 2 particles per thread, then near rows
- * with and without Verlet lists in turn (five trials); steps_per_trial steps each, the
- * first untimed), keeps the fastest, and caches
+/* 1 where a batch's gathers run on the row kernels (the default), 0 on the list
+ * kernels, which a list setting in the environment asks for at its creation. */
+int fgb_batch_row_kernels(const fgb_batch *b, int *rows);
+/* Autotuner of the list kernels: runs the batch's next steps under each candidate
+ * launch shape (gather CTA size 64, 128, 256 at the current Verlet skin, then skins
+ * 0.1-0.3 h at the best size, then persistent tile queues of 1 and 2 particles per
+ * thread, then near rows with and without Verlet lists in turn (five trials);
+ * steps_per_trial steps each, the first untimed), keeps the fastest, and caches
  * it in the solver for every later batch of the same physics profile and size
  * bucket (floor(log2(particles))).  The trial steps are ordinary steps: no knob
  * changes a result, so a tuned batch computes the same bits as an untuned one.
+ * The row kernels choose their shapes by the scene's size: there the same number of
+ * steps is run and timed, nothing is chosen or cached, and the result holds the
+ * batch's settings as they are (persistent 0, verlet 0).
  * No counterpart in the reference (work-group sizes are left to the OpenCL
  * runtime, oclsph.hpp:597). */
 typedef struct fgb_tune_result {
     uint32_t block;      /* threads per CTA of the gather kernels */
     float skin;          /* Verlet skin, in units of h */
-    float ms_per_step;   /* of the chosen shape */
+    float ms_per_step;   /* of the chosen shape (row kernels: of all trials) */
     uint32_t trials, steps;
     uint32_t persistent; /* 1: the gathers run as persistent grids over a tile queue */
     uint32_t particles_per_thread;  /* of a persistent grid's tiles (1 otherwise) */

@@ -265,6 +265,7 @@ _SIGS = {
     "fgb_batch_host_io": (ctypes.c_int, [c_void_p, P(ctypes.c_int)]),
     "fgb_batch_prepare": (ctypes.c_int, [c_void_p]),
     "fgb_batch_launch_count": (ctypes.c_uint64, [c_void_p]),
+    "fgb_batch_row_kernels": (ctypes.c_int, [c_void_p, P(ctypes.c_int)]),
     "fgb_batch_set_timing": (ctypes.c_int, [c_void_p, ctypes.c_int]),
     "fgb_batch_autotune": (ctypes.c_int, [c_void_p, ctypes.c_uint32, P(TuneResult)]),
     "fgb_batch_sources_drains": (ctypes.c_int, [c_void_p, ctypes.c_uint32, P(Source), ctypes.c_uint32, P(Drain),

@@ -880,12 +880,37 @@ struct fgb_batch {
     // launch shape: CTA sizes first at the current skin, then skins at the best CTA
     // size.  Neither knob changes a result (the lists are exact for any skin, and
     // each thread owns one particle), so these are ordinary steps of the batch.
+    static constexpr int kTrials = 14;  // of a full search below
     int autotune(uint32_t per_trial, fgb_tune_result *out) {
         if (per_trial < 2) per_trial = 2;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         FGB_CUDA(cudaEventCreate(&e0), "autotune event");
         FGB_CUDA(cudaEventCreate(&e1), "autotune event");
         uint32_t trials = 0, steps = 0;
+        // `per_trial` steps, the first untimed
+        auto timed = [&](float *ms) -> int {
+            int rc = step(1);
+            if (!rc) rc = cudaEventRecord(e0, stream()) == cudaSuccess ? FGB_OK : fail(FGB_ERR_CUDA, "autotune");
+            if (!rc) rc = step(per_trial - 1);
+            if (!rc) rc = cudaEventRecord(e1, stream()) == cudaSuccess ? FGB_OK : fail(FGB_ERR_CUDA, "autotune");
+            if (!rc && cudaEventSynchronize(e1) != cudaSuccess) rc = fail(FGB_ERR_CUDA, "autotune sync");
+            float t = 0.f;
+            if (!rc) cudaEventElapsedTime(&t, e0, e1);
+            *ms = t / (float)(per_trial - 1);
+            trials++;
+            steps += per_trial;
+            return rc;
+        };
+        if (cell_rows) {
+            // nothing to choose: the steps that the trials of the list kernels are, timed
+            float sum = 0.f, ms = 0.f;
+            int rc = FGB_OK;
+            for (int k = 0; k < kTrials && !rc; ++k, sum += ms) rc = timed(&ms);
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            if (!rc && out) *out = fgb_tune_result{(uint32_t)block, skin_frac, sum / kTrials, trials, steps, 0u, 1u, 0u};
+            return rc;
+        }
         auto trial = [&](int blk, float skin, bool pers, uint32_t per_thread, float *ms, bool voff = false) -> int {
             block = blk;
             skin_frac = skin;
@@ -905,17 +930,7 @@ struct fgb_batch {
             for (auto &g : graph)
                 if (g) cudaGraphExecDestroy(g), g = nullptr;
             graphs_ok = false;
-            int rc = step(1);
-            if (!rc) rc = cudaEventRecord(e0, stream()) == cudaSuccess ? FGB_OK : fail(FGB_ERR_CUDA, "autotune");
-            if (!rc) rc = step(per_trial - 1);
-            if (!rc) rc = cudaEventRecord(e1, stream()) == cudaSuccess ? FGB_OK : fail(FGB_ERR_CUDA, "autotune");
-            if (!rc && cudaEventSynchronize(e1) != cudaSuccess) rc = fail(FGB_ERR_CUDA, "autotune sync");
-            float t = 0.f;
-            if (!rc) cudaEventElapsedTime(&t, e0, e1);
-            *ms = t / (float)(per_trial - 1);
-            trials++;
-            steps += per_trial;
-            return rc;
+            return timed(ms);
         };
         int rc = FGB_OK;
         int best_block = block;
@@ -2303,6 +2318,12 @@ int fgb_batch_prepare(fgb_batch *b) {
 int fgb_batch_host_io(const fgb_batch *b, int *direct) {
     if (!b || !direct) return fail(FGB_ERR_INVALID, "host_io: bad argument");
     *direct = b->direct ? 1 : 0;
+    return FGB_OK;
+}
+
+int fgb_batch_row_kernels(const fgb_batch *b, int *rows) {
+    if (!b || !rows) return fail(FGB_ERR_INVALID, "row_kernels: null argument");
+    *rows = b->cell_rows ? 1 : 0;
     return FGB_OK;
 }
 

@@ -167,8 +167,9 @@ class Batch:
         return self.counts[k]
 
     def autotune(self, steps_per_trial=3):
-        """Pick the fastest launch shape on this batch's next steps (they are ordinary
-        steps) and cache it in the solver for its size bucket; returns TuneResult."""
+        """Pick the list kernels' fastest launch shape on this batch's next steps (they are
+        ordinary steps) and cache it in the solver for its size bucket; returns TuneResult.
+        On the row kernels (row_kernels) the steps are run and timed, and nothing is chosen."""
         r = capi.TuneResult()
         capi.check(self.lib.fgb_batch_autotune(self._h, steps_per_trial, ctypes.byref(r)))
         return r
@@ -238,6 +239,12 @@ class Batch:
         capi.check(self.lib.fgb_batch_query(self._h, k, qs, nq, res, ctypes.byref(nres)))
         return [(int(res[i].id), tuple(res[i].point), int(res[i].neighbours), int(res[i].average_colour))
                 for i in range(nres.value)]
+
+    def row_kernels(self):
+        """True on the row kernels (the default), False on the list kernels."""
+        r = ctypes.c_int()
+        capi.check(self.lib.fgb_batch_row_kernels(self._h, ctypes.byref(r)))
+        return bool(r.value)
 
     def error_flags(self):
         f = ctypes.c_uint32()
