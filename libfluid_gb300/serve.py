@@ -50,7 +50,7 @@ class Server:
         mesh = capi.Mesh()
         try:
             capi.check(self.lib.fgb_serve_fetch(self._h, ticket, ctypes.byref(pv), ctypes.byref(mesh)))
-            return out, capi.mesh_to_numpy(mesh)
+            return out, capi.take_mesh(mesh)
         finally:
             self.lib.fgb_mesh_free(ctypes.byref(mesh))
 

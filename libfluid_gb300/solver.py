@@ -65,7 +65,7 @@ class SphSolver:
                                   ctypes.byref(mesh))
         try:
             capi.check(rc)
-            return capi.mesh_to_numpy(mesh) if config.surface else None
+            return capi.take_mesh(mesh) if config.surface else None
         finally:
             self.lib.fgb_mesh_free(ctypes.byref(mesh))
 
@@ -91,7 +91,7 @@ class SphSolver:
             capi.check(rc)
             out = [(int(res[i].id), tuple(res[i].point), int(res[i].neighbours), int(res[i].average_colour))
                    for i in range(nres.value)]
-            return (capi.mesh_to_numpy(mesh) if config.surface else None), out
+            return (capi.take_mesh(mesh) if config.surface else None), out
         finally:
             self.lib.fgb_mesh_free(ctypes.byref(mesh))
 
@@ -192,7 +192,7 @@ class Batch:
         mesh = capi.Mesh()
         try:
             capi.check(self.lib.fgb_batch_surface(self._h, k, ctypes.byref(mesh)))
-            return capi.mesh_to_numpy(mesh)
+            return capi.take_mesh(mesh)
         finally:
             self.lib.fgb_mesh_free(ctypes.byref(mesh))
 
@@ -205,7 +205,7 @@ class Batch:
         mesh = capi.Mesh()
         try:
             capi.check(self.lib.fgb_batch_surface_fetch(self._h, k, ctypes.byref(mesh)))
-            return capi.mesh_to_numpy(mesh)
+            return capi.take_mesh(mesh)
         finally:
             self.lib.fgb_mesh_free(ctypes.byref(mesh))
 
