@@ -283,7 +283,7 @@ int fgb_batch_stage_times(fgb_batch *b, float *ms, uint32_t max, uint32_t *count
 #define FGB_PROBE_DENSITY     5 /* f32 density of the last solver iteration */
 #define FGB_PROBE_LATTICE     6 /* f32x4 MC lattice (value, normal) of the last surface call */
 #define FGB_PROBE_CUBE_CASES  7 /* u8 MC case index per cube of the last surface call */
-/* 8, 9, 10 and 11 are of the list kernels; 0xffff, 0, 0 and 0 on the row kernels */
+/* 8, 9 and 11 are of the list kernels; the row kernels have no such list: 0xffff, 0 and 0 */
 #define FGB_PROBE_LIST_COUNT  8 /* u16 neighbour-list length per particle (0xffff: overflow) */
 #define FGB_PROBE_LIST_VALID  9 /* u8 per particle: 1 if its list served the last vorticity pass */
 #define FGB_PROBE_DISPLACEMENT 10 /* f32 distance moved since the grid was built (last delta) */

@@ -177,6 +177,7 @@ cudaError_t launch_row_lambda(const StepView &s, const float4 *ps, int iteration
 cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_out, bool last, cudaStream_t st);
 cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaStream_t st,
                                       const std::function<void()> &between);
+void launch_displacement(const StepView &s, float *out, cudaStream_t st);
 uint32_t row_later_search_launches(int profile, uint64_t n);  // kernels of a search after the first
 uint32_t row_group_mask(int profile, uint64_t n);  // StepView::group_mask for n particles
 // ref-profile colour diffusion of the sorted colours (col1, in place); agg and count

@@ -1016,6 +1016,15 @@ __global__ void __launch_bounds__(128)
     sum.finish(ph, S, a, pa, oa, vx, v, x, hout);
 }
 
+// How far the step's corrections moved each particle from its grid position (a probe).
+__global__ void k_displacement(const float4 *__restrict__ ps_grid, const float4 *__restrict__ ps, uint32_t n,
+                               float *__restrict__ out) {
+    for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
+        const float ex = ps[a].x - ps_grid[a].x, ey = ps[a].y - ps_grid[a].y, ez = ps[a].z - ps_grid[a].z;
+        out[a] = sqrtf(ex * ex + ey * ey + ez * ez);
+    }
+}
+
 RowArgs row_args(const StepView &s) {
     RowArgs A;
     A.scenes = s.scenes;
@@ -1158,6 +1167,12 @@ cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_
 cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaStream_t st,
                                        const std::function<void()> &between) {
     return s.ph.fast_root ? velocity_as<true>(s, ps, st, between) : velocity_as<false>(s, ps, st, between);
+}
+
+void launch_displacement(const StepView &s, float *out, cudaStream_t st) {
+    const float4 *last = (s.iterations & 1) ? s.ps_a : s.ps_b;
+    k_displacement<<<(unsigned)std::min<uint64_t>(((uint64_t)s.n + 255) / 256, 1216), 256, 0, st>>>(s.ps_grid, last,
+                                                                                                  s.n, out);
 }
 
 uint32_t row_later_search_launches(int profile, uint64_t n) {

@@ -2412,7 +2412,16 @@ int fgb_batch_probe(fgb_batch *b, uint32_t what, void *host_out, uint64_t bytes)
     case FGB_PROBE_DISPLACEMENT: src = b->disp.p; break;
     case FGB_PROBE_NEAR_ROW: src = b->near.p; break;
     }
-    if (b->cell_rows && what >= FGB_PROBE_LIST_COUNT && what <= FGB_PROBE_NEAR_ROW) {
+    Dev<float> moved;
+    if (b->cell_rows && what == FGB_PROBE_DISPLACEMENT) {
+        if (int rc = b->usable()) return rc;
+        if (!b->n) return FGB_OK;
+        PoolScope scope(&b->solver->pool);
+        FGB_CUDA(moved.alloc(b->n), "probe alloc");
+        launch_displacement(b->view(b->cur), moved.p, b->stream());
+        FGB_CUDA(cudaGetLastError(), "probe");
+        src = moved.p;
+    } else if (b->cell_rows && what >= FGB_PROBE_LIST_COUNT && what <= FGB_PROBE_NEAR_ROW) {
         // the kernels of rows.cu keep no lists or near rows: every list is overflowed, none valid
         memset(host_out, what == FGB_PROBE_LIST_COUNT ? 0xff : 0, bytes);
         return FGB_OK;
