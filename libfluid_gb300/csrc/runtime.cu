@@ -591,9 +591,10 @@ struct fgb_batch {
     Dev<uint32_t> over;
     Pinned<uint32_t> st_over;
     bool row_stats = false;
-    // the device error flags (err) as of the end of each step, copied by the step
-    // graph; fgb_batch_step, fgb_batch_sync and fgb_advance turn them into a status
+    // the device error flags (err) as of the end of a call's steps, and of every kReportEvery
+    // of them; fgb_batch_step, fgb_batch_sync and fgb_advance turn them into a status
     Pinned<uint32_t> st_flags;
+    static constexpr uint32_t kReportEvery = 16;
     Dev<char> wire;         // packed-record staging (wire.cu)
     int cur = 0;
     // step
@@ -1200,14 +1201,15 @@ struct fgb_batch {
             FGB_CUDA(cudaGraphLaunch(graph[cur], stream()), "graph launch");
             cur ^= 1;
             launches += launches_per_step;
+            query_ok = true;
+            if (k % kReportEvery != kReportEvery - 1 && k + 1 != steps) continue;
+            // At the end of a call and in a long one every so often, by a kernel: two copies at
+            // the end of every step, which change engines, made a step of 4 k particles 115 us
+            // instead of 107, of 14 k 135 instead of 126.
+            k_report<<<1, 1, 0, stream()>>>(over.p, err.p, report_obstacles, st_over.p, st_flags.p, st_count.p);
+            FGB_CUDA(cudaGetLastError(), "step: report");
+            launches += 1;
         }
-        if (!steps) return FGB_OK;
-        query_ok = true;
-        // Once a call, by a kernel: two copies at the end of every step, which change engines,
-        // made a step of 4 k particles 115 us instead of 107, of 14 k 135 instead of 126.
-        k_report<<<1, 1, 0, stream()>>>(over.p, err.p, report_obstacles, st_over.p, st_flags.p, st_count.p);
-        FGB_CUDA(cudaGetLastError(), "step: report");
-        launches += 1;
         return FGB_OK;
     }
 
