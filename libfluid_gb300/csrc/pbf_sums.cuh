@@ -1,5 +1,5 @@
 // pbf_sums.cuh -- the pair sums of the gather passes and what each particle does with
-// them, shared by the row kernels (pbf.cu) and the tile kernels (tiles.cu).
+// them, shared by the row kernels (rows.cu) and the list kernels (pbf.cu).
 //
 // Every sum adds its neighbours in the order it is given them, with the reference's
 // formulas; both kernel families visit the same neighbours in the same order, so they

@@ -10,13 +10,11 @@
 //
 // The test runs on pairs of candidates in 16 bits, relative to the group's first particle,
 // with a margin that covers its rounding (kHalfMargin): rows hold all that 32 bits would
-// find and about 1 % more, which the passes drop.  Instruction issue bounds the search: of
-// 175 warp instructions a particle (1 M dam break, before the candidates were gathered
-// straight to their lanes), 21 went to a cell's setup, 34 to its candidates, 120 to the
-// particle: 36 tests, 27 appends, 10 the running sum, 12 the writing of its row.  In 32 bits
-// with a ballot for every 32 candidates it took 222.  The first lambda stage (search and
-// sums) of the 1 M dam break at steps 5, 30 and 100: 357, 387 and 357 us before, 318, 328
-// and 319 now.
+// find and about 1 % more, which the passes drop.  A step's first search executes 159 warp
+// instructions a particle (262 k cube; in 32 bits with a ballot for every 32 candidates it
+// took 222) and is bound by the L1 data pipe (83 % at 1 M): the candidates' scattered 16-byte
+// loads.  The first lambda stage (search and sums) of the 1 M dam break at steps 5, 30 and
+// 100: 357, 387 and 357 us in 32 bits, 316, 328 and 319 now.
 //
 // Rows that last.  The step's first search keeps every candidate within h plus a skin of
 // the grid positions.  Such a row holds every neighbour within h, in order, while no
@@ -191,7 +189,7 @@ enum Search {
 // 2.13); 262 k 461 and 484 us a step, 110 k 271 and 276, 64 k 228 and 219, 14 k 181 and 162:
 // hence kListFrom.  With the ref profile's constants hardly any row lasts (262 k 1480 and
 // 1466): its searches ask as they go.  L1 lookups bound it, 54 scattered ones a group.
-__global__ void __launch_bounds__(128, 8) k_stale_groups(RowArgs A, uint32_t n_scenes, int count_use) {
+__global__ void __launch_bounds__(128, 8) k_stale_groups(RowArgs A, int count_use) {
     const uint32_t groups = *A.group_count, lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t c0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < groups; c0 += stride) {
@@ -1092,7 +1090,7 @@ cudaError_t rows_of(const StepView &s, const float4 *ps, uint32_t pass, cudaStre
         A.stale_count = s.group_count + pass;  // one a pass, zeroed with the groups' number
         e = resident_grid(k_stale_groups, s, 128, &grid);
         if (e != cudaSuccess) return e;
-        k_stale_groups<<<grid, 128, 0, st>>>(A, s.n_scenes, pass == 1);
+        k_stale_groups<<<grid, 128, 0, st>>>(A, pass == 1);
         e = resident_grid(k_cell_rows<kStaleSearch>, s, kCellBlock, &grid);
         if (e != cudaSuccess) return e;
         k_cell_rows<kStaleSearch><<<grid, kCellBlock, 0, st>>>(A, ps, r2max, s.n_scenes, 0);
@@ -1181,10 +1179,12 @@ uint32_t row_later_search_launches(int profile, uint64_t n) {
 
 // Particles of a group.  A cell's setup is shared by the particles of its group, but small
 // scenes have too few cells to fill the GPU, and the ref profile's constants clump the fluid
-// into few crowded ones, so a cell's particles go to several warps.  us a step, groups that
-// end at multiples of 4 / 8 / 16 / 256: baseline 4 k 144 / 147 / 152 / 152, 14 k 163 / 158 /
-// 159 / 158, 64 k 235 / 227 / 223 / 222, 110 k 311 / 295 / 285 / 276; ref 14 k - / 441 / 471
-// / -, 64 k - / 594 / 589 / -, 262 k - / 1511 / 1472 / -.
+// into few crowded ones, so a cell's particles go to several warps.  us a step (cubes at rest,
+// steps 10 to 30), groups that end at multiples of 4 / 8 / 16 / 32 / 256: baseline 4 k 107 / 111
+// / 113 / 113 / 115, 14 k 126 / 120 / 122 / 122 / 121, 64 k 248 / 229 / 221 / 217 / 212, 110 k
+// 272 / 266 / 264 / 260 / 258; ref 14 k 319 / 323 / 355 / 427 / 581, 33 k 640 / 614 / 620 / 676
+// / 821, 64 k 969 / 931 / 937 / 1004 / 1099, 123 k 1349 / 1261 / 1258 / 1303 / 1429, 250 k
+// 2182 / 1996 / 1933 / 1957 / 2068, 1 M 6412 / 5664 / 5312 / 5190 / 5202.
 uint32_t row_group_mask(int profile, uint64_t n) {
     if (profile == FGB_PROFILE_REF) return n < 65536 ? 7u : 15u;
     return n < 8000 ? 3u : 255u;
