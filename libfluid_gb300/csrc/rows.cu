@@ -1146,7 +1146,10 @@ cudaError_t velocity_as(const StepView &s, const float4 *ps, cudaStream_t st, co
 
 }  // namespace
 
+// A batch without particles (scenes that are yet to be filled, or drained) has nothing to launch.
+
 cudaError_t launch_row_lambda(const StepView &s, const float4 *ps, int iteration, cudaStream_t st) {
+    if (!s.n) return cudaSuccess;
     if (s.ph.profile == FGB_PROFILE_REF)
         return s.ph.fast_root ? lambda_as<FGB_PROFILE_REF, true>(s, ps, iteration, st)
                               : lambda_as<FGB_PROFILE_REF, false>(s, ps, iteration, st);
@@ -1155,6 +1158,7 @@ cudaError_t launch_row_lambda(const StepView &s, const float4 *ps, int iteration
 }
 
 cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_out, bool last, cudaStream_t st) {
+    if (!s.n) return cudaSuccess;
     if (s.ph.profile == FGB_PROFILE_REF)
         return s.ph.fast_root ? delta_as<FGB_PROFILE_REF, true>(s, ps_in, ps_out, last, st)
                               : delta_as<FGB_PROFILE_REF, false>(s, ps_in, ps_out, last, st);
@@ -1164,6 +1168,10 @@ cudaError_t launch_row_delta(const StepView &s, const float4 *ps_in, float4 *ps_
 
 cudaError_t launch_row_velocity_terms(const StepView &s, const float4 *ps, cudaStream_t st,
                                        const std::function<void()> &between) {
+    if (!s.n) {
+        if (between) between();
+        return cudaSuccess;
+    }
     return s.ph.fast_root ? velocity_as<true>(s, ps, st, between) : velocity_as<false>(s, ps, st, between);
 }
 
