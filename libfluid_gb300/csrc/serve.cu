@@ -84,7 +84,7 @@ struct Request {
 // active requests -- the step latency stays flat while requests come and go.
 struct ServeGroup {
     fgb_batch *batch = nullptr;
-    std::vector<Request *> scenes;  // scene k of `batch` is scenes[k]
+    std::vector<Request *> scenes;  // scene k of `batch` is scenes[k] (null: it is finished)
     std::vector<Request *> want;    // membership for the next tick
     uint64_t particles = 0;         // of `want`
     uint32_t mbits = 0;             // largest Morton key width in `want`
@@ -434,6 +434,8 @@ struct fgb_server {
             r->t_done = t();
             used -= r->footprint;
             completed++;
+            // once fetched it is gone, and a later request may lie at its address
+            *std::find(g.scenes.begin(), g.scenes.end(), r) = nullptr;
         }
         if (!done.empty()) {
             std::vector<Request *> keep;
@@ -478,7 +480,8 @@ struct fgb_server {
             // device), then release the batches nothing uses any more
             std::map<Request *, Home> where;
             for (auto &g : groups)
-                for (size_t k = 0; k < g->scenes.size(); ++k) where[g->scenes[k]] = Home{g->batch, (uint32_t)k};
+                for (size_t k = 0; k < g->scenes.size(); ++k)
+                    if (g->scenes[k]) where[g->scenes[k]] = Home{g->batch, (uint32_t)k};
             std::vector<fgb_batch *> retired;
             for (auto &g : groups)
                 if (g->want != g->scenes) {
