@@ -167,6 +167,19 @@ __device__ __forceinline__ uint32_t morton_of(uint32_t key, uint32_t mbits) {
     return mbits >= 32 ? key : (key & ((1u << mbits) - 1u));
 }
 
+// The groups that a cell's particles form in the sorted order (rows.cu).  A group ends with its
+// cell, where its index wraps under `mask`, and in a crowded cell before 32 more particles of it
+// whose indices differ in their low five bits alone (a warp that had hundreds of a cell's particles
+// to itself would keep the others waiting).  So one begins at a cell's first particle, and at i:
+__host__ __device__ __forceinline__ bool group_begins(uint32_t i, uint32_t mask, bool crowd) {
+    return (i & mask) == 0 || ((i & 31u) == 0 && crowd);  // crowd: the particles [i, i + 32) share a cell
+}
+// The end of the group that begins at `first`, in the cell that ends at `to`.
+__host__ __device__ __forceinline__ uint32_t group_end(uint32_t first, uint32_t to, uint32_t mask) {
+    const uint32_t wrap = (first | mask) + 1, last = to < wrap ? to : wrap, next = (first | 31u) + 1;
+    return next + 32 <= to && next < last ? next : last;
+}
+
 // The next value of one axis's interleaved bits (mask m) of a Morton code: the bits
 // of the other axes are set so that the carry runs through them, then cleared.
 __device__ __forceinline__ uint32_t morton_inc(uint32_t s, uint32_t m) { return ((s | ~m) + 1u) & m; }

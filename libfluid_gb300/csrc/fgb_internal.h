@@ -137,8 +137,8 @@ struct StepView {
     // the build pass counts the Verlet rows [0] and hit rows [1] that overflowed
     uint32_t *over;
     // the gathers run on the hit rows of rows.cu, else (null) on the list kernels of
-    // pbf.cu: the first particle of every group -- a cell's particles up to where the
-    // index under group_mask wraps -- and the groups' number (zeroed every step)
+    // pbf.cu: the first particle of every group (group_end: of a cell's particles, under
+    // group_mask) and the groups' number (zeroed every step)
     uint32_t none;  // the entry past the particles that lies at infinity: what fills a hit row's last quad
     uint32_t *groups, *group_count, group_mask;
     float4 *pv;            // per particle: p* and mass, velocity after the last delta pass

@@ -165,7 +165,7 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
     uint32_t lo = 0xffffffffu, hi = 0xffffffffu;
     for (uint32_t from = blockIdx.x * blockDim.x; from < n; from += gridDim.x * blockDim.x) {
         const uint32_t i = from + threadIdx.x;
-        bool start = false;  // of a group
+        bool first = false;  // of a cell
         if (i < n) {
             const uint32_t j = vals[i];
             const uint32_t key = keys[i];
@@ -182,8 +182,7 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
             ps[i] = make_float4(p.x, p.y, p.z, xj.w);
             lo = min(lo, __float_as_uint(xj.w));
             hi = min(hi, ~__float_as_uint(xj.w));
-            const bool first = i == 0 || keys[i - 1] != key;
-            start = first || (i & group_mask) == 0;
+            first = i == 0 || keys[i - 1] != key;
             const uint64_t c = (uint64_t)S.table_base + morton_of(key, mbits);
             if (c >= cells_n) {
                 raise_error(err, ERR_CELL_RANGE);
@@ -195,6 +194,8 @@ __global__ void k_reorder_cells(const SceneDev *__restrict__ scenes, const WellD
         if (groups) {
             // list the groups of each cell's particles, by one atomic a CTA (one a warp cost
             // 8 us of 38 at 1 M particles, and left the list in less order)
+            const bool crowd = (__ballot_sync(0xffffffffu, first) & ~1u) == 0 && (i | 31u) < n;
+            const bool start = first || (i < n && group_begins(i, group_mask, crowd));
             const unsigned starts = __ballot_sync(0xffffffffu, start);
             if (threadIdx.x == 0) s_groups = 0;
             __syncthreads();
