@@ -54,6 +54,7 @@ struct RowArgs {
     uint32_t hcap;               // entries a hit row has room for (a multiple of four)
     uint32_t none;               // the index that fills a row's last quad: the far entry past the particles
     int fetch;                   // the passes ask for their rows ahead (fetch_rows)
+    uint32_t sparse;             // groups in 100 particles above which searches go by particles (0: never)
     const uint32_t *mass_range;
     uint32_t *over;              // hit rows that overflowed (null: not counted)
     const float4 *ps_grid;       // the grid positions
@@ -175,6 +176,60 @@ struct Pairs {
 // before its sign is settled add 2 * 2^-11 (it stays within 2): below 0.0086 in all.
 constexpr float kHalfReach = 2.f, kHalfMargin = 0.0087f;
 
+// Whether the step's searches go by particles: a thread builds the row of one by itself.  With
+// hardly more than a particle a cell a warp that takes a cell has one particle to share its
+// setup, and waits for the chain of loads to its candidates (sparse_above).  The rows carry no
+// skin then: a search goes through all of them again.
+__device__ __forceinline__ bool sparse(const RowArgs &A) {
+    return A.sparse && 100ull * *A.group_count > (uint64_t)A.sparse * A.n;
+}
+
+// The rows of positions ps, by a thread each.
+__device__ __forceinline__ void rows_by_particles(const RowArgs &A, const float4 *__restrict__ ps, float r2max) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < A.n; base += gridDim.x * blockDim.x) {
+        const uint32_t a = base + lane;
+        uint32_t found = 0;
+        if (a < A.n) {
+            const uint32_t key = A.keys[a], m = morton_of(key, A.mbits);
+            const SceneDev &S = A.scenes[scene_of(key, A.mbits)];
+            if (!(S.obstacles && A.type[a] == FGB_TYPE_OBSTACLE)) {  // no sums: an empty row
+                const float4 pa = __ldg(&ps[a]);
+                uint4 *row = row_of(A, a);
+                uint4 quad = make_uint4(A.none, A.none, A.none, A.none);
+#pragma unroll 1
+                for (int dz = -1; dz <= 1; ++dz) {
+                    uint2 range[9];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        uint32_t cell;
+                        range[k] = make_uint2(0, 0);
+                        if (neighbour_cell(S, m, k % 3 - 1, k / 3 - 1, dz, cell)) range[k] = __ldg(&A.cells[cell]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 9; ++k)
+                        for (uint32_t b = range[k].x; b < range[k].y; ++b) {
+                            const float4 p = __ldg(&ps[b]);
+                            if (!(dist2(p.x - pa.x, p.y - pa.y, p.z - pa.z) < r2max)) continue;
+                            const uint32_t at = found++ & 3u;
+                            if (at == 0) quad = make_uint4(b, A.none, A.none, A.none);
+                            else if (at == 1) quad.y = b;
+                            else if (at == 2) quad.z = b;
+                            else quad.w = b;
+                            if (at == 3 && found <= A.hcap) row[(found - 4) * 8] = quad;
+                        }
+                }
+                if ((found & 3u) && found <= A.hcap) row[(found >> 2) * 32] = quad;
+            }
+            A.hcount[a] = found > A.hcap ? kListOverflow : (uint16_t)found;
+        }
+        if (A.over) {
+            const unsigned full = __ballot_sync(0xffffffffu, found > A.hcap);
+            if (full && lane == 0) atomicAdd(A.over, (uint32_t)__popc(full));
+        }
+    }
+}
+
 enum Search {
     kFirstSearch,  // the step's first one (the grid positions): all groups
     kLaterSearch,  // leaves the groups whose rows still last
@@ -190,6 +245,7 @@ enum Search {
 // hence kListFrom.  With the ref profile's constants hardly any row lasts (262 k 1480 and
 // 1466): its searches ask as they go.  L1 lookups bound it, 54 scattered ones a group.
 __global__ void __launch_bounds__(128, 8) k_stale_groups(RowArgs A, int count_use) {
+    if (sparse(A)) return;
     const uint32_t groups = *A.group_count, lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t c0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); c0 < groups; c0 += stride) {
@@ -265,6 +321,7 @@ __global__ void __launch_bounds__(kCellBlock, 7)
     const uint32_t warps = gridDim.x * kCellWarps, groups = kSearch == kStaleSearch ? *A.stale_count : *A.group_count;
     if (kFirst && blockIdx.x == 0)
         for (uint32_t k = threadIdx.x; k < n_scenes; k += kCellBlock) A.policy_next[k] = decide(A.policy[k]);
+    if (sparse(A)) return rows_by_particles(A, ps, r2max);  // all of them, at every search of the step
     // the lane's neighbour cell: x fastest; lanes 27 to 31 have none
     const int dz = (int)lane / 9 - 1, dy = (int)lane / 3 % 3 - 1, dx = (int)lane % 3 - 1;
     // particles of one scene that this warp asked and that used their rows
@@ -1023,6 +1080,17 @@ __global__ void k_displacement(const float4 *__restrict__ ps_grid, const float4 
     }
 }
 
+// RowArgs::sparse for n particles.  us a step by warps / by particles, of clouds of 0.1, 0.25, 0.5,
+// 1, 1.5, 2 and 3 particles a cell (99, 88, 79, 63, 52, 43 and 32 groups in 100 particles), baseline
+// profile: 10 k 119 / 109, 114 / 132, 105 / 153; 30 k 186 / 121, 185 / 144, 180 / 168, 175 / 219;
+// 50 k 266 / 141, 255 / 160, 247 / 188, 232 / 225, 221 / 261; 100 k 308 / 168, 413 / 190, 386 / 223,
+// 349 / 272, 333 / 313, 313 / 345; 1 M 2469 / 911, 3453 / 1029, 3123 / 1246, 2701 / 1593, 2424 /
+// 1877, 2222 / 2175, 1971 / 2602.  With the ref profile, whose fluid gathers, the lines would lie a
+// little higher: 30 k at 0.5 a cell 164 / 180, 1 M at 1.5 1830 / 1979.
+uint32_t sparse_above(uint64_t n) {
+    return n < 30000 ? 0u : n < 45000 ? 80u : n < 75000 ? 60u : n < 400000 ? 48u : 38u;
+}
+
 RowArgs row_args(const StepView &s) {
     RowArgs A;
     A.scenes = s.scenes;
@@ -1041,6 +1109,7 @@ RowArgs row_args(const StepView &s) {
     A.hcap = s.hcap;
     A.none = s.none;
     A.fetch = s.n >= kFetchFrom;
+    A.sparse = sparse_above(s.n);
     A.mass_range = s.mass_range;
     A.over = nullptr;
     A.ps_grid = s.ps_grid;
